@@ -104,6 +104,8 @@ def _params(case, seed, member=0):
     p.nodes_x, p.nodes_y, p.nodes_z = case["nx"], case["ny"], case["nz"]
     if case["flow"] == "forced" and case["nx"] >= 1024:
         p.f_nu, p.rk3_dt = 0.0008, 0.001
+    if case["flow"] == "decay":   # a stable step on the finer grids too
+        p.rk3_dt = min(p.rk3_dt, 0.5 / max(case["nx"], case["ny"], case["nz"]))
     if case["kind"] == "batch":
         p.f_nu = 0.01 * (64.0 / case["nx"])
     p.precision = pandora.PREC_FP32_MIXED if case["precision"] == "fp32_mixed" else pandora.PREC_FP64
