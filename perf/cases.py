@@ -78,8 +78,9 @@ def draw(rng):
     if kind == "batch":
         n = rng.choice(BATCH_LENGTHS)
         members = max(1, min(40, int((192 ** 3 / n ** 3) * 2 ** rng.uniform(-2.0, 1.0))))
+        steps = int(8.0e7 / (members * n ** 3) * rng.uniform(0.5, 1.0))
         return _batch(None, flow if flow != "forced" else "decay", n, members, precision,
-                      max(4, min(40, int(8.0e7 / (members * n ** 3)) + rng.randint(1, 4))), rng.choice([0, 1 << 14]))
+                      max(4, min(40, steps)) + rng.randint(0, 5), rng.choice([0, 1 << 14, int(2.0 ** rng.uniform(8.0, 15.0))]))
     while True:
         base = 24.0 * (448.0 / 24.0) ** rng.random()
         n = tuple(near(LENGTHS, base * 2 ** rng.uniform(-0.8, 0.8)) for _ in range(3))
