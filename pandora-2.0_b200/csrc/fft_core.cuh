@@ -97,95 +97,119 @@ template <class C> PD_HD C cmulc(C a, C b) {
 template <int S, class C> PD_HD C twmul(C a, C w) { return S < 0 ? cmul(a, w) : cmulc(a, w); }
 // a * (S i)
 template <int S, class C> PD_HD C mul_si(C a) { return S > 0 ? mk(-a.y, a.x) : mk(a.y, -a.x); }
-// a * (c + S i s)
-// = a * (cc, cc) + (-a.y, a.x) * (ss, ss)
-template <int S, class C> PD_HD C mul_cs(C a, double c, double s) {
-    using T = real_of<C>;
-    const T cc = (T)c, ss = (T)(S > 0 ? s : -s);
+// a + k b for a real constant k
+template <class C> PD_HD C axpy(C a, double k, C b) {
+    const real_of<C> t = (real_of<C>)k;
 #if PD_F32X2
-    if constexpr (packed_f32<C>()) return __ffma2_rn(a, mk(cc, cc), __fmul2_rn(mk(-a.y, a.x), mk(ss, ss)));
+    if constexpr (packed_f32<C>()) return __ffma2_rn(mk(t, t), b, a);
     else
 #endif
-    return mk(a.x * cc - a.y * ss, a.x * ss + a.y * cc);
+    return mk(a.x + t * b.x, a.y + t * b.y);
 }
+// The butterfly of a constant twiddle w = c + S i s: p = e + w o, m = e - w o, with the
+// larger of c and s taken out of w, so that the product of the twiddle and the two sums are
+// six fused multiply-adds (a complex product and two sums: four and four).  In the FP64 x pass,
+// bound by its FP64 instructions at 8 to 16 warps per SM, this, the zero inputs of truncated
+// spectra (below), the shared twiddles of wpass_n and one-warp CTAs took the 512-point pass of
+// 512^3 from 2.99 to 2.52 ms per stage, the 256-point one from 0.334 to 0.312, the R-conv one
+// at 192^3 from 0.445 to 0.306 (FP32-mixed at 512^3: 1.46 to 1.28).
+template <int S, class C> PD_HD void bfly_cs(C e, C o, double c, double s, C& p, C& m) {
+    const double cs = S * s;
+    const bool cl = (c < 0 ? -c : c) >= (s < 0 ? -s : s);   // folded: c and s are literals
+    const C io = mk(-o.y, o.x);
+    const C q = cl ? axpy(o, cs / c, io) : axpy(io, c / cs, o);
+    const double f = cl ? c : cs;
+    p = axpy(e, f, q);
+    m = axpy(e, -f, q);
+}
+// p = a + b, m = a - b, where ZA / ZB say that a / b is a zero known at compile time (an
+// input outside the band of a truncated spectrum): no arithmetic is spent on it.
+template <bool ZA, bool ZB, class C> PD_HD void addsub(C a, C b, C& p, C& m) {
+    if constexpr (ZB) { p = a; m = a; }
+    else if constexpr (ZA) { p = b; m = mk(-b.x, -b.y); }
+    else { p = add(a, b); m = sub(a, b); }
+}
+// The even / odd bits of an input mask.
+constexpr unsigned even_bits(unsigned z) {
+    unsigned r = 0;
+    for (int q = 0; q < 16; q++) r |= ((z >> (2 * q)) & 1u) << q;
+    return r;
+}
+constexpr unsigned odd_bits(unsigned z) { return even_bits(z >> 1); }
 
 constexpr double kSqrtHalf = 0.7071067811865475244008444;
 constexpr double kSin60 = 0.8660254037844386467637232;
 
-template <int S, class C> PD_HD void dft2(C* v) {
+// DFTs of 2..32 points in registers.  Z: mask of the inputs that are zero at compile time.
+template <int S, unsigned Z = 0, class C> PD_HD void dft2(C* v) {
     C a = v[0], b = v[1];
-    v[0] = add(a, b); v[1] = sub(a, b);
+    addsub<(Z & 1u) != 0, (Z & 2u) != 0>(a, b, v[0], v[1]);
 }
 template <int S, class C> PD_HD void dft3(C* v) {
-    C t = add(v[1], v[2]), d = sub(v[1], v[2]);
-    C m = sub(v[0], scl(t, 0.5));
-    C e = mul_si<S>(scl(d, kSin60));
+    const C t = add(v[1], v[2]), d = mul_si<S>(sub(v[1], v[2]));
+    const C m = axpy(v[0], -0.5, t);
     v[0] = add(v[0], t);
-    v[1] = add(m, e);
-    v[2] = sub(m, e);
+    v[1] = axpy(m, kSin60, d);
+    v[2] = axpy(m, -kSin60, d);
 }
-template <int S, class C> PD_HD void dft4(C* v) {
-    C a0 = add(v[0], v[2]), a1 = sub(v[0], v[2]);
-    C b0 = add(v[1], v[3]), b1 = mul_si<S>(sub(v[1], v[3]));
+template <int S, unsigned Z = 0, class C> PD_HD void dft4(C* v) {
+    C a0, a1, b0, b1;
+    addsub<(Z & 1u) != 0, (Z & 4u) != 0>(v[0], v[2], a0, a1);
+    addsub<(Z & 2u) != 0, (Z & 8u) != 0>(v[1], v[3], b0, b1);
+    b1 = mul_si<S>(b1);
     v[0] = add(a0, b0); v[2] = sub(a0, b0);
     v[1] = add(a1, b1); v[3] = sub(a1, b1);
 }
-template <int S, class C> PD_HD void dft8(C* v) {
+template <int S, unsigned Z = 0, class C> PD_HD void dft8(C* v) {
     C e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-    dft4<S>(e); dft4<S>(o);
-    o[1] = mul_cs<S>(o[1], kSqrtHalf, kSqrtHalf);
+    dft4<S, even_bits(Z)>(e); dft4<S, odd_bits(Z)>(o);
     o[2] = mul_si<S>(o[2]);
-    o[3] = mul_cs<S>(o[3], -kSqrtHalf, kSqrtHalf);
-#pragma unroll
-    for (int r = 0; r < 4; r++) { v[r] = add(e[r], o[r]); v[r + 4] = sub(e[r], o[r]); }
+    v[0] = add(e[0], o[0]); v[4] = sub(e[0], o[0]);
+    bfly_cs<S>(e[1], o[1], kSqrtHalf, kSqrtHalf, v[1], v[5]);
+    v[2] = add(e[2], o[2]); v[6] = sub(e[2], o[2]);
+    bfly_cs<S>(e[3], o[3], -kSqrtHalf, kSqrtHalf, v[3], v[7]);
 }
-template <int S, class C> PD_HD void dft16(C* v) {
+// cos and sin of pi r / 16, r = 0..8 (sin of r is cos of 8 - r)
+PD_HD double cos16(int r) {
+    return r == 0 ? 1.0 : r == 1 ? 0.9807852804032304491261822 : r == 2 ? 0.9238795325112867561281832
+         : r == 3 ? 0.8314696123025452370787884 : r == 4 ? kSqrtHalf : r == 5 ? 0.5555702330196022247428308
+         : r == 6 ? 0.38268343236508977172846 : r == 7 ? 0.1950903220161282678482849 : 0.0;
+}
+// Twiddle W_{2H}^(S r) = cos(pi r / H) + S i sin(pi r / H), H = 8 or 16, applied in the last
+// radix-2 step of an even/odd split: v[r], v[r + H] = e[r] +- w o[r].
+template <int S, int H, class C> PD_HD void combine(const C* e, const C* o, C* v) {
+    constexpr int q = 16 / H;   // units of pi / 16
+#pragma unroll
+    for (int r = 0; r < H; r++) {
+        if (r == 0) { v[0] = add(e[0], o[0]); v[H] = sub(e[0], o[0]); }
+        else if (2 * r == H) {
+            const C t = mul_si<S>(o[r]);
+            v[r] = add(e[r], t); v[r + H] = sub(e[r], t);
+        } else {
+            const double c = 2 * r < H ? cos16(q * r) : -cos16(16 - q * r);
+            const double s = 2 * r < H ? cos16(8 - q * r) : cos16(q * r - 8);
+            bfly_cs<S>(e[r], o[r], c, s, v[r], v[r + H]);
+        }
+    }
+}
+template <int S, unsigned Z = 0, class C> PD_HD void dft16(C* v) {
     C e[8], o[8];
 #pragma unroll
     for (int q = 0; q < 8; q++) { e[q] = v[2 * q]; o[q] = v[2 * q + 1]; }
-    dft8<S>(e); dft8<S>(o);
-    constexpr double c1 = 0.9238795325112867561281832, s1 = 0.38268343236508977172846;
-    o[1] = mul_cs<S>(o[1], c1, s1);
-    o[2] = mul_cs<S>(o[2], kSqrtHalf, kSqrtHalf);
-    o[3] = mul_cs<S>(o[3], s1, c1);
-    o[4] = mul_si<S>(o[4]);
-    o[5] = mul_cs<S>(o[5], -s1, c1);
-    o[6] = mul_cs<S>(o[6], -kSqrtHalf, kSqrtHalf);
-    o[7] = mul_cs<S>(o[7], -c1, s1);
-#pragma unroll
-    for (int r = 0; r < 8; r++) { v[r] = add(e[r], o[r]); v[r + 8] = sub(e[r], o[r]); }
+    dft8<S, even_bits(Z)>(e); dft8<S, odd_bits(Z)>(o);
+    combine<S, 8>(e, o, v);
 }
-// 32 = 2 x 16: radix-2 decimation in time over two length-16 DFTs, twiddles
-// W32^(S r) = cos(pi r / 16) + S i sin(pi r / 16) for r = 1..15.
-template <int S, class C> PD_HD void dft32(C* v) {
+// 32 = 2 x 16: radix-2 decimation in time over two length-16 DFTs.
+template <int S, unsigned Z = 0, class C> PD_HD void dft32(C* v) {
     C e[16], o[16];
 #pragma unroll
     for (int q = 0; q < 16; q++) { e[q] = v[2 * q]; o[q] = v[2 * q + 1]; }
-    dft16<S>(e); dft16<S>(o);
-    constexpr double c1 = 0.9807852804032304491261822, s1 = 0.1950903220161282678482849;
-    constexpr double c2 = 0.9238795325112867561281832, s2 = 0.38268343236508977172846;
-    constexpr double c3 = 0.8314696123025452370787884, s3 = 0.5555702330196022247428308;
-    o[1] = mul_cs<S>(o[1], c1, s1);
-    o[2] = mul_cs<S>(o[2], c2, s2);
-    o[3] = mul_cs<S>(o[3], c3, s3);
-    o[4] = mul_cs<S>(o[4], kSqrtHalf, kSqrtHalf);
-    o[5] = mul_cs<S>(o[5], s3, c3);
-    o[6] = mul_cs<S>(o[6], s2, c2);
-    o[7] = mul_cs<S>(o[7], s1, c1);
-    o[8] = mul_si<S>(o[8]);
-    o[9] = mul_cs<S>(o[9], -s1, c1);
-    o[10] = mul_cs<S>(o[10], -s2, c2);
-    o[11] = mul_cs<S>(o[11], -s3, c3);
-    o[12] = mul_cs<S>(o[12], -kSqrtHalf, kSqrtHalf);
-    o[13] = mul_cs<S>(o[13], -c3, s3);
-    o[14] = mul_cs<S>(o[14], -c2, s2);
-    o[15] = mul_cs<S>(o[15], -c1, s1);
-#pragma unroll
-    for (int r = 0; r < 16; r++) { v[r] = add(e[r], o[r]); v[r + 16] = sub(e[r], o[r]); }
+    dft16<S, even_bits(Z)>(e); dft16<S, odd_bits(Z)>(o);
+    combine<S, 16>(e, o, v);
 }
 // 12 = 3 x 4 (Cooley-Tukey): n = 4 n1 + n2, k = k1 + 3 k2.  Length-3 DFTs over n1
-// for each n2, twiddles W12^(S n2 k1) (multiples of 30 degrees), length-4 DFTs over
-// n2 for each k1.
+// for each n2, twiddles W12^(S n2 k1) (multiples of 30 degrees) folded into the first
+// butterflies of the length-4 DFTs over n2 for each k1.
 template <int S, class C> PD_HD void dft12(C* v) {
     C y[4][3];
 #pragma unroll
@@ -193,22 +217,26 @@ template <int S, class C> PD_HD void dft12(C* v) {
         y[n2][0] = v[n2]; y[n2][1] = v[4 + n2]; y[n2][2] = v[8 + n2];
         dft3<S>(y[n2]);
     }
-    // W12^m = cos(30 m deg) + S i sin(30 m deg) for m = n2 k1 in 1..6
-    y[1][1] = mul_cs<S>(y[1][1], kSin60, 0.5);            // m = 1
-    y[1][2] = mul_cs<S>(y[1][2], 0.5, kSin60);            // m = 2
-    y[2][1] = mul_cs<S>(y[2][1], 0.5, kSin60);            // m = 2
-    y[2][2] = mul_cs<S>(y[2][2], -0.5, kSin60);           // m = 4
-    y[3][1] = mul_si<S>(y[3][1]);                          // m = 3
-    y[3][2] = mk(-y[3][2].x, -y[3][2].y);                  // m = 6
+    C z[4] = {y[0][0], y[1][0], y[2][0], y[3][0]};
+    dft4<S>(z);
 #pragma unroll
-    for (int k1 = 0; k1 < 3; k1++) {
-        C z[4] = {y[0][k1], y[1][k1], y[2][k1], y[3][k1]};
-        dft4<S>(z);
-#pragma unroll
-        for (int k2 = 0; k2 < 4; k2++) v[k1 + 3 * k2] = z[k2];
-    }
+    for (int k2 = 0; k2 < 4; k2++) v[3 * k2] = z[k2];
+    C a0, a1, p, m;
+    // k1 = 1: twiddles 30, 60 and 90 degrees; p, m = i S y3 +- w1 y1
+    bfly_cs<S>(y[0][1], y[2][1], 0.5, kSin60, a0, a1);
+    bfly_cs<S>(mul_si<S>(y[3][1]), y[1][1], kSin60, 0.5, p, m);
+    m = mul_si<S>(m);
+    v[1] = add(a0, p); v[7] = sub(a0, p);
+    v[4] = sub(a1, m); v[10] = add(a1, m);
+    // k1 = 2: twiddles 60, 120 and 180 degrees; p, m = y3 +- w1 y1
+    bfly_cs<S>(y[0][2], y[2][2], -0.5, kSin60, a0, a1);
+    bfly_cs<S>(y[3][2], y[1][2], 0.5, kSin60, p, m);
+    p = mul_si<S>(p);
+    v[2] = sub(a0, m); v[8] = add(a0, m);
+    v[5] = add(a1, p); v[11] = sub(a1, p);
 }
-// odd prime R (5, 7): X_r = v0 + sum_{q=1}^{(R-1)/2} [C(qr)(v_q + v_{R-q}) + S i S(qr)(v_q - v_{R-q})]
+// odd prime R (5, 7): X_r, X_{R-r} = A_r +- S i B_r with A_r = v0 + sum_q C(qr)(v_q + v_{R-q}),
+// B_r = sum_q S(qr)(v_q - v_{R-q}), q = 1..(R-1)/2
 template <int R> struct PrimeTab;
 template <> struct PrimeTab<5> {
     static PD_HD double c(int m) {
@@ -230,36 +258,46 @@ template <> struct PrimeTab<7> {
              : m == 5 ? -0.9749279121818236070181317 : -0.7818314824680298087084445;
     }
 };
-template <int R, int S, class C> PD_HD void dft_prime(C* v) {
-    C sum[(R - 1) / 2], dif[(R - 1) / 2];
+template <int R, int S, unsigned Z = 0, class C> PD_HD void dft_prime(C* v) {
+    constexpr int H = (R - 1) / 2;
+    // the one input that can be zero at compile time: the middle one, v_H (pair H, H + 1)
+    constexpr bool zm = ((Z >> H) & 1u) != 0;
+    static_assert((Z & ~(1u << H)) == 0, "zero mask of a prime radix");
+    C sum[H], dif[H];
 #pragma unroll
-    for (int q = 1; q <= (R - 1) / 2; q++) { sum[q - 1] = add(v[q], v[R - q]); dif[q - 1] = sub(v[q], v[R - q]); }
-    C out[R];
-    C x0 = v[0];
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        C acc = x0;
-#pragma unroll
-        for (int q = 1; q <= (R - 1) / 2; q++) {
-            const int m = (q * r) % R;
-            acc = add(acc, scl(sum[q - 1], PrimeTab<R>::c(m)));
-            acc = add(acc, mul_si<S>(scl(dif[q - 1], PrimeTab<R>::s(m))));
-        }
-        out[r] = acc;
+    for (int q = 1; q <= H; q++) {
+        if (q == H) addsub<zm, false>(v[q], v[R - q], sum[q - 1], dif[q - 1]);
+        else addsub<false, false>(v[q], v[R - q], sum[q - 1], dif[q - 1]);
+        dif[q - 1] = mul_si<S>(dif[q - 1]);
     }
+    const C x0 = v[0];
+    C t = x0;
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = out[r];
+    for (int q = 0; q < H; q++) t = add(t, sum[q]);
+    v[0] = t;
+#pragma unroll
+    for (int r = 1; r <= H; r++) {
+        C a = x0, b = scl(dif[0], PrimeTab<R>::s(r));
+#pragma unroll
+        for (int q = 1; q <= H; q++) {
+            const int m = (q * r) % R;
+            a = axpy(a, PrimeTab<R>::c(m), sum[q - 1]);
+            if (q > 1) b = axpy(b, PrimeTab<R>::s(m), dif[q - 1]);
+        }
+        v[r] = add(a, b);
+        v[R - r] = sub(a, b);
+    }
 }
 
-template <int R, int S, class C> PD_HD void dft(C* v) {
-    if constexpr (R == 2) dft2<S>(v);
+template <int R, int S, unsigned Z = 0, class C> PD_HD void dft(C* v) {
+    if constexpr (R == 2) dft2<S, Z>(v);
     else if constexpr (R == 3) dft3<S>(v);
-    else if constexpr (R == 4) dft4<S>(v);
-    else if constexpr (R == 8) dft8<S>(v);
-    else if constexpr (R == 16) dft16<S>(v);
+    else if constexpr (R == 4) dft4<S, Z>(v);
+    else if constexpr (R == 8) dft8<S, Z>(v);
+    else if constexpr (R == 16) dft16<S, Z>(v);
     else if constexpr (R == 12) dft12<S>(v);
-    else if constexpr (R == 32) dft32<S>(v);
-    else if constexpr (R == 5 || R == 7) dft_prime<R, S>(v);
+    else if constexpr (R == 32) dft32<S, Z>(v);
+    else if constexpr (R == 5 || R == 7) dft_prime<R, S, Z>(v);
     else static_assert(R == 2, "unsupported radix");
 }
 
@@ -338,14 +376,42 @@ template <int R, class C> PD_HD void twiddles(const C* tw, int e, C* w) {
 // a transform whose outputs outside it are discarded).
 template <int N, int KB> PD_HD bool in_band(int n) { return KB == 0 || n <= KB || n >= N - KB; }
 
+// Of a first pass of radix R (element n = j + r N / R, j < N / R) or a last pass (output n
+// likewise), round r lies outside the band for every j (0), below its upper edge (1), above its
+// lower edge (2), or either (3: decided per element).
+template <int N, int R, int KB> constexpr int band_round(int r) {
+    const int lo = r * (N / R), hi = lo + N / R - 1;
+    if (KB == 0) return 3;
+    if (lo > KB && hi < N - KB) return 0;
+    if (hi <= KB) return 1;
+    if (lo >= N - KB) return 2;
+    return 3;
+}
+template <int N, int R, int KB> constexpr unsigned zero_mask() {
+    unsigned z = 0;
+    for (int r = 0; r < R; r++) z |= (band_round<N, R, KB>(r) == 0 ? 1u : 0u) << r;
+    return z;
+}
+// The band class of a round as a type, for load and store functors of truncated transforms.
+template <int B> struct Band { static constexpr int value = B; };
+template <int I> struct RoundIx { static constexpr int value = I; };
+template <int I, int R, class F> PD_HD void for_rounds(F& f) {
+    if constexpr (I < R) {
+        f(RoundIx<I>{});
+        for_rounds<I + 1, R>(f);
+    }
+}
+
 template <int N, int R, int NS, int S, int L, int LP, int PS = 0, int AS = 0, int KB = 0, class C>
 PD_HD void pass_load(const C* s, const C* tw, int w, C* v) {
     using T = real_of<C>;
     constexpr int NR = N / R;
     const int l = w % L, j = w / L;
+    static_assert(KB == 0 || NS == 1, "a band of loads belongs to a first pass");
 #pragma unroll
     for (int r = 0; r < R; r++) {
-        if constexpr (KB > 0) v[r] = in_band<N, KB>(j + r * NR) ? s[tidx<LP, PS, AS>(j + r * NR, l)] : mk(T(0), T(0));
+        const int b = band_round<N, R, KB>(r);
+        if (KB > 0 && (b == 0 || (b == 3 && !in_band<N, KB>(j + r * NR)))) v[r] = mk(T(0), T(0));
         else v[r] = s[tidx<LP, PS, AS>(j + r * NR, l)];
     }
     if constexpr (NS > 1) {
@@ -356,16 +422,19 @@ PD_HD void pass_load(const C* s, const C* tw, int w, C* v) {
 #pragma unroll
         for (int r = 1; r < R; r++) v[r] = twmul<S>(v[r], wt[r]);
     }
-    dft<R, S>(v);
+    dft<R, S, zero_mask<N, R, KB>()>(v);
 }
 template <int N, int R, int NS, int L, int LP, int PS = 0, int AS = 0, int KB = 0, class C>
 PD_HD void pass_store(C* s, int w, const C* v) {
     const int l = w % L, j = w / L;
     const int k = j % NS;
     const int d = (j / NS) * NS * R + k;
+    static_assert(KB == 0 || NS * R == N, "a band of stores belongs to a last pass");
 #pragma unroll
-    for (int r = 0; r < R; r++)
-        if (in_band<N, KB>(d + r * NS)) s[tidx<LP, PS, AS>(d + r * NS, l)] = v[r];
+    for (int r = 0; r < R; r++) {
+        const int b = band_round<N, R, KB>(r);   // of a last pass: d < NS = N / R
+        if (KB == 0 || b == 1 || b == 2 || (b == 3 && in_band<N, KB>(d + r * NS))) s[tidx<LP, PS, AS>(d + r * NS, l)] = v[r];
+    }
 }
 
 // Transforms whose first pass reads global memory and whose last pass writes it
@@ -377,36 +446,56 @@ PD_HD void pass_store(C* s, int w, const C* v) {
 // The first pass takes element n of line l from ld(n, l); the last pass hands
 // output n of line l to st(n, l, value).  A two-pass length costs one shared-memory
 // round trip per element instead of four.
-template <int N, int R, int S, int L, class C, class Ld>
+// With KB > 0 (a truncated spectrum) ld and st are called as ld(n, l, Band<B>) and
+// st(n, l, value, Band<B>), B the class of the round (band_round): rounds outside the band are
+// neither loaded nor stored, and only B = 3 needs a test of n.
+template <int N, int R, int S, int L, int KB = 0, int PS = 0, class C, class Ld>
 PD_HD void pass_first(C* s, int w, Ld& ld) {
+    using T = real_of<C>;
     constexpr int NR = N / R;
     const int l = w % L, j = w / L;
     C v[R];
+    auto load = [&](auto ix) {
+        constexpr int r = decltype(ix)::value, b = band_round<N, R, KB>(r);
+        if constexpr (KB == 0) v[r] = ld(j + r * NR, l);
+        else if constexpr (b == 0) v[r] = mk(T(0), T(0));
+        else v[r] = ld(j + r * NR, l, Band<b>{});
+    };
+    for_rounds<0, R>(load);
+    dft<R, S, zero_mask<N, R, KB>()>(v);
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = ld(j + r * NR, l);
-    dft<R, S>(v);
-#pragma unroll
-    for (int r = 0; r < R; r++) s[(j * R + r) * L + l] = v[r];
+    for (int r = 0; r < R; r++) s[prow<PS>(j * R + r) * L + l] = v[r];
 }
-template <int N, int R, int S, int L, class C, class St>
+template <int N, int R, int S, int L, int KB = 0, int PS = 0, class C, class St>
 PD_HD void pass_last(const C* s, const C* tw, int w, St& st) {
     constexpr int NS = N / R;
     C v[R];
-    pass_load<N, R, NS, S, L, L, 0>(s, tw, w, v);
+    pass_load<N, R, NS, S, L, L, PS>(s, tw, w, v);
     const int l = w % L, j = w / L;
-#pragma unroll
-    for (int r = 0; r < R; r++) st(j + r * NS, l, v[r]);
+    auto store = [&](auto ix) {
+        constexpr int r = decltype(ix)::value, b = band_round<N, R, KB>(r);
+        if constexpr (KB == 0) st(j + r * NS, l, v[r]);
+        else if constexpr (b != 0) st(j + r * NS, l, v[r], Band<b>{});
+    };
+    for_rounds<0, R>(store);
 }
 // Single-pass lengths: global to global, no shared memory.
-template <int N, int S, int L, class Ld, class St>
+template <int N, int S, int L, int KF = 0, int KS = 0, class Ld, class St>
 PD_HD void pass_only(int l, Ld& ld, St& st) {
-    using C = decltype(ld(0, 0));
+    auto get = [&](int n) {
+        if constexpr (KF == 0) return ld(n, l);
+        else return ld(n, l, Band<3>{});
+    };
+    using C = decltype(get(0));
     C v[N];
 #pragma unroll
-    for (int r = 0; r < N; r++) v[r] = ld(r, l);
+    for (int r = 0; r < N; r++) v[r] = get(r);
     dft<N, S>(v);
 #pragma unroll
-    for (int r = 0; r < N; r++) st(r, l, v[r]);
+    for (int r = 0; r < N; r++) {
+        if constexpr (KS == 0) st(r, l, v[r]);
+        else st(r, l, v[r], Band<3>{});
+    }
 }
 
 // Threads per CTA of a direct tile transform of L = 8 lines: one item per thread
@@ -519,6 +608,26 @@ __device__ __forceinline__ void wpass(C* s, const C* __restrict__ tw, int lane) 
 // their own lines, `lane` being the lane within the group).
 template <int N, int R, int NS, int S, int LP, int PS, int NA, int AS = 0, int KL = 0, int KS = 0, int W = 32, class C>
 __device__ __forceinline__ void wpass_n(C* s, const C* __restrict__ tw, int lane) {
+    if constexpr (NA > 1 && AS > 0 && NS > 1 && N / R == W) {
+        // One item per lane and array: the arrays' items of a lane share their twiddles
+        // (their products are a sixth of an FP64 radix-16 pass).
+        C wt[R], v[NA][R];
+        twiddles<R>(tw, (lane % NS) * (N / (NS * R)), wt);
+#pragma unroll
+        for (int a = 0; a < NA; a++) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                v[a][r] = s[tidx<LP, PS, AS>(lane + r * W, a)];
+                if (r > 0) v[a][r] = twmul<S>(v[a][r], wt[r]);
+            }
+            dft<R, S>(v[a]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int a = 0; a < NA; a++) pass_store<N, R, NS, 1, LP, PS, 0, KS>(s + a * AS, lane, v[a]);
+        __syncwarp();
+        return;
+    }
     constexpr int WORK = (N / R) * NA;
     constexpr int IT = (WORK + W - 1) / W;
     C v[IT][R];
@@ -600,25 +709,26 @@ __device__ __forceinline__ void pass(C* s, const C* __restrict__ tw, int tid) {
 struct NoMid {
     __device__ void operator()() const {}
 };
+// KF, KS: band of the loads and of the stores (0: every element).
 template <int N, int S, int L, int NT, int R0 = Plan<N>::r0, int R1 = Plan<N>::r1, int R2 = Plan<N>::r2,
-          class C, class Ld, class St, class Mid = NoMid>
+          int KF = 0, int KS = 0, class C, class Ld, class St, class Mid = NoMid>
 __device__ __forceinline__ void fft_tile_io(C* s, const C* __restrict__ tw, int tid, Ld& ld, St& st,
                                             const Mid& mid = Mid()) {
     static_assert(R0 * (R1 ? R1 : 1) * (R2 ? R2 : 1) == N, "radix plan does not factor N");
     if constexpr (R1 == 0) {
         mid();
-        for (int l = tid; l < L; l += NT) pass_only<N, S, L>(l, ld, st);
+        for (int l = tid; l < L; l += NT) pass_only<N, S, L, KF, KS>(l, ld, st);
     } else {
         constexpr int W0 = (N / R0) * L;
 #pragma unroll
-        for (int w = tid; w < W0; w += NT) pass_first<N, R0, S, L>(s, w, ld);
+        for (int w = tid; w < W0; w += NT) pass_first<N, R0, S, L, KF>(s, w, ld);
         __syncthreads();
         mid();
         if constexpr (R2 != 0) pass<N, R1, R0, S, L, L, NT>(s, tw, tid);   // in place, ends with a barrier
         constexpr int RL = R2 ? R2 : R1;
         constexpr int WL = (N / RL) * L;
 #pragma unroll
-        for (int w = tid; w < WL; w += NT) pass_last<N, RL, S, L>(s, tw, w, st);
+        for (int w = tid; w < WL; w += NT) pass_last<N, RL, S, L, KS>(s, tw, w, st);
     }
 }
 #endif

@@ -38,12 +38,16 @@ extern __shared__ __align__(16) unsigned char pd_smem[];
 template <class C> __device__ __forceinline__ C* smem_as() { return reinterpret_cast<C*>(pd_smem); }
 
 
-// K3 holds three complex arrays per warp, so long lines get fewer warps per CTA.
+// Warps per CTA of K3 and the CTAs per SM asked of the register allocator.  One warp: no warp
+// waits on another, an SM's lines start and end at their own times (the loads of one run under
+// the butterflies of the others), and a line's shared memory is free as soon as it is done.
+// Against CTAs of 8 warps (4 above 512 points) the step of 512^3 shear took 22.3 instead of
+// 23.0 ms, 128^3 0.403 instead of 0.420, 160 x 96 x 112 0.383 instead of 0.399, 1024^3
+// FP32-mixed 100.2 instead of 101.0; 256^3 is level.  2 warps: between the two.
 template <int N> struct Cfg {
-    static constexpr int NWX = (N <= 512) ? 8 : 4;
-    // K3 CTAs per SM: shared memory allows 2 FP64 CTAs up to N = 256, FP32 twice that
+    static constexpr int NWX = 1;
     template <class T> static constexpr int minbx() {
-        return sizeof(T) == 8 ? ((N <= 256) ? 2 : 1) : ((N <= 256) ? 3 : (N <= 512 ? 2 : 1));
+        return sizeof(T) == 8 ? (N <= 256 ? 16 : (N <= 512 ? 8 : 4)) : (N <= 256 ? 24 : (N <= 512 ? 16 : 4));
     }
 };
 
@@ -664,10 +668,11 @@ template <int N, bool TWO = false> struct TCfg {
     template <class T> static unsigned tiles(const Geo& g) {
         return (unsigned)((g.nkip + lines<T>() - 1) / lines<T>());
     }
-    template <int S, int L, class C, class Ld, class St, class Mid = pdfft::NoMid>
+    // KF, KS: band of the loads and of the stores (pdfft::pass_first, pass_last)
+    template <int S, int L, int KF, int KS, class C, class Ld, class St, class Mid = pdfft::NoMid>
     static __device__ __forceinline__ void transform(C* s, const C* tw, Ld& ld, St& st, const Mid& mid = Mid()) {
         using T = pdfft::real_of<C>;
-        pdfft::fft_tile_io<N, S, L, nt<T>(), r0<T>(), r1<T>(), r2<T>()>(s, tw, threadIdx.x, ld, st, mid);
+        pdfft::fft_tile_io<N, S, L, nt<T>(), r0<T>(), r1<T>(), r2<T>(), KF, KS>(s, tw, threadIdx.x, ld, st, mid);
     }
 };
 
@@ -724,11 +729,12 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<T>(),
     if constexpr (SHEAR) {
         if (f >= 3) bf = bf_as<T>(make_bf(g, F.clock));
     }
-    auto ld = [&](int z, int l) -> C {
+    auto ld = [&](int z, int l, auto band) -> C {
+        constexpr int B = decltype(band)::value;
         const int i = i0 + l;
         int k;
-        if (z <= KK) k = z;
-        else if (z >= NZ - KK) k = z - NZ + NKK;
+        if (B == 1 || (B == 3 && z <= KK)) k = z;
+        else if (B == 2 || z >= NZ - KK) k = z - NZ + NKK;
         else return mk(T(0), T(0));
         if (i >= nki) return mk(T(0), T(0));
         const long long m = row0 + l * istride + k;
@@ -789,7 +795,7 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<T>(),
         const C* uc = c == 0 ? u0 : (c == 1 ? u1 : u2);
         if (i < nki) prefetch_l2(uc + ((long long)i * nkj + j2) * NKK, NKK * sizeof(C));
     };
-    TCfg<NZ>::template transform<+1, LT>(s, F.tw_z, ld, st, mid);
+    TCfg<NZ>::template transform<+1, LT, KK, 0>(s, F.tw_z, ld, st, mid);
 }
 
 // ---------------------------------------------------------------------------
@@ -896,10 +902,11 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<double>(), 1) k_zpass_in
     const long long zs = (long long)g.nkj * g.nkip;
 #pragma unroll 1
     for (int f = 0; f < nf; f++) {
-        auto ld = [&](int z, int l) -> C {
+        auto ld = [&](int z, int l, auto band) -> C {
+            constexpr int B = decltype(band)::value;
             int k;
-            if (z <= KK) k = z;
-            else if (z >= NZ - KK) k = z - NZ + (2 * KK + 1);
+            if (B == 1 || (B == 3 && z <= KK)) k = z;
+            else if (B == 2 || z >= NZ - KK) k = z - NZ + (2 * KK + 1);
             else return mk(0.0, 0.0);
             if constexpr (FORM == 3) {   // u_c, i k2 u_c, i k3 u_c (f_RK3Derivative, src/pf_rk3.f90:3735-3743)
                 const int c = f % 3;
@@ -936,7 +943,7 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<double>(), 1) k_zpass_in
         };
         C* dst = F.zb + (((long long)f * NZ) * g.nkj + j) * g.nkip + i0;
         auto st = [&](int z, int l, C v) { dst[z * zs + l] = v; };
-        TCfg<NZ>::template transform<+1, LT>(s, F.tw_z, ld, st);
+        TCfg<NZ>::template transform<+1, LT, KK, 0>(s, F.tw_z, ld, st);
         __syncthreads();   // the tile buffer is read by the last pass before the next field's first pass
     }
 }
@@ -965,17 +972,18 @@ __global__ void __launch_bounds__(TCfg<NY, true>::template nt<T>(), TCfg<NY, tru
     const long long rs = nkip_;
     const C* __restrict__ src = F.zb + (((long long)f * nz_ + z) * NKJ) * rs + i0;
     C* dst = F.yb + (((long long)f * nz_ + z) * NY) * rs + i0;
-    auto ld = [&](int y, int l) -> C {
+    auto ld = [&](int y, int l, auto band) -> C {
+        constexpr int B = decltype(band)::value;
         if (LT > 8 && l >= lmax) return mk(T(0), T(0));
-        if (y <= KJ) return src[y * rs + l];
-        if (y >= NY - KJ) return src[(y - NY + NKJ) * rs + l];
+        if (B == 1 || (B == 3 && y <= KJ)) return src[y * rs + l];
+        if (B == 2 || y >= NY - KJ) return src[(y - NY + NKJ) * rs + l];
         return mk(T(0), T(0));
     };
     auto st = [&](int y, int l, C v) {
         if (LT > 8 && l >= lmax) return;
         dst[y * rs + l] = v;
     };
-    TCfg<NY, true>::template transform<+1, LT>(s, F.tw_y, ld, st);
+    TCfg<NY, true>::template transform<+1, LT, KJ, 0>(s, F.tw_y, ld, st);
 }
 
 // K4: forward y transforms of NL field f = blockIdx.z, truncated to j
@@ -1004,12 +1012,13 @@ __global__ void __launch_bounds__(TCfg<NY, true>::template nt<T>(), TCfg<NY, tru
         if (LT > 8 && l >= lmax) return mk(T(0), T(0));
         return src[y * rs + l];
     };
-    auto st = [&](int y, int l, C v) {
+    auto st = [&](int y, int l, C v, auto band) {
+        constexpr int B = decltype(band)::value;
         if (LT > 8 && l >= lmax) return;
-        if (y <= KJ) dst[y * rs + l] = v;
-        else if (y >= NY - KJ) dst[(y - NY + NKJ) * rs + l] = v;
+        if (B == 1 || (B == 3 && y <= KJ)) dst[y * rs + l] = v;
+        else if (B == 2 || y >= NY - KJ) dst[(y - NY + NKJ) * rs + l] = v;
     };
-    TCfg<NY, true>::template transform<-1, LT>(s, F.tw_y, ld, st);
+    TCfg<NY, true>::template transform<-1, LT, 0, KJ>(s, F.tw_y, ld, st);
 }
 
 // K5a: forward z transforms of NL field f = blockIdx.z, x 1/(NX NY NZ), truncated
@@ -1031,7 +1040,8 @@ __global__ void __launch_bounds__(TCfg<NZ, true>::template nt<T>(), TCfg<NZ, tru
     // NL-hat into the y-pencil buffer, or (mode 1) into rk
     Out3<C> nlh;
     for (int c = 0; c < 3; c++) nlh.p[c] = (mode == 1) ? F.rk[c] : F.yb + c * g.S;
-    const int KK = g.kk, NKK = g.nkk, nki = g.nki;
+    constexpr int KK = NZ / 3, NKK = 2 * KK + 1;   // g.kk, g.nkk (the 2/3 rule)
+    const int nki = g.nki;
     const long long zs = (long long)g.nkj * g.nkip;
     const C* __restrict__ src = F.zb + (((long long)f * NZ) * g.nkj + j) * g.nkip + i0;
     C* dst = (f == 0 ? nlh.p[0] : (f == 1 ? nlh.p[1] : nlh.p[2])) + ((long long)i0 * g.nkj + j) * NKK;
@@ -1041,15 +1051,16 @@ __global__ void __launch_bounds__(TCfg<NZ, true>::template nt<T>(), TCfg<NZ, tru
         if (LT > 8 && l >= lmax) return mk(T(0), T(0));
         return src[z * zs + l];
     };
-    auto st = [&](int z, int l, C v) {
+    auto st = [&](int z, int l, C v, auto band) {
+        constexpr int B = decltype(band)::value;
         if (i0 + l >= nki) return;
         int k;
-        if (z <= KK) k = z;
-        else if (z >= NZ - KK) k = z - NZ + NKK;
+        if (B == 1 || (B == 3 && z <= KK)) k = z;
+        else if (B == 2 || z >= NZ - KK) k = z - NZ + NKK;
         else return;
         dst[l * istride + k] = mk(v.x * norm, v.y * norm);
     };
-    TCfg<NZ, true>::template transform<-1, LT>(s, F.tw_z, ld, st);
+    TCfg<NZ, true>::template transform<-1, LT, 0, KK>(s, F.tw_z, ld, st);
 }
 
 
