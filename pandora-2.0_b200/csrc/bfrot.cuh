@@ -46,77 +46,49 @@ template <class R> __device__ __forceinline__ BFT<R> bf_as(const BF& f) {
     return r;
 }
 
-// f_RK3VorticityBFRot (src/pf_rk3.f90:3786-3843), summed over the three velocity
-// components: w = sum_n omega(u_n).  Structurally w[0] has no term in u[0] and
-// w[1] none in u[1] (bex), so a caller that needs only w[0] or w[1] may pass zero
-// for that component.
-// ONLY >= 0: only component ONLY of w is formed (the others are left zero).
-template <int ONLY = -1, class R, class C>
-__device__ __forceinline__ void vort_bf(const BFT<R>& f, const C* u, const R* k, C* w) {
-    w[0].x = R(0); w[0].y = R(0); w[1] = w[0]; w[2] = w[0];
-#pragma unroll
-    for (int n = 0; n < 3; n++) {
-        const C un = u[n];
-#pragma unroll
-        for (int m = 0; m < 3; m++) {
-            if (bex(m, 0)) {
-                if ((ONLY < 0 || ONLY == 1) && bex(2, n)) { const R c = f.bm[m][0] * f.bi[2][n] * k[m]; w[1].y -= c * un.x; w[1].x += c * un.y; }
-                if ((ONLY < 0 || ONLY == 2) && bex(1, n)) { const R c = f.bm[m][0] * f.bi[1][n] * k[m]; w[2].y += c * un.x; w[2].x -= c * un.y; }
-            }
-            if (bex(m, 1)) {
-                if ((ONLY < 0 || ONLY == 0) && bex(2, n)) { const R c = f.bm[m][1] * f.bi[2][n] * k[m]; w[0].y += c * un.x; w[0].x -= c * un.y; }
-                if ((ONLY < 0 || ONLY == 2) && bex(0, n)) { const R c = f.bm[m][1] * f.bi[0][n] * k[m]; w[2].y -= c * un.x; w[2].x += c * un.y; }
-            }
-            if (bex(m, 2)) {
-                if ((ONLY < 0 || ONLY == 0) && bex(1, n)) { const R c = f.bm[m][2] * f.bi[1][n] * k[m]; w[0].y -= c * un.x; w[0].x += c * un.y; }
-                if ((ONLY < 0 || ONLY == 1) && bex(0, n)) { const R c = f.bm[m][2] * f.bi[0][n] * k[m]; w[1].y += c * un.x; w[1].x -= c * un.y; }
-            }
-        }
+// One vorticity component of one (k1, k2) line as a linear form in the stored velocity:
+// omega = i [ (aA + bA k3) u_A + (aB + bB k3) u_B + aC u_C ].  omega = D x v with the
+// wave vector D = (bmat(1,1) k1, bmat(2,2) k2, bmat(1,3) k1 + bmat(3,3) k3) of the moving grid
+// (d/dx_j = i sum_m bmat(m,j) k_m) and the laboratory velocity v:
+//   FORM 0  isotropic: D = k, v = u (src/pf_rk3.f90:402-407,520-525,630-634);
+//   FORM 1  BF-rot: v = binv u (f_RK3VorticityBFRot, src/pf_rk3.f90:3786-3843);
+//   FORM 2  R-rot: v = u (f_RK3DerivativeRRot, src/pf_rk3.f90:3749-3780, 416-421, 470-475, 585-590).
+// A, B, C are components 2, 3 (omega 1), 1, 3 (omega 2) and 1, 2, 3 (omega 3; C in BF-rot
+// only).  The coefficients are formed once per line, so that a mode costs a fused multiply-add
+// and two per component, and a kernel over the components holds five numbers instead of the
+// frame tensors (K1's staged form spilled 64 bytes with them).
+template <class R> struct VortLine {
+    R aA, bA, aB, bB, aC;
+};
+template <int FORM, class R>
+__device__ __forceinline__ VortLine<R> vort_line(const BFT<R>& f, int comp, R k1, R k2) {
+    const R d1 = FORM == 0 ? k1 : f.bm[0][0] * k1, d2 = FORM == 0 ? k2 : f.bm[1][1] * k2;
+    const R d3a = FORM == 0 ? R(0) : f.bm[0][2] * k1, d3b = FORM == 0 ? R(1) : f.bm[2][2];   // D3 = d3a + d3b k3
+    const R i0 = FORM == 1 ? f.bi[0][0] : R(1), i1 = FORM == 1 ? f.bi[1][1] : R(1), i2 = FORM == 1 ? f.bi[2][2] : R(1);
+    const R i02 = FORM == 1 ? f.bi[0][2] : R(0);
+    VortLine<R> v;
+    v.aC = R(0);
+    if (comp == 0) {          // D2 v3 - D3 v2
+        v.aA = -d3a * i1; v.bA = -d3b * i1;
+        v.aB = d2 * i2; v.bB = R(0);
+    } else if (comp == 1) {   // D3 v1 - D1 v3
+        v.aA = d3a * i0; v.bA = d3b * i0;
+        v.aB = d3a * i02 - d1 * i2; v.bB = d3b * i02;
+    } else {                  // D1 v2 - D2 v1
+        v.aA = -d2 * i0; v.bA = R(0);
+        v.aB = d1 * i1; v.bB = R(0);
+        v.aC = -d2 * i02;
     }
+    return v;
 }
-
-// R-rot form (NS_DEFORMED = NS_R_ROT): the velocity components are laboratory ones on
-// the sheared wavenumber grid.  f_RK3DerivativeRRot (src/pf_rk3.f90:3749-3780):
-// d/dx_j = i sum_m bmat(m,j) k_m over every m; the vorticity w = D x u assembled per
-// velocity component as the reference does (src/pf_rk3.f90:416-421, 470-475, 585-590).
-template <class R, class C>
-__device__ __forceinline__ C deriv_rrot(const BFT<R>& f, C u, const R* k, int j) {
-    C d;
-    d.x = R(0); d.y = R(0);
-#pragma unroll
-    for (int m = 0; m < 3; m++) {
-        d.y = d.y + (f.bm[m][j] * k[m] * u.x);
-        d.x = d.x - (f.bm[m][j] * k[m] * u.y);
-    }
-    return d;
-}
-// ONLY >= 0: only component ONLY of w is formed, from its two derivatives (the others
-// are left zero); the same operations in the same order as for all three.
-template <int ONLY = -1, class R, class C>
-__device__ __forceinline__ void vort_rrot(const BFT<R>& f, const C* u, const R* k, C* w) {
-    constexpr bool A0 = ONLY < 0 || ONLY == 0, A1 = ONLY < 0 || ONLY == 1, A2 = ONLY < 0 || ONLY == 2;
-    w[0].x = R(0); w[0].y = R(0); w[1] = w[0]; w[2] = w[0];
-    if constexpr (A1) w[1] = deriv_rrot(f, u[0], k, 2);
-    if constexpr (A2) {
-        const C dudy = deriv_rrot(f, u[0], k, 1);
-        w[2].x = -dudy.x; w[2].y = -dudy.y;
-    }
-    if constexpr (A0) {
-        const C dvdz = deriv_rrot(f, u[1], k, 2);
-        w[0].x = w[0].x - dvdz.x; w[0].y = w[0].y - dvdz.y;
-    }
-    if constexpr (A2) {
-        const C dvdx = deriv_rrot(f, u[1], k, 0);
-        w[2].x = w[2].x + dvdx.x; w[2].y = w[2].y + dvdx.y;
-    }
-    if constexpr (A0) {
-        const C dwdy = deriv_rrot(f, u[2], k, 1);
-        w[0].x = w[0].x + dwdy.x; w[0].y = w[0].y + dwdy.y;
-    }
-    if constexpr (A1) {
-        const C dwdx = deriv_rrot(f, u[2], k, 0);
-        w[1].x = w[1].x - dwdx.x; w[1].y = w[1].y - dwdx.y;
-    }
+// c: u_C, or null where the component has none
+template <class R, class C> __device__ __forceinline__ C vort_mode(const VortLine<R>& v, R k3, C a, C b, const C* c) {
+    const R ca = v.aA + v.bA * k3, cb = v.aB + v.bB * k3;
+    C w;
+    w.x = -ca * a.y - cb * b.y;
+    w.y = ca * a.x + cb * b.x;
+    if (c) { w.x -= v.aC * c->y; w.y += v.aC * c->x; }
+    return w;
 }
 
 // f_RK3FormFRRot for F_SHEAR_DNS (src/pf_rk3.f90:2680-2856): viscous (f_RK3RRotViscous)

@@ -336,11 +336,14 @@ template <int N> constexpr bool plan_ok() {
     return Plan<N>::r0 * (Plan<N>::r1 ? Plan<N>::r1 : 1) * (Plan<N>::r2 ? Plan<N>::r2 : 1) == N;
 }
 
-// Row of element n in a tile: with PS > 0 one pad row follows every 2^PS rows,
-// which spreads the stride-R stores of the first passes over distinct banks
-// when a warp owns a single line.
-template <int PS> PD_HD int prow(int n) { return PS > 0 ? n + (n >> PS) : n; }
-template <int N, int PS> constexpr int tile_rows() { return PS > 0 ? N + (N >> PS) : N; }
+// Row of element n in a tile: with PS = a > 0 one pad row follows every 2^a rows, with
+// PS = a + 16 b another every 2^b rows, which spreads the stores of the passes, of stride the
+// radix, over distinct banks when a warp owns whole lines.  (Shifts of n, not an exclusive-or
+// swizzle: n = j + r N / R then keeps a compile-time offset per r.)
+template <int PS> PD_HD constexpr int prow(int n) {
+    return PS <= 0 ? n : (PS < 16 ? n + (n >> PS) : n + (n >> (PS & 15)) + (n >> (PS >> 4)));
+}
+template <int N, int PS> constexpr int tile_rows() { return prow<PS>(N - 1) + 1; }
 
 // One pass, split into a load/compute half and a store half so that a CPU
 // emulator can run all items' first halves before any second half (that is
@@ -350,6 +353,12 @@ template <int N, int PS> constexpr int tile_rows() { return PS > 0 ? N + (N >> P
 template <int LP, int PS, int AS> PD_HD int tidx(int n, int l) {
     return AS ? l * AS + prow<PS>(n) : prow<PS>(n) * LP + l;
 }
+
+// Line and index of item w of a pass with NR items per line: the lines of a tile interleave
+// (neighbouring items are one butterfly of neighbouring lines); separate arrays that share a
+// warp's lanes (NR <= 16) follow one another, so that the lanes of a wavefront stay in one.
+template <int NR, int L, int AS> PD_HD int item_line(int w) { return AS && NR <= 16 ? w / NR : w % L; }
+template <int NR, int L, int AS> PD_HD int item_index(int w) { return AS && NR <= 16 ? w % NR : w / L; }
 
 // Twiddles w[r] = tw[r e] (r = 1..R-1) of one butterfly: the entries at power-of-two
 // multiples r = 2^a are read from the table (log2 R loads), the others are products
@@ -406,7 +415,7 @@ template <int N, int R, int NS, int S, int L, int LP, int PS = 0, int AS = 0, in
 PD_HD void pass_load(const C* s, const C* tw, int w, C* v) {
     using T = real_of<C>;
     constexpr int NR = N / R;
-    const int l = w % L, j = w / L;
+    const int l = item_line<NR, L, AS>(w), j = item_index<NR, L, AS>(w);
     static_assert(KB == 0 || NS == 1, "a band of loads belongs to a first pass");
 #pragma unroll
     for (int r = 0; r < R; r++) {
@@ -426,7 +435,7 @@ PD_HD void pass_load(const C* s, const C* tw, int w, C* v) {
 }
 template <int N, int R, int NS, int L, int LP, int PS = 0, int AS = 0, int KB = 0, class C>
 PD_HD void pass_store(C* s, int w, const C* v) {
-    const int l = w % L, j = w / L;
+    const int l = item_line<N / R, L, AS>(w), j = item_index<N / R, L, AS>(w);
     const int k = j % NS;
     const int d = (j / NS) * NS * R + k;
     static_assert(KB == 0 || NS * R == N, "a band of stores belongs to a last pass");
@@ -498,15 +507,23 @@ PD_HD void pass_only(int l, Ld& ld, St& st) {
     }
 }
 
+// Pad interval (log2) of a tile whose rows (one element of every line) are ROWB bytes, after a
+// first pass of radix R0.  Rows of 128 bytes need none.  With shorter rows a wavefront of a store
+// of the first pass holds several butterflies' rows, R0 rows apart: for an even R0 in the same
+// banks, unless a pad row lies between them.
+template <int ROWB, int R0> constexpr int tile_pad() {
+    return (ROWB >= 128 || R0 % 2 != 0) ? 0 : (R0 == 8 ? 3 : (R0 == 16 ? 4 : (R0 == 32 ? 5 : (R0 == 4 ? 2 : 0))));
+}
+
 // Threads per CTA of a direct tile transform of L = 8 lines: one item per thread
 // in the widest pass, at most 512.
-// Threads of a tile transform of 8 lines with the radix plan (R0, R1, R2): one
+// Threads of a tile transform of L lines with the radix plan (R0, R1, R2): one
 // butterfly per thread in the pass with the most, 64..512.
-template <int N, int R0, int R1, int R2> constexpr int tile_threads_for() {
+template <int N, int R0, int R1, int R2, int L = 8> constexpr int tile_threads_for() {
     constexpr int a = N / R0;
     constexpr int b = R1 ? N / R1 : 0;
     constexpr int c = R2 ? N / R2 : 0;
-    constexpr int m = 8 * (a > b ? (a > c ? a : c) : (b > c ? b : c));
+    constexpr int m = L * (a > b ? (a > c ? a : c) : (b > c ? b : c));
     return m < 64 ? 64 : (m > 512 ? 512 : m);
 }
 template <int N> constexpr int tile_threads() { return tile_threads_for<N, Plan<N>::r0, Plan<N>::r1, Plan<N>::r2>(); }
@@ -682,7 +699,7 @@ __device__ __forceinline__ void fft_warp(C* s, const C* __restrict__ tw, int lan
 }
 
 // In-place pass over a [N][LP] shared tile with NT threads; items w = tid + it*NT.
-template <int N, int R, int NS, int S, int L, int LP, int NT, class C>
+template <int N, int R, int NS, int S, int L, int LP, int NT, int PS = 0, class C>
 __device__ __forceinline__ void pass(C* s, const C* __restrict__ tw, int tid) {
     constexpr int WORK = (N / R) * L;
     constexpr int IT = (WORK + NT - 1) / NT;
@@ -690,13 +707,13 @@ __device__ __forceinline__ void pass(C* s, const C* __restrict__ tw, int tid) {
 #pragma unroll
     for (int it = 0; it < IT; it++) {
         const int w = tid + it * NT;
-        if (WORK % NT == 0 || w < WORK) pass_load<N, R, NS, S, L, LP>(s, tw, w, v[it]);
+        if (WORK % NT == 0 || w < WORK) pass_load<N, R, NS, S, L, LP, PS>(s, tw, w, v[it]);
     }
     __syncthreads();
 #pragma unroll
     for (int it = 0; it < IT; it++) {
         const int w = tid + it * NT;
-        if (WORK % NT == 0 || w < WORK) pass_store<N, R, NS, L, LP>(s, w, v[it]);
+        if (WORK % NT == 0 || w < WORK) pass_store<N, R, NS, L, LP, PS>(s, w, v[it]);
     }
     __syncthreads();
 }
@@ -709,9 +726,10 @@ __device__ __forceinline__ void pass(C* s, const C* __restrict__ tw, int tid) {
 struct NoMid {
     __device__ void operator()() const {}
 };
-// KF, KS: band of the loads and of the stores (0: every element).
+// KF, KS: band of the loads and of the stores (0: every element).  PS: one pad row after every
+// 2^PS rows (tile_pad).
 template <int N, int S, int L, int NT, int R0 = Plan<N>::r0, int R1 = Plan<N>::r1, int R2 = Plan<N>::r2,
-          int KF = 0, int KS = 0, class C, class Ld, class St, class Mid = NoMid>
+          int KF = 0, int KS = 0, int PS = 0, class C, class Ld, class St, class Mid = NoMid>
 __device__ __forceinline__ void fft_tile_io(C* s, const C* __restrict__ tw, int tid, Ld& ld, St& st,
                                             const Mid& mid = Mid()) {
     static_assert(R0 * (R1 ? R1 : 1) * (R2 ? R2 : 1) == N, "radix plan does not factor N");
@@ -721,14 +739,14 @@ __device__ __forceinline__ void fft_tile_io(C* s, const C* __restrict__ tw, int 
     } else {
         constexpr int W0 = (N / R0) * L;
 #pragma unroll
-        for (int w = tid; w < W0; w += NT) pass_first<N, R0, S, L, KF>(s, w, ld);
+        for (int w = tid; w < W0; w += NT) pass_first<N, R0, S, L, KF, PS>(s, w, ld);
         __syncthreads();
         mid();
-        if constexpr (R2 != 0) pass<N, R1, R0, S, L, L, NT>(s, tw, tid);   // in place, ends with a barrier
+        if constexpr (R2 != 0) pass<N, R1, R0, S, L, L, NT, PS>(s, tw, tid);   // in place, ends with a barrier
         constexpr int RL = R2 ? R2 : R1;
         constexpr int WL = (N / RL) * L;
 #pragma unroll
-        for (int w = tid; w < WL; w += NT) pass_last<N, RL, S, L, KS>(s, tw, w, st);
+        for (int w = tid; w < WL; w += NT) pass_last<N, RL, S, L, KS, PS>(s, tw, w, st);
     }
 }
 #endif

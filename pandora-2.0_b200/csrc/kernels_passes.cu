@@ -127,11 +127,11 @@ typedef CUresult (*TensorMapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuui
 
 cudaError_t make_zmaps(const Geo& g, double2* const* u, ZMaps* out, bool* ok) {
     *ok = false;
-    int bk = 0;
+    int bk = 0, lines = 0;
     switch (g.nz) {
-#define PD_L(N)                                               \
-    case N:                                                   \
-        if constexpr (ZStage<N>::enabled) bk = ZStage<N>::BK; \
+#define PD_L(N)                                                                            \
+    case N:                                                                                \
+        if constexpr (ZStage<N>::enabled) { bk = ZStage<N>::BK; lines = ZStage<N>::lines; } \
         break;
         PD_FOR_EACH_N(PD_L)
 #undef PD_L
@@ -153,7 +153,7 @@ cudaError_t make_zmaps(const Geo& g, double2* const* u, ZMaps* out, bool* ok) {
     const cuuint64_t dims[3] = {(cuuint64_t)2 * g.nkk, (cuuint64_t)g.nkj, (cuuint64_t)g.nki};
     const cuuint64_t strides[2] = {(cuuint64_t)2 * g.nkk * sizeof(double),
                                    (cuuint64_t)2 * g.nkk * g.nkj * sizeof(double)};
-    const cuuint32_t box[3] = {(cuuint32_t)(2 * bk), 1u, 8u};
+    const cuuint32_t box[3] = {(cuuint32_t)(2 * bk), 1u, (cuuint32_t)lines};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     for (int c = 0; c < 3; c++) {
         if (encode(&out->u[c], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, (void*)u[c], dims, strides, box, estr,

@@ -230,7 +230,7 @@ template <class T, class Fn> inline cudaError_t for_member_sets(const Member<T>*
 // type, common to its members), M a host array of its B member descriptors
 // (passed by value to the kernels, kBatchChunk members per launch).
 // Tensor maps of the three FP64 velocity components in the [i][j][k] layout (dims k as
-// 2 NKK doubles, j, i; boxes of BK k x 1 j x 8 i), for the K1 whose velocity rows are
+// 2 NKK doubles, j, i; boxes of BK k x 1 j x 4 i), for the K1 whose velocity rows are
 // staged by tensor copies.
 struct ZMaps {
     CUtensorMap u[3];

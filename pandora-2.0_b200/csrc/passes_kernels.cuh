@@ -38,18 +38,11 @@ extern __shared__ __align__(16) unsigned char pd_smem[];
 template <class C> __device__ __forceinline__ C* smem_as() { return reinterpret_cast<C*>(pd_smem); }
 
 
-// Warps per CTA of K3 and the CTAs per SM asked of the register allocator.  One warp: no warp
-// waits on another, an SM's lines start and end at their own times (the loads of one run under
-// the butterflies of the others), and a line's shared memory is free as soon as it is done.
-// Against CTAs of 8 warps (4 above 512 points) the step of 512^3 shear took 22.3 instead of
-// 23.0 ms, 128^3 0.403 instead of 0.420, 160 x 96 x 112 0.383 instead of 0.399, 1024^3
-// FP32-mixed 100.2 instead of 101.0; 256^3 is level.  2 warps: between the two.
-template <int N> struct Cfg {
-    static constexpr int NWX = 1;
-    template <class T> static constexpr int minbx() {
-        return sizeof(T) == 8 ? (N <= 256 ? 16 : (N <= 512 ? 8 : 4)) : (N <= 256 ? 24 : (N <= 512 ? 16 : 4));
-    }
-};
+// K3 runs one warp per CTA: no warp waits on another, an SM's lines start and end at their own
+// times (the loads of one run under the butterflies of the others), and a line's shared memory
+// is free as soon as it is done.  Against CTAs of 8 warps (4 above 512 points) the step of 512^3
+// shear took 22.3 instead of 23.0 ms, 128^3 0.403 instead of 0.420, 160 x 96 x 112 0.383
+// instead of 0.399, 1024^3 FP32-mixed 100.2 instead of 101.0; 256^3 is level.
 
 // Transform lengths built: 2^a x {1, 3, 5, 7} from 16 to 1024 (the reference's rule,
 // src/pg_domain.f90:274-292), each a radix plan of at most three passes.
@@ -68,14 +61,11 @@ template <int N> struct Cfg {
 // truncated to i = 0..KI (src/pf_fftw.f90:780).  NL overwrites yb fields 0..2 of
 // the same line.  Optionally writes the physical velocity (arr_u*_3r,
 // src/pf_rk3.f90:1108-1115) and the CFL maximum (src/pf_fluidstats.f90:913-917).
-// Warp shared region: three arrays XAS elements apart (XAS = 4 mod 8 in 16-byte
-// units), element n of array p at s[p*XAS + prow<XPS>(n)].  Up to N = 512 the
-// warp transforms arrays 0 and 1 in lockstep (a radix-16 or radix-32 pass of one
-// array leaves lanes idle); with the offset of 4 bank groups between the two
-// arrays and XPS chosen per length, those passes are free of bank conflicts.
-// The warp plans are two passes up to N = 1024 (radix 32 at 512 and 1024): the
-// kernel is bound by shared-memory wavefronts, and each pass is a full read and
-// write of the three arrays.
+// Shared region of a line: three arrays XC::as elements apart, element n of array p at
+// s[p*as + prow<ps>(n)], the pads chosen per length.  Up to N = 512 arrays 0 and 1 go through a
+// pass in lockstep where one array leaves lanes idle.  The warp plans are two passes up to
+// N = 1024 (radix 32 at 512 and 1024): the kernel is bound by shared-memory wavefronts, and
+// each pass through shared memory is a full read and write of the arrays.
 // ---------------------------------------------------------------------------
 // Bulk prefetch of [p, p + bytes) into L2 (a hint: no data moves to the SM),
 // trimmed inward to the 16-byte boundaries the bulk copy requires.
@@ -91,6 +81,49 @@ template <int N> constexpr int xps() {
          : ((N == 24 || N == 64 || N == 96) ? 3 : ((N == 384 || N == 512 || N == 1024) ? 5 : 4));
 }
 template <int N> constexpr int xas() { return (tile_rows<N, xps<N>()>() + 7) / 8 * 8 + 4; }
+
+// Schedule of the x pass at length N.
+template <int N, class T> struct XCfg {
+    using FP = pdfft::FusedPlan<N>;
+    static constexpr int w32 = (int)sizeof(T) / 4;   // registers per real
+    // `triple`: the last backward pass of all three arrays, the product and the first forward
+    // pass of the two product arrays run in registers, one butterfly of each array per lane, so
+    // that the physical fields never pass through shared memory (a sixth of the pass's shared
+    // wavefronts, which bound it: 68% of the L1 data pipe's rate at 512 points with the FP64 pipe
+    // at 48%).  Wants a line's butterflies on one warp and 3 R complex values a lane in registers.
+    // Per stage, with the physical fields through shared memory and so: 128^3 FP64 0.058 -> 0.037
+    // ms, 256^3 0.312 -> 0.278 (FP32-mixed 0.183 -> 0.140), 512^3 2.52 -> 2.47 (1.28 -> 1.10),
+    // 1024^3 FP32-mixed 10.4 -> 10.0; 32 batched members of 32^3 118 -> 128 thousand
+    // member-steps/s, 16 of 64^3 22.1 -> 24.8.
+    static constexpr bool triple = FP::nrl <= 32 && 6 * FP::rl * w32 <= 192;
+    // lines per warp, so that a short line's butterflies fill the lanes
+    static constexpr int lpw = !triple ? 1 : (FP::nrl <= 8 ? 4 : (FP::nrl <= 16 ? 2 : 1));
+    // Pads per length: the fewest wavefronts of all accesses of the pass, counted over quarter
+    // (FP64) or half warps (FP32) with this lane mapping.
+    static constexpr int pad64() {
+        return N == 16 ? 2 : N == 48 ? 3 + 16 * 5 : (N == 56 || N == 112 || N == 224 || N == 256) ? 4
+             : N == 80 ? 3 + 16 * 4 : N == 128 ? 3 + 16 * 6 : (N == 192 || N == 512) ? 4 + 16 * 7 : N == 384 ? 5 : 3;
+    }
+    static constexpr int pad32() {
+        return N == 16 ? 2 : N == 48 ? 3 + 16 * 5 : (N == 56 || N == 112 || N == 128 || N == 256) ? 4
+             : N == 80 ? 3 + 16 * 4 : N == 192 ? 4 + 16 * 6 : N == 512 ? 4 + 16 * 8
+             : (N == 160 || N == 224 || N == 384 || N == 1024) ? 5 : 3;
+    }
+    static constexpr int ps = !triple ? xps<N>() : (sizeof(T) == 8 ? pad64() : pad32());
+    static constexpr int q = sizeof(T) == 8 ? 8 : 16;
+    static constexpr int as = !triple ? xas<N>() : (tile_rows<N, ps>() + q - 1) / q * q;   // distance of the arrays
+    template <int LPW> static constexpr int ls() { return 3 * as + (triple && LPW == 4 && sizeof(T) == 4 ? 8 : 0); }   // of the lines of a warp
+    // CTAs (warps) per SM asked of the register allocator: 4 warps a step, since a register file
+    // partition's registers are shared by a quarter of them (8: 255 a thread, 12: 168, 16: 128,
+    // 20: 96, 24: 80)
+    static constexpr int ctas() {
+        if (!triple) return sizeof(T) == 8 ? (N <= 256 ? 16 : (N <= 512 ? 8 : 4)) : (N <= 256 ? 24 : (N <= 512 ? 16 : 4));
+        constexpr int r = FP::rl, r0 = FP::r0;
+        if (sizeof(T) == 8) return r >= 12 || r0 == 32 ? 8 : 12;
+        return r == 32 ? 8 : (r >= 12 || r0 == 32 ? 16 : 20);
+    }
+};
+
 // arrays transformed in lockstep: 2 while a lane's items of a pass fit its registers
 template <int N> constexpr int xna() { return N <= 512 ? 2 : 1; }
 
@@ -136,12 +169,21 @@ __device__ __forceinline__ void rs_point(double* acc, double* mx, bool shear, co
     mx[1] = fmax(mx[1], fabs(w1)); mx[2] = fmax(mx[2], fabs(w2)); mx[3] = fmax(mx[3], fabs(w3));
 }
 
+// The statistics pass keeps the physical fields in shared memory (its moments hold the registers).
+template <int N, class T> struct XCfgStats {
+    using FP = pdfft::FusedPlan<N>;
+    static constexpr bool triple = false;
+    static constexpr int ps = xps<N>(), as = xas<N>();
+    template <int LPW> static constexpr int ls() { return 3 * as; }
+    static constexpr int ctas() { return sizeof(T) == 8 ? (N <= 256 ? 16 : (N <= 512 ? 8 : 4)) : (N <= 256 ? 24 : (N <= 512 ? 16 : 4)); }
+};
+
 // RS: the real-space statistics pass (the same transforms, plus the moments of every
 // point, reduced per warp into one of kRsSlots copies of the sums in `rs`).
 // LPW: lines per warp (LPW > 1 for short, unfused lines: each group of 32 / LPW lanes
 // transforms its own line).
 template <int NX, class T, int CAP, bool RS = false, int LPW = 1>
-__global__ void __launch_bounds__(32 * Cfg<NX>::NWX, Cfg<NX>::template minbx<T>()) k_xpass(const __grid_constant__ MemberSet<T, CAP> ms,
+__global__ void __launch_bounds__(32, RS ? XCfgStats<NX, T>::ctas() : XCfg<NX, T>::ctas()) k_xpass(const __grid_constant__ MemberSet<T, CAP> ms,
                                                                                         int want_phys,
                                                                                         int want_cfl,
                                                                                         long long pf_lines,
@@ -155,20 +197,22 @@ __global__ void __launch_bounds__(32 * Cfg<NX>::NWX, Cfg<NX>::template minbx<T>(
     }
     const FieldsT<T> F = mm.F;
     const Geo g = mm.g;
-    constexpr int XPS = xps<NX>(), XAS = xas<NX>(), NA = xna<NX>();
+    using XC = std::conditional_t<RS, XCfgStats<NX, T>, XCfg<NX, T>>;
+    constexpr bool TRIPLE = XC::triple;
+    constexpr int XPS = XC::ps, XAS = XC::as, NA = xna<NX>();
     constexpr int KB = NX / 3;   // the kept band of the x spectrum, i <= KI
-    static_assert(LPW == 1 || (!XP::fused && !RS), "several lines per warp: unfused plans, no statistics");
+    static_assert(LPW == 1 || TRIPLE, "several lines per warp: the triple schedule");
     constexpr int W = 32 / LPW;  // lanes per line
     C* smem = smem_as<C>();
-    const int tid = threadIdx.x, lane = (tid & 31) % W, sub = (tid & 31) / W, w = tid >> 5;
+    const int tid = threadIdx.x, lane = tid % W, sub = tid / W;
     const long long lines = (long long)g.ny * g.nz;
     const C* tw = F.tw_x;
-    const long long qw = ((long long)blockIdx.x * Cfg<NX>::NWX + w) * LPW;   // the warp's first line
-    if (qw >= lines) return;                      // whole warp; no block barrier follows
+    const long long qw = (long long)blockIdx.x * LPW;   // the warp's first line
+    if (qw >= lines) return;
     // a group past the last line transforms the last line again and stores nothing
     const bool valid = qw + sub < lines;
     const long long q = valid ? qw + sub : lines - 1;
-    C* s = smem + ((size_t)w * LPW + sub) * 3 * XAS;
+    C* s = smem + (size_t)sub * XC::template ls<LPW>();
     constexpr int NKI = NX / 3 + 1, NKIP = (NKI + 7) / 8 * 8;   // g.nki, g.nkip
     const long long fstride = lines * NKIP;       // distance between fields in yb
     C* b = F.yb + q * NKIP;
@@ -227,14 +271,52 @@ __global__ void __launch_bounds__(32 * Cfg<NX>::NWX, Cfg<NX>::template minbx<T>(
     }
     __syncwarp();
     constexpr int R0 = XP::r0, R1 = XP::r1, R2 = XP::r2, NP = XP::np;
-    if constexpr (NA == 2) {
-        pdfft::wpasses<NX, +1, 1, XPS, 2, XAS, R0, R1, R2, 0, NP, KB, 0, W>(s, tw, lane);
+    constexpr int PB = TRIPLE ? NP - 1 : NP;   // backward passes through shared memory
+    if constexpr (TRIPLE && 2 * (NX / R0) > W) {   // an array's butterflies fill the lanes
+#pragma unroll 1
+        for (int a = 0; a < 3; a++) pdfft::wpasses<NX, +1, 1, XPS, 1, 0, R0, R1, R2, 0, PB, KB, 0, W>(s + a * XAS, tw, lane);
+    } else if constexpr (NA == 2) {
+        pdfft::wpasses<NX, +1, 1, XPS, 2, XAS, R0, R1, R2, 0, PB, KB, 0, W>(s, tw, lane);
+        if constexpr (TRIPLE) pdfft::wpasses<NX, +1, 1, XPS, 1, 0, R0, R1, R2, 0, PB, KB, 0, W>(s + 2 * XAS, tw, lane);
     } else {   // one array at a time, one copy of the code (instruction-cache footprint)
 #pragma unroll 1
-        for (int a = 0; a < 2; a++) pdfft::wpasses<NX, +1, 1, XPS, 1, 0, R0, R1, R2, 0, NP, KB, 0, W>(s + a * XAS, tw, lane);
+        for (int a = 0; a < (TRIPLE ? 3 : 2); a++) pdfft::wpasses<NX, +1, 1, XPS, 1, 0, R0, R1, R2, 0, PB, KB, 0, W>(s + a * XAS, tw, lane);
     }
     T umax = T(0);
-    if constexpr (XP::fused) {
+    if constexpr (TRIPLE) {
+        // item `lane` of each array's last backward pass: the fields at n = lane + r * NRL; item
+        // `lane` of the first forward pass (the plan reversed) takes the same points
+        constexpr int RL = XP::rl, NRL = XP::nrl;
+        const bool on = NRL == W || lane < NRL;
+        C v0[RL], v1[RL], v2[RL];
+        if (on) {
+            pdfft::pass_load<NX, RL, NRL, +1, 1, 1, XPS, 0>(s, tw, lane, v0);
+            pdfft::pass_load<NX, RL, NRL, +1, 1, 1, XPS, 0>(s + XAS, tw, lane, v1);
+            pdfft::pass_load<NX, RL, NRL, +1, 1, 1, XPS, 0>(s + 2 * XAS, tw, lane, v2);
+#pragma unroll
+            for (int r = 0; r < RL; r++) {
+                const int n = lane + r * NRL;
+                const T u1 = v0[r].x, u2 = v0[r].y, u3 = v1[r].x, w1 = v1[r].y, w2 = v2[r].x, w3 = v2[r].y;
+                if (want_phys && valid) {
+                    F.phys[q * NX + n] = u1;
+                    F.phys[g.R + q * NX + n] = u2;
+                    F.phys[2 * g.R + q * NX + n] = u3;
+                }
+                if (want_cfl) umax = fmax(umax, fabs(u1) + fabs(u2) + fabs(u3));
+                T n3;
+                v0[r] = nl_point<T, C>(bf, g.shear && !g.rrot, u1, u2, u3, w1, w2, w3, n3);
+                v1[r] = mk(n3, T(0));
+            }
+        }
+        __syncwarp();   // every lane has read the arrays
+        if (on) {
+            pdfft::dft<RL, -1>(v0);
+            pdfft::pass_store<NX, RL, 1, 1, 1, XPS, 0>(s, lane, v0);
+            pdfft::dft<RL, -1>(v1);
+            pdfft::pass_store<NX, RL, 1, 1, 1, XPS, 0>(s + XAS, lane, v1);
+        }
+        __syncwarp();
+    } else if constexpr (XP::fused) {
         constexpr int RL = XP::rl, NRL = XP::nrl;
         pdfft::wpasses<NX, +1, 1, XPS, 1, 0, R0, R1, R2, 0, NP - 1, KB>(s + 2 * XAS, tw, lane);
         C v[RL];
@@ -290,7 +372,7 @@ __global__ void __launch_bounds__(32 * Cfg<NX>::NWX, Cfg<NX>::template minbx<T>(
     }
     if (want_cfl) {
         for (int o = 16; o > 0; o >>= 1) umax = fmax(umax, __shfl_xor_sync(0xffffffffu, umax, o));
-        if ((tid & 31) == 0) atomicMax(&F.clock->ucfl_bits, (unsigned long long)__double_as_longlong((double)umax));
+        if (tid == 0) atomicMax(&F.clock->ucfl_bits, (unsigned long long)__double_as_longlong((double)umax));
     }
     if constexpr (RS) {   // the warp's sums into slot q % kRsSlots
         double* slot = rs + (size_t)(q % kRsSlots) * kRsWords;
@@ -315,8 +397,12 @@ __global__ void __launch_bounds__(32 * Cfg<NX>::NWX, Cfg<NX>::template minbx<T>(
     if (pf_lines > 0 && valid && q + pf_lines < lines && lane < 6)
         prefetch_l2(F.yb + lane * fstride + (q + pf_lines) * NKIP, NKI * sizeof(C));
     // forward transforms of the product arrays; only the band is written
-    constexpr int F0 = XP::f0, F1 = XP::f1, F2 = XP::f2, P0 = XP::fused ? 1 : 0;
-    if constexpr (NA == 2) {
+    constexpr bool REV = TRIPLE || XP::fused;   // the forward plan is the backward one reversed
+    constexpr int F0 = REV ? XP::rl : XP::f0, F1 = REV ? (R2 ? R1 : R0) : XP::f1, F2 = REV ? (R2 ? R0 : 0) : XP::f2, P0 = REV ? 1 : 0;
+    if constexpr (TRIPLE && 2 * (NX / F1) > W && NX / F1 != W) {
+#pragma unroll 1
+        for (int a = 0; a < 2; a++) pdfft::wpasses<NX, -1, 1, XPS, 1, 0, F0, F1, F2, P0, NP, 0, KB, W>(s + a * XAS, tw, lane);
+    } else if constexpr (NA == 2) {
         pdfft::wpasses<NX, -1, 1, XPS, 2, XAS, F0, F1, F2, P0, NP, 0, KB, W>(s, tw, lane);
     } else {
 #pragma unroll 1
@@ -662,7 +748,14 @@ template <int N, bool TWO = false> struct TCfg {
         return (sizeof(T) == 8 || lines<T>() == 16) ? (NT <= 128 ? (N == 192 ? 4 : 5) : (NT <= 256 ? 2 : (N == 512 ? 2 : 1)))
                                                     : (NT <= 128 ? (N == 192 ? 6 : 8) : (NT <= 256 ? 4 : 2));
     }
-    template <class T> static constexpr size_t smem() { return sizeof(typename Cplx<T>::type) * (size_t)N * lines<T>(); }
+    // pad rows of the FP32 tiles of 8 lines (64-byte rows); at 1024 points, two butterflies per
+    // thread, the padded index does not fit the 64 registers (K2 of 1024^3 5.50 -> 5.85 ms)
+    template <class T> static constexpr int ps() {
+        return N == 1024 ? 0 : pdfft::tile_pad<(int)sizeof(typename Cplx<T>::type) * lines<T>(), r0<T>()>();
+    }
+    template <class T> static constexpr size_t smem() {
+        return sizeof(typename Cplx<T>::type) * (size_t)tile_rows<N, ps<T>()>() * lines<T>();
+    }
     // tiles along i; with 16 lines the last one may be partial (nkip is a multiple
     // of 8), and its loads and stores stop at nkip
     template <class T> static unsigned tiles(const Geo& g) {
@@ -672,7 +765,7 @@ template <int N, bool TWO = false> struct TCfg {
     template <int S, int L, int KF, int KS, class C, class Ld, class St, class Mid = pdfft::NoMid>
     static __device__ __forceinline__ void transform(C* s, const C* tw, Ld& ld, St& st, const Mid& mid = Mid()) {
         using T = pdfft::real_of<C>;
-        pdfft::fft_tile_io<N, S, L, nt<T>(), r0<T>(), r1<T>(), r2<T>(), KF, KS>(s, tw, threadIdx.x, ld, st, mid);
+        pdfft::fft_tile_io<N, S, L, nt<T>(), r0<T>(), r1<T>(), r2<T>(), KF, KS, ps<T>()>(s, tw, threadIdx.x, ld, st, mid);
     }
 };
 
@@ -693,7 +786,6 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<T>(),
     k_zpass_inv(const __grid_constant__ MemberSet<T, CAP> ms, int stage,
                                                                                                    long long pf_ctas) {
     using C = typename FieldsT<T>::C;
-    constexpr bool SHEAR = FORM != 0;
     constexpr int nf = FORM == 3 ? 9 : 6;
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.x / nf];
     if (!mm.active) return;
@@ -716,19 +808,23 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<T>(),
     const T k2t = (T)k2;
     const long long istride = (long long)nkj_ * NKK;
     const long long row0 = ((long long)i0 * nkj_ + j) * NKK;
-    // velocity: u_f; vorticity omega_{f-3} = i (ka a - kb b): omega1 = i (k2 u3 - k3 u2),
-    // omega2 = i (k3 u1 - k1 u3), omega3 = i (k1 u2 - k2 u1).  R-conv: fields 3 + c and
-    // 6 + c are d u_c / dy and d u_c / dz (d u_c / dx is formed in the x pass).
+    // velocity: u_f; vorticity omega_{f-3}: a linear form of the line (vort_line).  R-conv: fields
+    // 3 + c and 6 + c are d u_c / dy and d u_c / dz (d u_c / dx is formed in the x pass).
     // (selects, not an index into F.u: a computed index would move F to local memory)
     constexpr bool rconv = FORM == 3;
     const int fc = rconv ? f % 3 : -1;
     const C* const pa = rconv ? (fc == 0 ? F.u[0] : (fc == 1 ? F.u[1] : F.u[2]))
-                              : ((f == 0 || f == 4) ? F.u[0] : ((f == 1 || f == 5) ? F.u[1] : F.u[2]));
-    const C* pb = (f == 3) ? F.u[1] : ((f == 4) ? F.u[2] : F.u[0]);
-    BFT<T> bf;
-    if constexpr (SHEAR) {
-        if (f >= 3) bf = bf_as<T>(make_bf(g, F.clock));
+                              : ((f == 0 || f >= 4) ? F.u[0] : ((f == 1 || f == 3) ? F.u[1] : F.u[2]));
+    // vorticity omega_{f-3}: components A and B (and in BF-rot's omega3 the third)
+    const C* const pb = f == 5 ? F.u[1] : F.u[2];
+    const C* const pc = F.u[2];
+    const bool three = FORM == 1 && f == 5;
+    VortLine<T> vl;
+    if constexpr (FORM == 1 || FORM == 2) {
+        if (f >= 3)   // a thread's items of the first pass all have line tid % LT
+            vl = vort_line<FORM, T>(bf_as<T>(make_bf(g, F.clock)), f - 3, (T)(i0 + (int)threadIdx.x % LT), k2t);
     }
+    static_assert(TCfg<NZ>::template nt<T>() % LT == 0, "a thread owns one line of the tile");
     auto ld = [&](int z, int l, auto band) -> C {
         constexpr int B = decltype(band)::value;
         const int i = i0 + l;
@@ -739,34 +835,20 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<T>(),
         if (i >= nki) return mk(T(0), T(0));
         const long long m = row0 + l * istride + k;
         if (f < 3) return pa[m];
+        const T k3 = B == 1 ? (T)z : (B == 2 ? (T)(z - NZ) : (T)wvn(k, KK));
         if constexpr (FORM == 3) {   // f_RK3Derivative (src/pf_rk3.f90:3735-3743): i k2 u_c or i k3 u_c
-            const T kd = f < 6 ? k2t : (T)wvn(k, KK);
+            const T kd = f < 6 ? k2t : k3;
             const C uc = pa[m];
             return mk(-kd * uc.y, kd * uc.x);
-        } else if constexpr (SHEAR) {
-            // BF-rot vorticity (f_RK3VorticityBFRot) or the R-rot sheared curl, in T
-            const T kv[3] = {(T)i, k2t, (T)wvn(k, KK)};
-            const C zero = mk(T(0), T(0));
-            // omega1 has no term in u1 and omega2 none in u2: those loads are skipped
-            const C uv[3] = {f != 3 ? F.u[0][m] : zero, f != 4 ? F.u[1][m] : zero, F.u[2][m]};
-            C w3[3];
-            // only the CTA's own component (f is uniform over the CTA)
-            if constexpr (FORM == 2) {
-                if (f == 3) vort_rrot<0>(bf, uv, kv, w3);
-                else if (f == 4) vort_rrot<1>(bf, uv, kv, w3);
-                else vort_rrot<2>(bf, uv, kv, w3);
-            } else {
-                if (f == 3) vort_bf<0>(bf, uv, kv, w3);
-                else if (f == 4) vort_bf<1>(bf, uv, kv, w3);
-                else vort_bf<2>(bf, uv, kv, w3);
-            }
-            return f == 3 ? w3[0] : (f == 4 ? w3[1] : w3[2]);
-        } else {
-            const T k1 = (T)i, k3 = (T)wvn(k, KK);
-            const T ka = (f == 3) ? k2t : ((f == 4) ? k3 : k1);
-            const T kb = (f == 3) ? k3 : ((f == 4) ? k1 : k2t);
+        } else if constexpr (FORM == 0) {   // omega = i (ka u_A - kb u_B), in the order of the components
+            const T k1 = (T)i;
+            const T ka = f == 3 ? -k3 : (f == 4 ? k3 : -k2t), kb = f == 3 ? -k2t : (f == 4 ? k1 : -k1);
             const C a = pa[m], b = pb[m];
-            return mk((-ka * a.y) - (-kb * b.y), (ka * a.x) - (kb * b.x));
+            return mk(-ka * a.y - -kb * b.y, ka * a.x - kb * b.x);
+        } else {
+            C c3;
+            if (three) c3 = pc[m];
+            return vort_mode<T, C>(vl, k3, pa[m], pb[m], three ? &c3 : nullptr);
         }
     };
     C* dst = F.zb + (((long long)f * NZ) * nkj_ + j) * nkip_ + i0;
@@ -807,19 +889,29 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<T>(),
 // one mbarrier; rows past NKI and k past NKK are filled with zeros by the copy engine).
 // Each field's backward z transform then takes its first-pass inputs from that staging
 // (velocity, or vorticity / gradients formed on the fly) instead of from global memory,
-// and stores z rows of 8 i as K1 does.  u is read from HBM once per tile, in whole rows,
+// and stores z rows of 4 i.  u is read from HBM once per tile, in whole rows,
 // instead of element-wise by each field's CTA.
 // ---------------------------------------------------------------------------
 template <int NZ> struct ZStage {
     static constexpr int NKK = 2 * (NZ / 3) + 1;
     static constexpr int NB = (NKK + 127) / 128;                 // boxes along k (<= 128 complex each)
     static constexpr int BK0 = (NKK + NB - 1) / NB;
-    static constexpr int BK = BK0 + (9 - BK0 % 8) % 8;           // = 1 mod 8: the 8 rows of a box on distinct banks
+    static constexpr int lines = 4;
+    // row pitch: the rows of a box, and the 8 / lines consecutive k a quarter warp reads of each,
+    // on distinct banks
+    static constexpr int BK = BK0 + ((8 / lines - BK0 % 8) % 8 + 8) % 8;
     static_assert(BK <= 128, "tensor box wider than 256 doubles");
-    static constexpr int words = 3 * NB * 8 * BK;                // staged complex values
-    static constexpr size_t smem = sizeof(double2) * words + TCfg<NZ>::template smem<double>() + 16;
-    // measured at 512 only (one CTA of 512 threads per SM): as fast as the element-wise K1
-    // at 512^3, with u read from HBM once per tile in whole rows
+    static constexpr int words = 3 * NB * lines * BK;            // staged complex values
+    static constexpr int r0 = pdfft::Plan<NZ>::r0, r1 = pdfft::Plan<NZ>::r1, r2 = pdfft::Plan<NZ>::r2;
+    static constexpr int ps = pdfft::tile_pad<16 * lines, r0>();
+    static constexpr int nt = pdfft::tile_threads_for<NZ, r0, r1, r2, lines>();
+    static_assert(nt % lines == 0, "a thread owns one line of the tile");
+    static constexpr size_t smem = sizeof(double2) * (words + tile_rows<NZ, ps>() * lines + NZ) + 16;   // + twiddles, barrier
+    // Two CTAs of 4 lines per SM: the copies of one run under the transforms of the other (one CTA
+    // of 8 lines waited for its 139 KB before it began: 1.19 ms per stage at 512^3, 1.15 with
+    // two; with the twiddles in shared memory, whose reads missed the little L1 that is left,
+    // and the vorticity as linear forms, 1.05).  At 512 only: a shorter line's plan leaves too
+    // few threads per CTA, a longer one's staging does not fit twice.
     static constexpr bool enabled = NZ == 512;
 };
 
@@ -839,12 +931,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 }
 
 template <int NZ, int FORM>
-__global__ void __launch_bounds__(TCfg<NZ>::template nt<double>(), 1) k_zpass_inv_tma(const __grid_constant__ MemberSet<double, 1> ms,
+__global__ void __launch_bounds__(ZStage<NZ>::nt, 2) k_zpass_inv_tma(const __grid_constant__ MemberSet<double, 1> ms,
                                                                                      const __grid_constant__ ZMaps maps,
                                                                                      int stage) {
     using C = double2;
     using ZS = ZStage<NZ>;
-    constexpr int LT = 8, BK = ZS::BK, NB = ZS::NB;
+    constexpr int LT = ZS::lines, BK = ZS::BK, NB = ZS::NB;
     constexpr int nf = FORM == 3 ? 9 : 6;
     const Member<double>& mm = ms.m[0];
     if (!mm.active) return;
@@ -852,7 +944,8 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<double>(), 1) k_zpass_in
     const Geo g = mm.g;
     C* stg = smem_as<C>();
     C* s = stg + ZS::words;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(s + NZ * LT);
+    C* const tw = s + tile_rows<NZ, ZS::ps>() * LT;   // the twiddle table: six transforms' worth of reads, which L1 does not hold
+    uint64_t* bar = reinterpret_cast<uint64_t*>(tw + NZ);
     const int i0 = blockIdx.x * LT, j = blockIdx.y, tid = threadIdx.x;
     if (stage == 1 && blockIdx.x == 0 && j == 0 && tid == 0) F.clock->ucfl_bits = 0ull;
     const uint32_t ba = smem_u32(bar);
@@ -878,10 +971,12 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<double>(), 1) k_zpass_in
             for (int b = 0; b < NB; b++)
                 asm volatile(
                     "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                    " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(stg + (c * NB + b) * 8 * BK)),
+                    " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(stg + (c * NB + b) * LT * BK)),
                     "l"(reinterpret_cast<uint64_t>(&maps.u[c])), "r"(2 * b * BK), "r"(j), "r"(i0), "r"(ba)
                     : "memory");
     }
+    for (int e = tid; e < NZ; e += ZS::nt) tw[e] = F.tw_z[e];
+    __syncthreads();
     // bounded wait (about 2 s of SM clocks); on a timeout the status word records it and,
     // after a second bounded wait for the copies in flight, the CTA returns
     constexpr long long kLimit = 4000000000ll;
@@ -892,16 +987,21 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<double>(), 1) k_zpass_in
     }
     constexpr int KK = NZ / 3;   // g.kk (the 2/3 rule)
     const double k2 = wvn(j, g.kj);
-    BF bf;
-    if constexpr (FORM == 1 || FORM == 2) bf = make_bf(g, F.clock);
     // staged value of component c at (line l, k)
     auto su = [&](int c, int l, int k) -> C {
         const int b = k / BK;
-        return stg[((c * NB + b) * 8 + l) * BK + (k - b * BK)];
+        return stg[((c * NB + b) * LT + l) * BK + (k - b * BK)];
     };
     const long long zs = (long long)g.nkj * g.nkip;
 #pragma unroll 1
     for (int f = 0; f < nf; f++) {
+        // vorticity: the components and coefficients of the thread's line (tid % LT)
+        const int ca = f == 3 ? 1 : 0, cb = f == 5 ? 1 : 2;
+        const bool three = FORM == 1 && f == 5;
+        VortLine<double> vl;
+        if constexpr (FORM == 1 || FORM == 2) {
+            if (f >= 3) vl = vort_line<FORM, double>(make_bf(g, F.clock), f - 3, (double)(i0 + tid % LT), k2);
+        }
         auto ld = [&](int z, int l, auto band) -> C {
             constexpr int B = decltype(band)::value;
             int k;
@@ -916,34 +1016,21 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<double>(), 1) k_zpass_in
                 return mk(-kd * uc.y, kd * uc.x);
             } else {
                 if (f < 3) return su(f, l, k);
-                const double k1 = (double)(i0 + l), k3 = wvn(k, KK);
-                if constexpr (FORM == 1 || FORM == 2) {
-                    const double kv[3] = {k1, k2, k3};
-                    const C zero = mk(0.0, 0.0);
-                    const C uv[3] = {f != 3 ? su(0, l, k) : zero, f != 4 ? su(1, l, k) : zero, su(2, l, k)};
-                    C w3[3];
-                    if constexpr (FORM == 2) {
-                        if (f == 3) vort_rrot<0>(bf, uv, kv, w3);
-                        else if (f == 4) vort_rrot<1>(bf, uv, kv, w3);
-                        else vort_rrot<2>(bf, uv, kv, w3);
-                    } else {
-                        if (f == 3) vort_bf<0>(bf, uv, kv, w3);
-                        else if (f == 4) vort_bf<1>(bf, uv, kv, w3);
-                        else vort_bf<2>(bf, uv, kv, w3);
-                    }
-                    return f == 3 ? w3[0] : (f == 4 ? w3[1] : w3[2]);
-                } else {   // omega = i k x u (f_RK3PrepareVelocity, src/pf_rk3.f90:402-407,520-525,630-634)
-                    const double ka = (f == 3) ? k2 : ((f == 4) ? k3 : k1);
-                    const double kb = (f == 3) ? k3 : ((f == 4) ? k1 : k2);
-                    const int ca = (f == 3) ? 2 : ((f == 4) ? 0 : 1), cb = (f == 3) ? 1 : ((f == 4) ? 2 : 0);
+                const double k3 = B == 1 ? (double)z : (B == 2 ? (double)(z - NZ) : wvn(k, KK));
+                if constexpr (FORM == 0) {
+                    const double k1 = (double)(i0 + l);
+                    const double ka = f == 3 ? -k3 : (f == 4 ? k3 : -k2), kb = f == 3 ? -k2 : (f == 4 ? k1 : -k1);
                     const C a = su(ca, l, k), bb = su(cb, l, k);
-                    return mk((-ka * a.y) - (-kb * bb.y), (ka * a.x) - (kb * bb.x));
+                    return mk(-ka * a.y - -kb * bb.y, ka * a.x - kb * bb.x);
                 }
+                C c3;
+                if (three) c3 = su(2, l, k);
+                return vort_mode<double, C>(vl, k3, su(ca, l, k), su(cb, l, k), three ? &c3 : nullptr);
             }
         };
         C* dst = F.zb + (((long long)f * NZ) * g.nkj + j) * g.nkip + i0;
         auto st = [&](int z, int l, C v) { dst[z * zs + l] = v; };
-        TCfg<NZ>::template transform<+1, LT, KK, 0>(s, F.tw_z, ld, st);
+        pdfft::fft_tile_io<NZ, +1, LT, ZS::nt, ZS::r0, ZS::r1, ZS::r2, KK, 0, ZS::ps>(s, tw, tid, ld, st);
         __syncthreads();   // the tile buffer is read by the last pass before the next field's first pass
     }
 }
@@ -1064,18 +1151,8 @@ __global__ void __launch_bounds__(TCfg<NZ, true>::template nt<T>(), TCfg<NZ, tru
 }
 
 
-// x lengths whose x pass has instantiations with several lines per warp (short, unfused
-// lines, where one line leaves most lanes idle in its loads and passes).
+// x lengths whose x pass has instantiations for every x_lines_per_warp.
 template <int N> constexpr bool xlpw_len() { return N <= 64; }
-// Lines per warp of the x pass when the simulation leaves the choice to the library,
-// measured on B200 (decaying flow, FP64): batches of 32 members run 4 lines per warp up to
-// 48 points (32^3: 80K -> 106K member-steps/s, 48^3: 22.2K -> 27.1K) and 2 at 64 points
-// (17.0K -> 21.2K); a single simulation, whose step is bound by its launches at these
-// sizes, 2 from 48 points (64^3: 0.109 -> 0.101 ms per step).
-template <int N, class T, int CAP> constexpr int default_xlpw() {
-    return CAP > 1 ? (N <= 48 ? 4 : 2) : (N >= 48 ? 2 : 1);
-}
-
 // Lengths whose K1, K2 and K4 have instantiations for cubic grids (every size a
 // compile-time constant, so the index arithmetic folds): FP32-mixed, the benchmark and
 // ensemble sizes.  Measured at 512^3 shear: K1 0.74 -> 0.69, K2 0.70 -> 0.58, K4 0.32 ->

@@ -5,8 +5,8 @@
 
 namespace pd {
 
-template <int N, class T, int LPW = 1> static size_t smem_kx() {
-    return sizeof(typename Cplx<T>::type) * ((size_t)Cfg<N>::NWX * LPW * 3 * xas<N>());
+template <int N, class T, int LPW = XCfg<N, T>::lpw> static size_t smem_kx() {
+    return sizeof(typename Cplx<T>::type) * (size_t)LPW * XCfg<N, T>::template ls<LPW>();
 }
 
 // CTAs of `kernel` resident on the whole device at once.
@@ -53,10 +53,13 @@ template <int N, class T, int CAP> static cudaError_t configure_cap(const Geo& g
         if ((e = set_smem(k_ypass_fwd<N, T, CAP>, TCfg<N, true>::template smem<T>()))) return e;
     }
     if (g.nx == N) {
-        if ((e = set_smem(k_xpass<N, T, CAP>, smem_kx<N, T>()))) return e;
-        if constexpr (xlpw_len<N>()) {
+        if constexpr (xlpw_len<N>()) {   // at most 20 KB per warp: no opt-in needed beyond this
+            if ((e = set_smem(k_xpass<N, T, CAP, false, 1>, smem_kx<N, T, 1>()))) return e;
             if ((e = set_smem(k_xpass<N, T, CAP, false, 2>, smem_kx<N, T, 2>()))) return e;
             if ((e = set_smem(k_xpass<N, T, CAP, false, 4>, smem_kx<N, T, 4>()))) return e;
+        } else {
+            constexpr int LPW = XCfg<N, T>::lpw;
+            if ((e = set_smem(k_xpass<N, T, CAP, false, LPW>, smem_kx<N, T>()))) return e;
         }
         if (g.rconv && (e = set_smem(k_xpass_conv<N, T, CAP>, ConvCfg<N, T>::smem))) return e;
     }
@@ -88,8 +91,8 @@ cudaError_t zpass_inv_n(const Geo& g, const Member<T>* M, int B, int stage, cuda
         if (maps && B == 1) {
             MemberSet<double, 1> one;
             one.m[0] = M[0];
-            const dim3 grid(TCfg<N>::template tiles<double>(g), g.nkj);
-            constexpr int NT = TCfg<N>::template nt<double>();
+            const dim3 grid((unsigned)(g.nkip / ZStage<N>::lines), g.nkj);
+            constexpr int NT = ZStage<N>::nt;
             constexpr size_t sm = ZStage<N>::smem;
             if (!g.shear) k_zpass_inv_tma<N, 0><<<grid, NT, sm, st>>>(one, *maps, stage);
             else if (!g.rrot) k_zpass_inv_tma<N, 1><<<grid, NT, sm, st>>>(one, *maps, stage);
@@ -154,22 +157,19 @@ cudaError_t xpass_n(const Geo& g, const Member<T>* M, int B, int want_phys, int 
             }
             auto go = [&](auto lpwc) {
                 constexpr int LPW = decltype(lpwc)::value;
-                constexpr int LB = Cfg<N>::NWX * LPW;   // lines per CTA
-                const long long nl = (lines + LB - 1) / LB;
+                const long long nl = (lines + LPW - 1) / LPW;
                 // L2 prefetch distance: one wave of resident CTAs (single simulations)
-                const long long pf = CAP == 1 ? LB * resident_ctas(k_xpass<N, T, CAP, false, LPW>, 32 * Cfg<N>::NWX,
-                                                                   smem_kx<N, T, LPW>())
-                                              : 0;
-                k_xpass<N, T, CAP, false, LPW><<<dim3((unsigned)nl, nb), 32 * Cfg<N>::NWX, smem_kx<N, T, LPW>(), st>>>(
-                    ms, want_phys, want_cfl, pf, nullptr);
+                const long long pf = CAP == 1 ? LPW * resident_ctas(k_xpass<N, T, CAP, false, LPW>, 32, smem_kx<N, T, LPW>()) : 0;
+                k_xpass<N, T, CAP, false, LPW><<<dim3((unsigned)nl, nb), 32, smem_kx<N, T, LPW>(), st>>>(ms, want_phys,
+                                                                                                       want_cfl, pf, nullptr);
             };
             if constexpr (xlpw_len<N>()) {
-                const int lpw = g.xlpw > 0 ? g.xlpw : default_xlpw<N, T, CAP>();
+                const int lpw = g.xlpw > 0 ? g.xlpw : XCfg<N, T>::lpw;
                 if (lpw == 4) go(std::integral_constant<int, 4>{});
                 else if (lpw == 2) go(std::integral_constant<int, 2>{});
                 else go(std::integral_constant<int, 1>{});
             } else {
-                go(std::integral_constant<int, 1>{});
+                go(std::integral_constant<int, XCfg<N, T>::lpw>{});
             }
         }
     });
@@ -179,12 +179,12 @@ cudaError_t xpass_n(const Geo& g, const Member<T>* M, int B, int want_phys, int 
 // point into `rs` (kRsSlots x kRsWords doubles, zeroed by the caller).
 template <int N, class T> cudaError_t xpass_stats_n(const Geo& g, const Member<T>* M, double* rs, cudaStream_t st) {
     const long long lines = (long long)g.ny * g.nz;
-    cudaError_t e = set_smem(k_xpass<N, T, 1, true>, smem_kx<N, T>());
+    constexpr size_t sm = sizeof(typename Cplx<T>::type) * 3 * (size_t)xas<N>();
+    cudaError_t e = set_smem(k_xpass<N, T, 1, true>, sm);
     if (e) return e;
     MemberSet<T, 1> ms;
     ms.m[0] = M[0];
-    const long long nl = (lines + Cfg<N>::NWX - 1) / Cfg<N>::NWX;
-    k_xpass<N, T, 1, true><<<dim3((unsigned)nl, 1), 32 * Cfg<N>::NWX, smem_kx<N, T>(), st>>>(ms, 0, 0, 0, rs);
+    k_xpass<N, T, 1, true><<<dim3((unsigned)lines, 1), 32, sm, st>>>(ms, 0, 0, 0, rs);
     return cudaGetLastError();
 }
 
