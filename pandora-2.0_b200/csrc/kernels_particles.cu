@@ -1,6 +1,6 @@
 // kernels_particles.cu -- Lagrangian particle advance on sm_100a.
 //
-// One thread per particle: tensor-product Lagrange interpolation of order ORD
+// A group of threads per particle: tensor-product Lagrange interpolation of order ORD
 // of the physical velocity of the current stage (the reference evaluates the
 // same polynomial by Neville's scheme, p_InterpInterpolate3D / FindMolecule /
 // Neville3D, src/pp_interp.f90:313-560), the tracer or Stokes-drag RK3 update
@@ -8,7 +8,8 @@
 // wrap (p_MPICorrectPosition, src/pp_mpi.f90:1011-1057; x3 uses '>' where x1
 // and x2 use '>=').  The reference fetches a halo of NHALO = order/2 planes by
 // DMGlobalToLocal (src/pp_interp.f90:115-264); on one GPU the stencil indices
-// wrap modulo N.  Physical velocity layout: [c][z][y][x].
+// wrap modulo N.  Physical velocity layout: [z][y][x][4], the three components of a point
+// side by side (and a pad), so that a stencil point is one vector load.
 //
 // Particles are kept sorted by spatial bin (z slowest), re-sorted once per step,
 // so that a wave of threads reads a compact set of velocity rows that stays in
@@ -20,8 +21,6 @@
 #include "bfrot.cuh"
 
 namespace pd {
-
-constexpr int kMaxOrder = 6;
 
 // Lagrange basis weight m at x over the ORD nodes: prod_{n != m} (x - x_n) / (x_m - x_n),
 // formed as one quotient of the two products (one FP64 division per weight).
@@ -41,147 +40,209 @@ __device__ __forceinline__ double lagrange_weight(double x, const double* nodes,
 // G threads per particle (G = the power of two at or above ORD): thread `sub` of a
 // group gathers the stencil column x = i0 + sub (threads sub >= ORD add nothing),
 // so one warp load touches 32/G particles' rows of consecutive values instead of
-// 32 scattered rows; the group sums its partial results with shuffles and its
-// first thread does the update.
+// 32 scattered rows; the group sums its partial results with shuffles.
+// The kernel is bound by the L1 lookups of its gathers and by the trips to memory of each
+// group's chain (position, stencil, RK3 state).  Against one component per field (48 loads of 8
+// bytes a thread at order 4, 84 sectors a particle; the state read at the end by one thread in
+// four; every thread dividing for all three directions): 16 loads of 32 bytes, 64 sectors; the
+// state asked for first and updated by one thread per component.  0.320 -> 0.230 ms per stage for
+// 2^20 tracers in 256^3 (FP32-mixed 0.300 -> 0.213), 0.246 -> 0.156 for 2^18 in 512^3 (0.188 ->
+// 0.124).
 template <int ORD> constexpr int part_group() { return ORD <= 1 ? 1 : (ORD <= 2 ? 2 : (ORD <= 4 ? 4 : 8)); }
+// CTAs of 256 threads per SM asked of the register allocator: 80 registers hold a plane of the
+// order-4 FP64 stencil in flight, 64 two planes of the FP32 one.  2^20 tracers in 256^3: FP64
+// 0.230 ms with 3 (0.286 with 4), FP32-mixed 0.213 with 4 (0.225 with 3).
+template <int ORD, class T> constexpr int part_ctas() { return ORD <= 4 && sizeof(T) == 4 ? 4 : 3; }
+
+// Stencil index q wrapped into [0, n): one period away at most for a position inside the
+// domain, so the division is off the common path.
+__device__ __forceinline__ int wrap_index(int q, int n) {
+    if ((unsigned)q >= (unsigned)n) {
+        q %= n;
+        if (q < 0) q += n;
+    }
+    return q;
+}
+
+// Start of the stencil along one direction, from the same rounded arithmetic as
+// p_InterpFindMolecule (src/pp_interp.f90:313-560).
+template <int ORD> __device__ __forceinline__ int stencil_start(double x, double d) {
+    constexpr int nh = ORD / 2;
+    double halo = __dmul_rn((double)nh, d);
+    double xd;
+    if ((ORD & 1) == 0) {
+        halo = __dsub_rn(halo, __dmul_rn(0.5, d));
+        xd = __dadd_rn(__dadd_rn(__dadd_rn(x, halo), d), __dmul_rn(0.5, d));
+    } else {
+        xd = __dadd_rn(__dadd_rn(x, halo), __dmul_rn(0.5, d));
+    }
+    return (int)__ddiv_rn(xd, d) - nh - nh;
+}
+
+// The velocity of all three components at one grid point: one 32-byte (FP64) or 16-byte
+// (FP32) load of the interleaved field.
+__device__ __forceinline__ void load_point(const double* p, double* v) {
+    asm("{\n .reg .f64 pad;\n ld.global.nc.v4.f64 {%0, %1, %2, pad}, [%3];\n}" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]) : "l"(p));
+}
+__device__ __forceinline__ void load_point(const float* p, double* v) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = (double)q.x; v[1] = (double)q.y; v[2] = (double)q.z;
+}
+__device__ __forceinline__ double pick(int c, double a, double b, double d) { return c == 0 ? a : (c == 1 ? b : d); }
+__device__ __forceinline__ double* pick(int c, double* const* p) { return c == 0 ? p[0] : (c == 1 ? p[1] : p[2]); }
 
 // T: precision of the stored physical velocity (the particle state and its
 // arithmetic are FP64 in both forms).
 template <int ORD, class T, int CAP>
-__global__ void __launch_bounds__(256, 2) k_particles(const __grid_constant__ MemberSet<T, CAP> ms, int stage) {
+__global__ void __launch_bounds__(256, part_ctas<ORD, T>()) k_particles(const __grid_constant__ MemberSet<T, CAP> ms, int stage) {
     constexpr int G = part_group<ORD>();
+    // Components a thread advances: with four or more threads per particle, thread c < 3 of
+    // the group holds and updates component c; with one or two, the first thread all three.
+    constexpr int NC = G >= 4 ? 1 : 3;
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.y];
     if (!mm.active) return;
     if constexpr (CAP > 1) {   // a batch slot between members
         if (mm.F.clock->status & PD_ST_IDLE) return;
     }                             // uniform over the CTA
-    const Particles P = mm.P;
-    const Geo g = mm.g;
+    const Particles& P = mm.P;
+    const Geo& g = mm.g;
     const T* __restrict__ phys = mm.F.phys;
     Clock* ck = mm.F.clock;
-    const PartParams pp = mm.pp;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long n = t / G;
     const int sub = (int)(t % G);
     const int tstep = ck->tstep;
-    if (tstep < pp.release) return;                     // uniform over the member
+    if (tstep < mm.pp.release) return;                  // uniform over the member
     if (G == 1 && n >= P.np) return;
     // With G > 1 every lane of a warp reaches the shuffles: lanes past the last
     // particle (whole groups at the tail) gather for the last particle and store nothing.
     const bool valid = n < P.np;
     const long long nn = valid ? n : P.np - 1;
+    const int base = (threadIdx.x & 31) & ~(G - 1);     // the group's first lane
+    double xp[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) xp[c] = P.xp[c][nn];
+    // the RK3 state, asked for ahead of the gather; a tracer's velocity is the fluid's and its
+    // velocity register idle, so neither is read
+    const double dpv = P.dp[nn];
+    double up[NC], ur[NC], pr[NC];
+#pragma unroll
+    for (int q = 0; q < NC; q++) {
+        const int c = G >= 4 ? (sub < 3 ? sub : 2) : q;
+        ur[q] = pick(c, P.uprk)[nn];
+        up[q] = pr[q] = 0.0;
+        if (dpv > 0.0) { up[q] = pick(c, P.up)[nn]; pr[q] = pick(c, P.prk)[nn]; }
+    }
+    // the stencil's start: with four or more threads per particle each of the first three
+    // forms one direction's (one FP64 division instead of three) and the group exchanges them
+    int i0[3];
+    if constexpr (G >= 4) {
+        const int mine = stencil_start<ORD>(pick(sub, xp[0], xp[1], xp[2]), pick(sub, g.dx, g.dy, g.dz));
+#pragma unroll
+        for (int c = 0; c < 3; c++) i0[c] = __shfl_sync(0xffffffffu, mine, base + c);
+    } else {
+        i0[0] = stencil_start<ORD>(xp[0], g.dx);
+        i0[1] = stencil_start<ORD>(xp[1], g.dy);
+        i0[2] = stencil_start<ORD>(xp[2], g.dz);
+    }
+    // weights of x (this thread's column), y and z: each thread of the group forms the
+    // weight of its own offset in every direction; those of y and z the group exchanges
+    double wx[G == 1 ? ORD : 1], wy[ORD], wz[G == 1 ? ORD : 1];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const double d = c == 0 ? g.dx : (c == 1 ? g.dy : g.dz);
+        double nodes[ORD];
+#pragma unroll
+        for (int m = 0; m < ORD; m++) nodes[m] = __dmul_rn((double)(i0[c] + m), d);
+        if constexpr (G == 1) {
+            double* w = c == 0 ? wx : (c == 1 ? wy : wz);
+#pragma unroll
+            for (int m = 0; m < ORD; m++) w[m] = lagrange_weight<ORD>(xp[c], nodes, m);
+        } else {
+            const double mine = lagrange_weight<ORD>(xp[c], nodes, sub < ORD ? sub : ORD - 1);
+            if (c == 0) wx[0] = sub < ORD ? mine : 0.0;
+            else if (c == 2) wz[0] = mine;   // exchanged plane by plane below
+            else {
+#pragma unroll
+                for (int m = 0; m < ORD; m++) wy[m] = __shfl_sync(0xffffffffu, mine, base + m);
+            }
+        }
+    }
+    // gather: a point's three components are one load of 4 T (32 bytes in FP64)
+    double uf[3] = {0.0, 0.0, 0.0};
+    int yo[ORD];
+#pragma unroll
+    for (int m = 0; m < ORD; m++) yo[m] = wrap_index(i0[1] + m, g.ny) * g.nx;
+    if constexpr (G == 1) {
+        int xo[ORD];
+#pragma unroll
+        for (int m = 0; m < ORD; m++) xo[m] = wrap_index(i0[0] + m, g.nx);
+#pragma unroll
+        for (int zi = 0; zi < ORD; zi++) {
+            const T* pl = phys + 4 * ((long long)wrap_index(i0[2] + zi, g.nz) * g.ny * g.nx);
+            double ay[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int yi = 0; yi < ORD; yi++) {
+                double ax[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+                for (int xi = 0; xi < ORD; xi++) {
+                    double v[3];
+                    load_point(pl + 4 * (long long)(yo[yi] + xo[xi]), v);
+#pragma unroll
+                    for (int c = 0; c < 3; c++) ax[c] += wx[xi] * v[c];
+                }
+#pragma unroll
+                for (int c = 0; c < 3; c++) ay[c] += wy[yi] * ax[c];
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++) uf[c] += wz[zi] * ay[c];
+        }
+    } else {
+        // column x = i0 + sub (lanes past the stencil: its last column, weight 0); the x
+        // weight is applied before the group sum
+        const int xs = wrap_index(i0[0] + (sub < ORD ? sub : ORD - 1), g.nx);
+#pragma unroll(ORD > 4 ? 1 : (sizeof(T) == 8 ? ORD : 2))
+        for (int zi = 0; zi < ORD; zi++) {
+            const T* pl = phys + 4 * ((long long)wrap_index(i0[2] + zi, g.nz) * g.ny * g.nx + xs);
+            const double w = __shfl_sync(0xffffffffu, wz[0], base + zi);
+            double v[ORD][3];
+#pragma unroll
+            for (int yi = 0; yi < ORD; yi++) load_point(pl + 4 * (long long)yo[yi], v[yi]);
+            double ay[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int yi = 0; yi < ORD; yi++)
+#pragma unroll
+                for (int c = 0; c < 3; c++) ay[c] += wy[yi] * v[yi][c];
+#pragma unroll
+            for (int c = 0; c < 3; c++) uf[c] += w * ay[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            double v = wx[0] * uf[c];
+#pragma unroll
+            for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            uf[c] = v;
+        }
+        if (NC == 3 && (sub != 0 || !valid)) return;   // NC == 1: the group exchanges components below
+    }
     const double dt = ck->dt;
     double beta, gamma;
     if (stage == 1) { beta = 0.0; gamma = 1.0 / 3.0; }
     else if (stage == 2) { beta = -(5.0 / 9.0); gamma = 15.0 / 16.0; }
     else { beta = -(153.0 / 128.0); gamma = 8.0 / 15.0; }
-    constexpr int nh = ORD / 2;
-    const double D[3] = {g.dx, g.dy, g.dz};
-    const int NN[3] = {g.nx, g.ny, g.nz};
-    double xp[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) xp[c] = P.xp[c][nn];
-    // p_InterpFindMolecule: stencil start from the same rounded arithmetic
-    double w[3][ORD];
-    int idx[3][ORD];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        double halo = __dmul_rn((double)nh, D[c]);
-        double xd;
-        if ((ORD & 1) == 0) {
-            halo = __dsub_rn(halo, __dmul_rn(0.5, D[c]));
-            xd = __dadd_rn(__dadd_rn(__dadd_rn(xp[c], halo), D[c]), __dmul_rn(0.5, D[c]));
-        } else {
-            xd = __dadd_rn(__dadd_rn(xp[c], halo), __dmul_rn(0.5, D[c]));
-        }
-        const int i0 = (int)__ddiv_rn(xd, D[c]) - nh - nh;
-        double nodes[ORD];
-#pragma unroll
-        for (int m = 0; m < ORD; m++) {
-            nodes[m] = __dmul_rn((double)(i0 + m), D[c]);
-            int q = (i0 + m) % NN[c];
-            idx[c][m] = q < 0 ? q + NN[c] : q;
-        }
-        if constexpr (G == 1) {
-#pragma unroll
-            for (int m = 0; m < ORD; m++) w[c][m] = lagrange_weight<ORD>(xp[c], nodes, m);
-        } else {
-            // each thread of the group forms the weight of its own offset; the
-            // group exchanges them (lanes of a group are consecutive)
-            const double mine = lagrange_weight<ORD>(xp[c], nodes, sub < ORD ? sub : ORD - 1);
-            const int base = (threadIdx.x & 31) & ~(G - 1);
-#pragma unroll
-            for (int m = 0; m < ORD; m++) w[c][m] = __shfl_sync(0xffffffffu, mine, base + m);
-        }
-    }
-    double uf[3];
-    if constexpr (G == 1) {
-        long long rowoff[ORD][ORD];
-#pragma unroll
-        for (int zi = 0; zi < ORD; zi++)
-#pragma unroll
-            for (int yi = 0; yi < ORD; yi++) rowoff[zi][yi] = ((long long)idx[2][zi] * g.ny + idx[1][yi]) * g.nx;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const T* f = phys + (long long)c * g.R;
-            double acc_z = 0.0;
-#pragma unroll
-            for (int zi = 0; zi < ORD; zi++) {
-                double acc_y = 0.0;
-#pragma unroll
-                for (int yi = 0; yi < ORD; yi++) {
-                    const T* row = f + rowoff[zi][yi];
-                    double acc_x = 0.0;
-#pragma unroll
-                    for (int xi = 0; xi < ORD; xi++) acc_x += w[0][xi] * (double)__ldg(row + idx[0][xi]);
-                    acc_y += w[1][yi] * acc_x;
-                }
-                acc_z += w[2][zi] * acc_y;
-            }
-            uf[c] = acc_z;
-        }
-    } else {
-        // column x = idx[0][sub]; the x weights are applied before the group sum
-        int xs = idx[0][0];
-        double wx = (sub == 0) ? w[0][0] : 0.0;
-#pragma unroll
-        for (int xi = 1; xi < ORD; xi++)
-            if (sub == xi) { xs = idx[0][xi]; wx = w[0][xi]; }
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const T* f = phys + (long long)c * g.R + xs;
-            double acc_z = 0.0;
-#pragma unroll
-            for (int zi = 0; zi < ORD; zi++) {
-                double acc_y = 0.0;
-#pragma unroll
-                for (int yi = 0; yi < ORD; yi++)
-                    acc_y += w[1][yi] * (double)__ldg(f + ((long long)idx[2][zi] * g.ny + idx[1][yi]) * g.nx);
-                acc_z += w[2][zi] * acc_y;
-            }
-            double v = wx * acc_z;
-#pragma unroll
-            for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            uf[c] = v;
-        }
-        if (sub != 0 || !valid) return;
-    }
-    // the particle's RK3 state, read only by the thread that updates it, after the
-    // gather (not held in registers across it)
-    double up[3], ur[3], pr[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) { up[c] = P.up[c][nn]; ur[c] = P.uprk[c][nn]; pr[c] = P.prk[c][nn]; }
-    double xw[3] = {xp[0], xp[1], xp[2]};   // frame in which the RK3 update runs
+    const bool release = tstep == mm.pp.release && stage == 1;
     // BF-rot shear transforms to the laboratory frame and back; the R forms
     // (p_RK3SolveParticleR, src/pp_rk3.f90:307-403, dispatched at src/pp_control.f90:
     // 568-571) interpolate laboratory components and advance the moving position with
     // them directly, the isotropic arithmetic
     const bool bfrot = g.shear && !g.rrot;
+    double xw[3] = {xp[0], xp[1], xp[2]};   // frame in which the RK3 update runs
+    BF bf;
     if (bfrot) {
         // p_RK3SolveParticleBF (src/pp_rk3.f90:169-303): velocity and position to
         // the laboratory frame (p_RK3Mov2Lab, src/pp_rk3.f90:989-1014), RK3 there,
         // back with p_RK3Lab2Mov (1016-1042) at the same B.
-        const BF bf = make_bf(g, ck);
+        bf = make_bf(g, ck);
         double xl[3] = {0.0, 0.0, 0.0}, ul[3] = {0.0, 0.0, 0.0};
 #pragma unroll
         for (int a = 0; a < 3; a++)
@@ -191,60 +252,66 @@ __global__ void __launch_bounds__(256, 2) k_particles(const __grid_constant__ Me
 #pragma unroll
         for (int c = 0; c < 3; c++) { xw[c] = xl[c]; uf[c] = ul[c]; }
     }
-    // p_ControlInitPartVelocity(BF) at the release step (src/pp_control.f90:378-516)
-    if (tstep == pp.release && stage == 1) {
+    // the components of this thread
+    double xc[NC], uc[NC];
 #pragma unroll
-        for (int c = 0; c < 3; c++) { up[c] = uf[c]; pr[c] = 0.0; ur[c] = 0.0; }
+    for (int q = 0; q < NC; q++) {
+        xc[q] = NC == 3 ? xw[q] : pick(sub, xw[0], xw[1], xw[2]);
+        uc[q] = NC == 3 ? uf[q] : pick(sub, uf[0], uf[1], uf[2]);
+        // p_ControlInitPartVelocity(BF) at the release step (src/pp_control.f90:378-516)
+        if (release) { up[q] = uc[q]; pr[q] = 0.0; ur[q] = 0.0; }
     }
-    const double dpv = P.dp[n];
-    if (dpv > 0.0) {
-        const double tau = ((dpv * dpv) / (18.0 * pp.f_nu)) * (pp.p_rho / pp.f_rho);
+    if (dpv > 0.0) {   // uniform over the group
+        const double tau = ((dpv * dpv) / (18.0 * mm.pp.f_nu)) * (mm.pp.p_rho / mm.pp.f_rho);
         // shear: minus the homogeneous source amat up (p_RK3ComputeHomogeneousSourceTerm,
         // src/pp_rk3.f90:1080-1102); amat has the single entry (1,3)
-        const double hs0 = bfrot ? g.shear_s * up[2] : 0.0;
+        double up3 = up[NC - 1];
+        if constexpr (NC == 1) up3 = __shfl_sync(__activemask(), up[0], base + 2);
+        const double hs0 = bfrot ? g.shear_s * up3 : 0.0;
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const double acc = ((uf[c] - up[c]) / tau) - (c == 0 ? hs0 : 0.0);
-            pr[c] = (beta * pr[c]) + acc;
-            up[c] = up[c] + (gamma * dt * pr[c]);
+        for (int q = 0; q < NC; q++) {
+            const bool first = NC == 3 ? q == 0 : sub == 0;
+            const double acc = ((uc[q] - up[q]) / tau) - (first ? hs0 : 0.0);
+            pr[q] = (beta * pr[q]) + acc;
+            up[q] = up[q] + (gamma * dt * pr[q]);
         }
     } else {
 #pragma unroll
-        for (int c = 0; c < 3; c++) up[c] = uf[c];
+        for (int q = 0; q < NC; q++) up[q] = uc[q];
     }
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        ur[c] = (beta * ur[c]) + up[c];
-        xw[c] = xw[c] + (gamma * dt * ur[c]);
+    for (int q = 0; q < NC; q++) {
+        ur[q] = (beta * ur[q]) + up[q];
+        xc[q] = xc[q] + (gamma * dt * ur[q]);
     }
-    if (bfrot) {
-        const BF bf = make_bf(g, ck);
+    if (bfrot) {   // back to the moving frame: bmat has the diagonal and (1,3)
+        double x3 = xc[NC - 1];
+        if constexpr (NC == 1) x3 = __shfl_sync(0xffffffffu, xc[0], base + 2);
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
+        for (int q = 0; q < NC; q++) {
+            const bool first = NC == 3 ? q == 0 : sub == 0;
             double v = 0.0;
-#pragma unroll
-            for (int b = 0; b < 3; b++)
-                if (bex(a, b)) v += bf.bm[a][b] * xw[b];
-            xp[a] = v;
+            v += (NC == 3 ? bf.bm[q][q] : pick(sub, bf.bm[0][0], bf.bm[1][1], bf.bm[2][2])) * xc[q];
+            if (first) v += bf.bm[0][2] * x3;
+            xc[q] = v;
         }
-    } else {
-#pragma unroll
-        for (int c = 0; c < 3; c++) xp[c] = xw[c];
     }
-    const double x1min = -0.5 * g.dx, x2min = -0.5 * g.dy, x3min = -0.5 * g.dz;
-    const double x1max = x1min + g.lx, x2max = x2min + g.ly, x3max = x3min + g.lz;
-    if (xp[0] < x1min) xp[0] = xp[0] + g.lx;
-    if (xp[0] >= x1max) xp[0] = xp[0] - g.lx;
-    if (xp[1] < x2min) xp[1] = xp[1] + g.ly;
-    if (xp[1] >= x2max) xp[1] = xp[1] - g.ly;
-    if (xp[2] < x3min) xp[2] = xp[2] + g.lz;
-    if (xp[2] > x3max) xp[2] = xp[2] - g.lz;
-    const double ymin = -(0.5 * g.dy), ymax = (double)g.ny * g.dy - (0.5 * g.dy);
-    const double zmin = -(0.5 * g.dz), zmax = (double)g.nz * g.dz - (0.5 * g.dz);
-    if (!(xp[1] >= ymin && xp[1] < ymax && xp[2] >= zmin && xp[2] < zmax)) atomicOr(&ck->status, PD_ST_LOST);
+    if (NC == 1 && (sub >= 3 || !valid)) return;
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        P.xp[c][n] = xp[c]; P.up[c][n] = up[c]; P.uprk[c][n] = ur[c]; P.prk[c][n] = pr[c];
+    for (int q = 0; q < NC; q++) {
+        const int c = NC == 3 ? q : sub;
+        const double d = pick(c, g.dx, g.dy, g.dz), l = pick(c, g.lx, g.ly, g.lz);
+        const double lo = -0.5 * d, hi = lo + l;
+        double x = xc[q];
+        if (x < lo) x = x + l;
+        if (c < 2 ? x >= hi : x > hi) x = x - l;
+        // lost: outside the domain after the wrap (components 2 and 3)
+        const double mn = -(0.5 * d), mx = (double)(c == 1 ? g.ny : g.nz) * d - (0.5 * d);
+        if (c > 0 && !(x >= mn && x < mx)) atomicOr(&ck->status, PD_ST_LOST);
+        pick(c, P.xp)[n] = x;
+        pick(c, P.up)[n] = up[q];
+        pick(c, P.uprk)[n] = ur[q];
+        if (dpv > 0.0 || release) pick(c, P.prk)[n] = pr[q];
     }
 }
 

@@ -187,6 +187,19 @@ cudaError_t launch_convert(const float2* in, double2* out, long long n, cudaStre
     return cudaGetLastError();
 }
 
+template <class T> __global__ void k_phys_component(const T* __restrict__ phys, int c, double* __restrict__ out, long long n) {
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
+        out[q] = (double)phys[4 * q + c];
+}
+cudaError_t launch_phys_component(const double* phys, int c, double* out, long long n, cudaStream_t st) {
+    k_phys_component<<<conv_blocks(n), 256, 0, st>>>(phys, c, out, n);
+    return cudaGetLastError();
+}
+cudaError_t launch_phys_component(const float* phys, int c, double* out, long long n, cudaStream_t st) {
+    k_phys_component<<<conv_blocks(n), 256, 0, st>>>(phys, c, out, n);
+    return cudaGetLastError();
+}
+
 #define PD_INST(T)                                                                                       \
     template cudaError_t configure_kernels<T>(const Geo&);                                               \
     template cudaError_t launch_zpass_inv<T>(const Geo&, const Member<T>*, int, int, cudaStream_t, const ZMaps*); \

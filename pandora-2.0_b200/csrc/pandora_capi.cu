@@ -291,7 +291,7 @@ extern "C" int pandora_create(const pandora_params* p, pandora_handle** out) {
     PD_ALLOC(h->fbuf, ce * 6 * (size_t)g.S);
     PD_ALLOC(h->F.zb, ce * (size_t)pass_fields(g) * g.nz * g.nkj * g.nkip);
     PD_ALLOC(h->F.yb, ce * (size_t)pass_fields(g) * g.nz * g.ny * g.nkip);
-    if (h->particles_on) PD_ALLOC(h->F.phys, ce / 2 * 3 * (size_t)g.R);
+    if (h->particles_on) PD_ALLOC(h->F.phys, ce / 2 * 4 * (size_t)g.R);
     PD_ALLOC(h->F.forcing, sizeof(double2) * 3 * (size_t)h->nforce);
     PD_ALLOC(h->tw, ce * (size_t)(g.nx + g.ny + g.nz));
     PD_ALLOC(h->clock, sizeof(Clock));
@@ -1004,18 +1004,14 @@ extern "C" int pandora_get_physical_velocity(pandora_handle* h, double* u1, doub
     if (!h->F.phys) return PANDORA_ERR_UNSUPPORTED;
     cudaSetDevice(h->dev);
     double* d[3] = {u1, u2, u3};
-    if (h->mixed) {   // stored FP32: widened on the host
-        std::vector<float> tmp((size_t)h->g.R);
-        for (int c = 0; c < 3; c++) {
-            PD_CK(cudaMemcpyAsync(tmp.data(), h->Ff.phys + c * h->g.R, sizeof(float) * h->g.R,
-                                  cudaMemcpyDeviceToHost, h->st));
-            PD_CK(cudaStreamSynchronize(h->st));
-            for (long long q = 0; q < h->g.R; q++) d[c][q] = tmp[(size_t)q];
-        }
-        return PANDORA_OK;
+    // the stored field is interleaved; each component passes through the z-pencil buffer (free
+    // between steps, 6 NZ NKJ NKIP values), widened to FP64 there in the mixed form
+    double* const scr = reinterpret_cast<double*>(h->F.zb);
+    for (int c = 0; c < 3; c++) {
+        if (h->mixed) PD_CK(launch_phys_component(h->Ff.phys, c, scr, h->g.R, h->st));
+        else PD_CK(launch_phys_component(h->F.phys, c, scr, h->g.R, h->st));
+        PD_CK(cudaMemcpyAsync(d[c], scr, sizeof(double) * h->g.R, cudaMemcpyDeviceToHost, h->st));
     }
-    for (int c = 0; c < 3; c++)
-        PD_CK(cudaMemcpyAsync(d[c], h->F.phys + c * h->g.R, sizeof(double) * h->g.R, cudaMemcpyDeviceToHost, h->st));
     PD_CK(cudaStreamSynchronize(h->st));
     return PANDORA_OK;
 }
@@ -1305,7 +1301,7 @@ extern "C" int pandora_batch_bytes(const pandora_params* p, int32_t capacity, in
     const long long np = p->p_track_part ? p->p_np_global : 0;
     const long long nfb = (p->f_type == PANDORA_F_SHEAR_DNS && p->ns_deformed == PANDORA_NS_R_CONV) ? 9 : 6;
     long long per = ce * 6 * S + ce * nfb * nz * nkj * nkip + ce * nfb * nz * ny * nkip + ce * (nx + ny + nz);
-    if (p->p_track_part) per += ce / 2 * 3 * R + 2 * 8 * 14 * np + 4 * np;
+    if (p->p_track_part) per += ce / 2 * 4 * R + 2 * 8 * 14 * np + 4 * np;
     per += 1 << 20;   // clock, forcing, shells, member descriptors, allocator granularity
     *bytes = per * capacity;
     return PANDORA_OK;

@@ -98,7 +98,7 @@ template <class T> struct FieldsT {
     C* rk[3];
     C* zb;              // [6][NZ][NKJ][NKIP]  after the z pass
     C* yb;              // [6][NZ][NY][NKIP]   after the y pass; NL written into fields 0..2
-    T* phys;            // [3][NZ][NY][NX]     physical velocity (particles), may be null
+    T* phys;            // [NZ][NY][NX][4]     physical velocity and a pad (particles), may be null
     double2* forcing;   // [3][NK+1][2NK+1][2NK+1]
     const C *tw_x, *tw_y, *tw_z;
     Clock* clock;
@@ -284,6 +284,9 @@ cudaError_t launch_particle_sort(const Geo& g, const Particles& p, const PartSor
 // n complex values from one precision to the other (FP64 <-> FP32 at the boundary).
 cudaError_t launch_convert(const double2* in, float2* out, long long n, cudaStream_t st);
 cudaError_t launch_convert(const float2* in, double2* out, long long n, cudaStream_t st);
+// One component of the interleaved physical velocity (n points) as FP64 values.
+cudaError_t launch_phys_component(const double* phys, int c, double* out, long long n, cudaStream_t st);
+cudaError_t launch_phys_component(const float* phys, int c, double* out, long long n, cudaStream_t st);
 size_t shell_words(const Geo& g);
 
 // Shared-memory configuration (set once per process per device).

@@ -76,6 +76,15 @@ __device__ __forceinline__ void prefetch_l2(const void* p, size_t bytes) {
     if (e > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(e - a)) : "memory");
 }
 
+// The physical velocity of one grid point, for the particle gather: the three components
+// and a pad in one 32-byte (FP64) or 16-byte (FP32) store.
+__device__ __forceinline__ void store_point(double* p, double a, double b, double c) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(0.0) : "memory");
+}
+__device__ __forceinline__ void store_point(float* p, float a, float b, float c) {
+    *reinterpret_cast<float4*>(p) = make_float4(a, b, c, 0.0f);
+}
+
 template <int N> constexpr int xps() {
     return (N == 16 || N == 32 || N == 48) ? 2
          : ((N == 24 || N == 64 || N == 96) ? 3 : ((N == 384 || N == 512 || N == 1024) ? 5 : 4));
@@ -216,6 +225,7 @@ __global__ void __launch_bounds__(32, RS ? XCfgStats<NX, T>::ctas() : XCfg<NX, T
     constexpr int NKI = NX / 3 + 1, NKIP = (NKI + 7) / 8 * 8;   // g.nki, g.nkip
     const long long fstride = lines * NKIP;       // distance between fields in yb
     C* b = F.yb + q * NKIP;
+    T* const phys = F.phys + 4 * (q * NX);   // the line's physical velocity
     BFT<T> bf;
     if (g.shear) bf = bf_as<T>(make_bf(g, F.clock));
     double racc[RS ? kRsSums : 1], rmax[RS ? kRsMax : 1];
@@ -297,11 +307,7 @@ __global__ void __launch_bounds__(32, RS ? XCfgStats<NX, T>::ctas() : XCfg<NX, T
             for (int r = 0; r < RL; r++) {
                 const int n = lane + r * NRL;
                 const T u1 = v0[r].x, u2 = v0[r].y, u3 = v1[r].x, w1 = v1[r].y, w2 = v2[r].x, w3 = v2[r].y;
-                if (want_phys && valid) {
-                    F.phys[q * NX + n] = u1;
-                    F.phys[g.R + q * NX + n] = u2;
-                    F.phys[2 * g.R + q * NX + n] = u3;
-                }
+                if (want_phys && valid) store_point(phys + 4 * n, u1, u2, u3);
                 if (want_cfl) umax = fmax(umax, fabs(u1) + fabs(u2) + fabs(u3));
                 T n3;
                 v0[r] = nl_point<T, C>(bf, g.shear && !g.rrot, u1, u2, u3, w1, w2, w3, n3);
@@ -330,11 +336,7 @@ __global__ void __launch_bounds__(32, RS ? XCfgStats<NX, T>::ctas() : XCfg<NX, T
                 const C* e = s + prow<XPS>(n);
                 const C a = e[0], bb = e[XAS];
                 const T u1 = a.x, u2 = a.y, u3 = bb.x, w1 = bb.y, w2 = v[r].x, w3 = v[r].y;
-                if (want_phys) {
-                    F.phys[q * NX + n] = u1;
-                    F.phys[g.R + q * NX + n] = u2;
-                    F.phys[2 * g.R + q * NX + n] = u3;
-                }
+                if (want_phys) store_point(phys + 4 * n, u1, u2, u3);
                 if (want_cfl) umax = fmax(umax, fabs(u1) + fabs(u2) + fabs(u3));
                 if constexpr (RS) rs_point(racc, rmax, g.shear, brs, u1, u2, u3, w1, w2, w3);
                 v[r] = nl_point<T, C>(bf, g.shear && !g.rrot, u1, u2, u3, w1, w2, w3, n3[r]);
@@ -357,11 +359,7 @@ __global__ void __launch_bounds__(32, RS ? XCfgStats<NX, T>::ctas() : XCfg<NX, T
             C* e = s + prow<XPS>(n);
             const C a = e[0], bb = e[XAS], c = e[2 * XAS];
             const T u1 = a.x, u2 = a.y, u3 = bb.x, w1 = bb.y, w2 = c.x, w3 = c.y;
-            if (want_phys && valid) {
-                F.phys[q * NX + n] = u1;
-                F.phys[g.R + q * NX + n] = u2;
-                F.phys[2 * g.R + q * NX + n] = u3;
-            }
+            if (want_phys && valid) store_point(phys + 4 * n, u1, u2, u3);
             if (want_cfl) umax = fmax(umax, fabs(u1) + fabs(u2) + fabs(u3));
             if constexpr (RS) rs_point(racc, rmax, g.shear, brs, u1, u2, u3, w1, w2, w3);
             T n3;
@@ -467,6 +465,7 @@ __global__ void __launch_bounds__(32 * ConvCfg<NX, T>::NW, 1) k_xpass_conv(const
     constexpr int NKI = NX / 3 + 1, NKIP = (NKI + 7) / 8 * 8;   // g.nki, g.nkip
     const long long fstride = lines * NKIP;
     C* b = F.yb + q * NKIP;
+    T* const phys = F.phys + 4 * (q * NX);   // the line's physical velocity
     const BFT<T> bf = bf_as<T>(make_bf(g, F.clock));
     // the Hermitian extension of the half spectra of fields fa and fb into array p, as K3;
     // xa, xb: i m times the field (its x derivative)
@@ -499,11 +498,7 @@ __global__ void __launch_bounds__(32 * ConvCfg<NX, T>::NW, 1) k_xpass_conv(const
         C* e = s + prow<XPS>(n);
         const C a = e[0], c1 = e[XAS];
         const T u[3] = {a.x, a.y, c1.x};
-        if (want_phys) {
-            F.phys[q * NX + n] = u[0];
-            F.phys[g.R + q * NX + n] = u[1];
-            F.phys[2 * g.R + q * NX + n] = u[2];
-        }
+        if (want_phys) store_point(phys + 4 * n, u[0], u[1], u[2]);
         if (want_cfl) umax = fmax(umax, fabs(u[0]) + fabs(u[1]) + fabs(u[2]));
         T v[3];
 #pragma unroll
