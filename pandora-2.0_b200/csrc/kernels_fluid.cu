@@ -40,8 +40,8 @@ __device__ __forceinline__ void neumaier(double& s, double& c, double x) {
 // [b R / G, (b+1) R / G) of (i, j), one warp per row, 32 consecutive k at a time.
 // Along a row the shell index is monotone on each half of k, so the lanes of a shell
 // form runs; a segmented sum over the runs (a fixed shuffle tree) leaves one
-// shared-memory update per run.  Each CTA writes its sums to the free y-pencil
-// buffer (G x nsh doubles).  k_stats_reduce adds the G partial sums of every output
+// shared-memory update per run.  Each CTA writes its sums to F.part (G x nsh doubles: a buffer
+// of their own, so that the statistics may run beside K1 to K5a).  k_stats_reduce adds the G partial sums of every output
 // word in CTA order with Neumaier compensation: the cross-CTA sum, where the terms
 // are many and of every size, carries about one rounding, and the result does not
 // depend on the order in which CTAs finish.
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256) k_stats(const __grid_constant__ MemberSet
         sp[threadIdx.x] = a;
     }
     __syncthreads();
-    double* part = reinterpret_cast<double*>(F.yb) + (size_t)blockIdx.x * nsh;
+    double* part = F.part + (size_t)blockIdx.x * nsh;
     for (int q = threadIdx.x; q < nsh; q += blockDim.x) part[q] = sh[q];
 }
 
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256) k_stats_reduce(const __grid_constant__ Me
     __shared__ double ps[8][32], pc[8][32];
     const int lane = threadIdx.x & 31, v = threadIdx.x >> 5;
     const int w = blockIdx.x * 32 + lane;
-    const double* part = reinterpret_cast<const double*>(F.yb);
+    const double* part = F.part;
     double s = 0.0, c = 0.0;
     if (w < nsh)
         for (int b = v; b < G; b += 8) neumaier(s, c, part[(size_t)b * nsh + w]);
@@ -208,8 +208,22 @@ __device__ int normal_pair(uint64_t key, uint64_t call, double& r1, double& r2) 
     return 0;
 }
 
+// simtime after stage s: t0 + {1/3, 3/4, 1} dt (src/pg_rk3.f90:109-127); the step
+// counter advances after stage 3.
+__device__ __forceinline__ void advance_clock(const Geo& g, Clock* ck, int stage) {
+    if (stage == 1) ck->simtime = ck->t0 + (1.0 / 3.0) * ck->dt;
+    else if (stage == 2) ck->simtime = ck->t0 + (3.0 / 4.0) * ck->dt;
+    else ck->simtime = ck->t0 + ck->dt;
+    if (g.shear) update_b(g, ck->tstep, ck->simtime, ck->b13, ck->bi13);
+    if (stage == 3) {
+        ck->t0 = ck->simtime;
+        ck->tstep += 1;
+    }
+}
+
+// advance: the kernel ends by advancing the stage's time (scalars_advance).
 template <class T, int CAP>
-__global__ void __launch_bounds__(256) k_stage_scalars(const __grid_constant__ MemberSet<T, CAP> ms, int stage) {
+__global__ void __launch_bounds__(256) k_stage_scalars(const __grid_constant__ MemberSet<T, CAP> ms, int stage, int advance) {
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.x];
     if (!mm.active) return;
     if constexpr (CAP > 1) {   // a batch slot between members
@@ -249,6 +263,8 @@ __global__ void __launch_bounds__(256) k_stage_scalars(const __grid_constant__ M
     const int tstep = ck->tstep;
     if (tstep >= fp.stop) {
         for (long long q = tid; q < 3 * fstride; q += blockDim.x) F.forcing[q] = mk(0.0, 0.0);
+        __syncthreads();   // every thread has read the step number
+        if (advance && tid == 0) advance_clock(g, ck, stage);
         return;
     }
     const long long calls = fp.calls_per_stage;
@@ -314,10 +330,9 @@ __global__ void __launch_bounds__(256) k_stage_scalars(const __grid_constant__ M
     }
     __syncthreads();
     for (int q = tid; q < 3 * plane; q += blockDim.x) ff[(q / plane) * fstride + q % plane] = pl[q];
+    if (advance && tid == 0) advance_clock(g, ck, stage);   // behind the barriers that follow its reads
 }
 
-// simtime after stage s: t0 + {1/3, 3/4, 1} dt (src/pg_rk3.f90:109-127); the step
-// counter advances after stage 3.
 template <class T, int CAP>
 __global__ void k_advance_time(const __grid_constant__ MemberSet<T, CAP> ms, int stage) {
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.x];
@@ -325,18 +340,7 @@ __global__ void k_advance_time(const __grid_constant__ MemberSet<T, CAP> ms, int
     if constexpr (CAP > 1) {   // a batch slot between members
         if (mm.F.clock->status & PD_ST_IDLE) return;
     }
-    const FieldsT<T> F = mm.F;
-    const Geo g = mm.g;
-
-    Clock* ck = F.clock;
-    if (stage == 1) ck->simtime = ck->t0 + (1.0 / 3.0) * ck->dt;
-    else if (stage == 2) ck->simtime = ck->t0 + (3.0 / 4.0) * ck->dt;
-    else ck->simtime = ck->t0 + ck->dt;
-    if (g.shear) update_b(g, ck->tstep, ck->simtime, ck->b13, ck->bi13);
-    if (stage == 3) {
-        ck->t0 = ck->simtime;
-        ck->tstep += 1;
-    }
+    advance_clock(mm.g, mm.F.clock, stage);
 }
 
 // A fresh clock (step tstep at time t, frame tensors b13 / bi13), set on the
@@ -352,6 +356,16 @@ __global__ void k_reset_clock(Clock* ck, int tstep, double t, double b13, double
 }
 cudaError_t launch_reset_clock(Clock* ck, int tstep, double t, double b13, double bi13, cudaStream_t st) {
     k_reset_clock<<<1, 1, 0, st>>>(ck, tstep, t, b13, bi13);
+    return cudaGetLastError();
+}
+__global__ void k_set_clock(Clock* ck, int tstep, double t, int frame, double b13, double bi13) {
+    ck->tstep = tstep;
+    ck->simtime = t;
+    ck->t0 = t;
+    if (frame) { ck->b13 = b13; ck->bi13 = bi13; }
+}
+cudaError_t launch_set_clock(Clock* ck, int tstep, double t, bool frame, double b13, double bi13, cudaStream_t st) {
+    k_set_clock<<<1, 1, 0, st>>>(ck, tstep, t, frame ? 1 : 0, b13, bi13);
     return cudaGetLastError();
 }
 // Marks a batch slot free (batched kernels skip it from the next launch on).
@@ -650,19 +664,16 @@ __global__ void k_check_finite(const __grid_constant__ MemberSet<T, CAP> ms) {
 // host launchers
 // ---------------------------------------------------------------------------
 
-// Statistics of every member into its own F.shell (shell_words doubles); the
-// per-CTA partial sums live in the member's y-pencil buffer, free at stage 1 and
-// between steps.
-template <class T>
-cudaError_t launch_stats(const Geo& g, const Member<T>* M, int B, double* shell, cudaStream_t st) {
-    (void)shell;
-    const size_t nsh = shell_words(g);
+int stats_ctas(const Geo& g) {
     const long long rows = (long long)g.nki * g.nkj;
-    const size_t yb_bytes = sizeof(typename Cplx<T>::type) * 6 * (size_t)g.nz * g.ny * g.nkip;
-    long long G = std::min<long long>(4LL * sm_count(), std::max<long long>(1, rows / 8));
-    G = std::min<long long>(G, (long long)(yb_bytes / (sizeof(double) * nsh)));
-    if (G < 1) return cudaErrorInvalidValue;
-    const int gi = (int)G;
+    return (int)std::min<long long>(4LL * sm_count(), std::max<long long>(1, rows / 8));
+}
+
+// Statistics of every member into its own F.shell (shell_words doubles).
+template <class T>
+cudaError_t launch_stats(const Geo& g, const Member<T>* M, int B, cudaStream_t st) {
+    const size_t nsh = shell_words(g);
+    const int gi = stats_ctas(g);
     cudaError_t e = for_member_sets(M, B, [&](const auto& ms, int nm) {
         k_stats<T, PD_CAP(ms)><<<dim3((unsigned)gi, nm), 256, sizeof(double) * nsh, st>>>(ms, gi);
     });
@@ -704,10 +715,10 @@ cudaError_t configure_fluid_kernels(const Geo& g, const ForceParams& fp) {
 }
 
 template <class T>
-cudaError_t launch_stage_scalars(const Geo& g, const Member<T>* M, int B, const ForceParams& fp, int stage,
+cudaError_t launch_stage_scalars(const Geo& g, const Member<T>* M, int B, const ForceParams& fp, int stage, bool advance,
                                  cudaStream_t st) {
     return for_member_sets(M, B, [&](const auto& ms, int nm) {
-        k_stage_scalars<T, PD_CAP(ms)><<<nm, 256, stage_scalars_smem(g, fp), st>>>(ms, stage);
+        k_stage_scalars<T, PD_CAP(ms)><<<nm, 256, stage_scalars_smem(g, fp), st>>>(ms, stage, advance ? 1 : 0);
     });
 }
 
@@ -791,8 +802,8 @@ template <class T> cudaError_t launch_xcorr_cospec(const Member<T>& m, double* P
 
 #define PD_INST(T)                                                                                   \
     template cudaError_t launch_xcorr_cospec<T>(const Member<T>&, double*, cudaStream_t);            \
-    template cudaError_t launch_stats<T>(const Geo&, const Member<T>*, int, double*, cudaStream_t);  \
-    template cudaError_t launch_stage_scalars<T>(const Geo&, const Member<T>*, int, const ForceParams&, int, \
+    template cudaError_t launch_stats<T>(const Geo&, const Member<T>*, int, cudaStream_t);           \
+    template cudaError_t launch_stage_scalars<T>(const Geo&, const Member<T>*, int, const ForceParams&, int, bool, \
                                                  cudaStream_t);                                      \
     template cudaError_t launch_advance_time<T>(const Geo&, const Member<T>*, int, int, cudaStream_t); \
     template cudaError_t launch_check_finite<T>(const Geo&, const Member<T>*, int, cudaStream_t);    \

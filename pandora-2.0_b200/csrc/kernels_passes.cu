@@ -96,7 +96,8 @@ template <class T> cudaError_t launch_ypass_fwd(const Geo& g, const Member<T>* M
 }
 
 template <class T>
-cudaError_t launch_zpass_fwd_update(const Geo& g, const Member<T>* M, int B, int stage, int mode, cudaStream_t st) {
+cudaError_t launch_zpass_fwd_update(const Geo& g, const Member<T>* M, int B, int stage, int mode, cudaStream_t st,
+                                    cudaEvent_t before_update) {
     cudaError_t e = cudaErrorInvalidValue;
     switch (g.nz) {
 #define PD_L(N)                                    \
@@ -108,6 +109,7 @@ cudaError_t launch_zpass_fwd_update(const Geo& g, const Member<T>* M, int B, int
     default: return cudaErrorInvalidValue;
     }
     if (e || mode == 1) return e;
+    if (before_update && (e = cudaStreamWaitEvent(st, before_update, 0)) != cudaSuccess) return e;
     return for_member_sets(M, B, [&](const auto& ms, int nb) {
         constexpr int CAP = std::decay_t<decltype(ms)>::cap;
         const dim3 grid((unsigned)((g.S + 255) / 256), nb);
@@ -207,7 +209,7 @@ cudaError_t launch_phys_component(const float* phys, int c, double* out, long lo
     template cudaError_t launch_xpass<T>(const Geo&, const Member<T>*, int, int, int, cudaStream_t);     \
     template cudaError_t launch_xpass_stats<T>(const Geo&, const Member<T>*, double*, cudaStream_t);    \
     template cudaError_t launch_ypass_fwd<T>(const Geo&, const Member<T>*, int, cudaStream_t);           \
-    template cudaError_t launch_zpass_fwd_update<T>(const Geo&, const Member<T>*, int, int, int, cudaStream_t);
+    template cudaError_t launch_zpass_fwd_update<T>(const Geo&, const Member<T>*, int, int, int, cudaStream_t, cudaEvent_t);
 PD_INST(double)
 PD_INST(float)
 #undef PD_INST

@@ -25,7 +25,7 @@ struct pandora_handle {
     cudaStream_t own = nullptr;
     cudaStream_t st = nullptr;
     cudaStream_t side = nullptr;      // particle branch of a stage (forked from st, joined back)
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_side = nullptr;
     int timing = 0;                   // pandora_set_pass_timing: bit p-1 times pass p
     bool timed[3][6] = {};
     cudaEvent_t tev[3][6][2] = {};
@@ -37,8 +37,9 @@ struct pandora_handle {
     void* tw = nullptr;               // tw_x | tw_y | tw_z
     Clock* clock = nullptr;
     Clock* clock_host = nullptr;      // pinned mirror
-    double* shell_step = nullptr;     // stats of the state at stage 1 of the last step
+    double* shell_step = nullptr;     // stats of the state at stage 1 of the last step (holds the next two)
     double* shell_now = nullptr;      // stats of pandora_stats()
+    double* shell_part = nullptr;     // the statistics' partial sums
     double* shell_host = nullptr;     // pinned
     std::vector<double> dens_mod;     // [kkmax + 1]
     long long nforce = 0;             // complex entries per forcing component
@@ -161,7 +162,7 @@ static void release(pandora_handle* h) {
     if (h->graph) cudaGraphDestroy(h->graph);
     cudaFree(h->fbuf); cudaFree(h->F.zb); cudaFree(h->F.yb); cudaFree(h->F.phys);
     cudaFree(h->F.forcing); cudaFree(h->tw); cudaFree(h->clock); cudaFree(h->shell_step);
-    cudaFree(h->shell_now); cudaFree(h->pbuf); cudaFree(h->pbuf2); cudaFree(h->nlbuf); cudaFree(h->rsbuf);
+    cudaFree(h->pbuf); cudaFree(h->pbuf2); cudaFree(h->nlbuf); cudaFree(h->rsbuf);
     cudaFree(h->sort.key); cudaFree(h->sort.count); cudaFree(h->sort.block_sums);
     if (h->clock_host) cudaFreeHost(h->clock_host);
     if (h->shell_host) cudaFreeHost(h->shell_host);
@@ -171,6 +172,7 @@ static void release(pandora_handle* h) {
                 if (e) cudaEventDestroy(e);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
+    if (h->ev_side) cudaEventDestroy(h->ev_side);
     if (h->side) cudaStreamDestroy(h->side);
     if (h->own) cudaStreamDestroy(h->own);
     delete h;
@@ -296,8 +298,9 @@ extern "C" int pandora_create(const pandora_params* p, pandora_handle** out) {
     PD_ALLOC(h->tw, ce * (size_t)(g.nx + g.ny + g.nz));
     PD_ALLOC(h->clock, sizeof(Clock));
     const size_t nsh = shell_words(g);
-    PD_ALLOC(h->shell_step, sizeof(double) * nsh);
-    PD_ALLOC(h->shell_now, sizeof(double) * nsh);
+    PD_ALLOC(h->shell_step, sizeof(double) * nsh * (2 + (size_t)stats_ctas(g)));
+    h->shell_now = h->shell_step + nsh;
+    h->shell_part = h->shell_now + nsh;
 #undef PD_ALLOC
     if (cudaMallocHost((void**)&h->clock_host, sizeof(Clock)) != cudaSuccess ||
         cudaMallocHost((void**)&h->shell_host, sizeof(double) * nsh) != cudaSuccess) {
@@ -306,7 +309,8 @@ extern "C" int pandora_create(const pandora_params* p, pandora_handle** out) {
     if ((e = cudaStreamCreateWithFlags(&h->own, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming)) != cudaSuccess) {
+        (e = cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&h->ev_side, cudaEventDisableTiming)) != cudaSuccess) {
         release(h); return cuda_fail(e, "cudaStreamCreate");
     }
     h->st = h->own;
@@ -365,6 +369,7 @@ extern "C" int pandora_create(const pandora_params* p, pandora_handle** out) {
     h->Ff.forcing = h->F.forcing;
     h->F.clock = h->clock; h->Ff.clock = h->clock;
     h->F.shell = h->shell_step; h->Ff.shell = h->shell_step;
+    h->F.part = h->shell_part; h->Ff.part = h->shell_part;
     h->sp.rk3_timestep = p->rk3_timestep; h->sp.f_type = p->f_type; h->sp.rk3_dt = p->rk3_dt;
     h->sp.rk3_cfl = p->rk3_cfl; h->sp.force_tf = p->force_tf; h->sp.f_deform_s = p->f_deform_s;
     h->sp.f_remesh_t = p->f_remesh_t;
@@ -636,7 +641,7 @@ template <class T> struct StepCtx {
     const ForceParams* fp;
     double* shell;
     cudaStream_t st, side;
-    cudaEvent_t ev_fork, ev_join;
+    cudaEvent_t ev_fork, ev_join, ev_side;
     const PartSort* sort;        // null: no per-step particle sort (batches)
     const Particles* sortP;      // the particles the sort reorders
     pandora_handle* timing;      // null: no pass timing
@@ -652,15 +657,21 @@ template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, 
     if (stage == 1 && g.shear) {
         PD_CK(launch_remesh(g, M, B, c.np, c.st)); n += part ? 2 : 1;
     }
+    // Beside the main stream (joined before what needs them): the spatial sort of the particles
+    // (before the advance), the statistics of stage 1 and, where no particle waits for dt, the
+    // stage's scalars (both before K5b, which changes u and reads dt and the forcing).  On the
+    // small grids, whose step is a chain of launches, these are a quarter of the chain.
     const bool sorted = stage == 1 && part && c.sort;
-    if (sorted) {   // the spatial sort runs beside the statistics and K1-K3, joined before the advance
+    if (stage == 1) {
         PD_CK(cudaEventRecord(c.ev_fork, c.st));
         PD_CK(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
+    }
+    if (sorted) {
         PD_CK(launch_particle_sort(g, *c.sortP, *c.sort, c.side, &n));
         PD_CK(cudaEventRecord(c.ev_join, c.side));
     }
-    if (stage == 1) {
-        PD_CK(launch_stats(g, M, B, c.shell, c.st)); n += 1;   // one kernel (plus a memset node)
+    if (stage == 1) {   // ahead of K1 where it first drops modes from u (DEALIASING 2/3)
+        PD_CK(launch_stats(g, M, B, g.dealias_cut > 0.0 ? c.st : c.side)); n += 1;   // two kernels, counted as one
     }
     // instrumentation: event pair around pass `ps` (1..6) when pass timing is on
     pandora_handle* h = c.timing;
@@ -680,7 +691,16 @@ template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, 
     PD_CK(mark(3, 0, c.st));
     PD_CK(launch_xpass(g, M, B, part ? 1 : 0, stage == 1 ? 1 : 0, c.st)); n++;
     PD_CK(mark(3, 1, c.st));
-    PD_CK(launch_stage_scalars(g, M, B, *c.fp, stage, c.st)); n++;
+    const bool adv = scalars_advance(g, c.np);
+    if (part) {
+        PD_CK(launch_stage_scalars(g, M, B, *c.fp, stage, adv, c.st)); n++;
+    } else {
+        PD_CK(cudaEventRecord(c.ev_fork, c.st));
+        PD_CK(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
+        PD_CK(launch_stage_scalars(g, M, B, *c.fp, stage, adv, c.side)); n++;
+    }
+    const bool side = stage == 1 || !part;   // work on the side stream to wait for
+    if (side) PD_CK(cudaEventRecord(c.ev_side, c.side));
     // The particle advance (it needs K3's physical velocity and the stage's dt) runs in
     // the main stream between K3 and K4: on a second stream beside K4/K5 it slowed them
     // by more than its own time (512^3 shear: K4 0.62 -> 0.85 ms beside a 0.08 ms advance).
@@ -694,9 +714,9 @@ template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, 
     PD_CK(launch_ypass_fwd(g, M, B, c.st)); n++;
     PD_CK(mark(4, 1, c.st));
     PD_CK(mark(5, 0, c.st));
-    PD_CK(launch_zpass_fwd_update(g, M, B, stage, 0, c.st)); n += 2;   // forward z FFT, RK update
+    PD_CK(launch_zpass_fwd_update(g, M, B, stage, 0, c.st, side ? c.ev_side : nullptr)); n += 2;   // forward z FFT, RK update
     PD_CK(mark(5, 1, c.st));
-    PD_CK(launch_advance_time(g, M, B, stage, c.st)); n++;
+    if (!adv) { PD_CK(launch_advance_time(g, M, B, stage, c.st)); n++; }
     if (nlaunch) *nlaunch += n;
     return PANDORA_OK;
 }
@@ -715,6 +735,7 @@ template <class T> static int enqueue_stage_t(pandora_handle* h, int stage, int*
     c.side = h->side;
     c.ev_fork = h->ev_fork;
     c.ev_join = h->ev_join;
+    c.ev_side = h->ev_side;
     c.sort = &h->sort;
     c.sortP = &h->P;
     c.timing = h;
@@ -757,18 +778,13 @@ static int status_to_rc(unsigned int st) {
     return PANDORA_OK;
 }
 
+// Step number, time and (shear) frame of the next step, set on the device in stream order: the
+// dt, ucfl and status there are kept and the host does not wait.
 static int set_clock(pandora_handle* h, int tstep, double simtime) {
-    // keep dt / ucfl / status from the device copy
-    PD_CK(cudaMemcpyAsync(h->clock_host, h->clock, sizeof(Clock), cudaMemcpyDeviceToHost, h->st));
-    PD_CK(cudaStreamSynchronize(h->st));
-    h->clock_host->tstep = tstep;
-    h->clock_host->simtime = simtime;
-    h->clock_host->t0 = simtime;
-    if (h->g.shear) {
-        // the frame of stage 1 of step tstep is the one g_RK3UpdateB set at the end of step tstep-1
-        update_b(h->g, tstep - 1, simtime, h->clock_host->b13, h->clock_host->bi13);
-    }
-    PD_CK(cudaMemcpyAsync(h->clock, h->clock_host, sizeof(Clock), cudaMemcpyHostToDevice, h->st));
+    double b13 = 0.0, bi13 = 0.0;
+    // the frame of stage 1 of step tstep is the one g_RK3UpdateB set at the end of step tstep-1
+    if (h->g.shear) update_b(h->g, tstep - 1, simtime, b13, bi13);
+    PD_CK(launch_set_clock(h->clock, tstep, simtime, h->g.shear != 0, b13, bi13, h->st));
     return PANDORA_OK;
 }
 
@@ -853,12 +869,12 @@ extern "C" int pandora_stats(pandora_handle* h, double* ek, int32_t kkmax, doubl
         FieldsT<float> Fs = h->Ff;
         Fs.shell = h->shell_now;
         const Member<float> mv = member_of<float>(h, Fs);
-        PD_CK(launch_stats(h->g, &mv, 1, h->shell_now, h->st));
+        PD_CK(launch_stats(h->g, &mv, 1, h->st));
     } else {
         Fields Fs = h->F;
         Fs.shell = h->shell_now;
         const Member<double> mv = member_of<double>(h, Fs);
-        PD_CK(launch_stats(h->g, &mv, 1, h->shell_now, h->st));
+        PD_CK(launch_stats(h->g, &mv, 1, h->st));
     }
     const size_t nsh = shell_words(h->g);
     PD_CK(cudaMemcpyAsync(h->shell_host, h->shell_now, sizeof(double) * nsh, cudaMemcpyDeviceToHost, h->st));
@@ -1041,7 +1057,7 @@ extern "C" int pandora_launches_per_step(pandora_handle* h, int32_t* n) {
     if (!h->launches_per_step) {
         // count without launching: same sequence as enqueue_step
         const bool part = h->particles_on && h->P.np > 0;
-        h->launches_per_step = 1 + 3 * (8 + (part ? 1 : 0)) + (part ? 5 : 0) + (h->g.shear ? (part ? 2 : 1) : 0);
+        h->launches_per_step = 1 + 3 * (8 + (part ? 1 : 0) - (scalars_advance(h->g, part ? h->P.np : 0) ? 1 : 0)) + (part ? 5 : 0) + (h->g.shear ? (part ? 2 : 1) : 0);
     }
     *n = h->launches_per_step;
     return PANDORA_OK;
@@ -1095,7 +1111,7 @@ template <class T> static int profile_pass_t(pandora_handle* h, int32_t pass, in
             if (!part) return PANDORA_ERR_INVALID_ARG;
             PD_CK(launch_particles(h->g, M, 1, h->P.np, h->pp.order, 2, h->st));
             break;
-        case 7: PD_CK(launch_stats(h->g, Mv, 1, h->shell_now, h->st)); break;
+        case 7: PD_CK(launch_stats(h->g, Mv, 1, h->st)); break;
         default: return PANDORA_ERR_INVALID_ARG;
         }
     }
@@ -1183,7 +1199,7 @@ struct pandora_batch {
     double* shell = nullptr;               // [cap][shell_words]
     size_t nsh = 0;
     cudaStream_t st = nullptr, side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_side = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int launches_per_step = 0;
@@ -1202,6 +1218,7 @@ static void batch_release(pandora_batch* b) {
     cudaFree(b->shell);
     if (b->ev_fork) cudaEventDestroy(b->ev_fork);
     if (b->ev_join) cudaEventDestroy(b->ev_join);
+    if (b->ev_side) cudaEventDestroy(b->ev_side);
     if (b->side) cudaStreamDestroy(b->side);
     if (b->st) cudaStreamDestroy(b->st);
     delete b;
@@ -1283,6 +1300,7 @@ template <class T> static int batch_enqueue_step(pandora_batch* b, int* nlaunch)
     c.side = b->side;
     c.ev_fork = b->ev_fork;
     c.ev_join = b->ev_join;
+    c.ev_side = b->ev_side;
     for (int s = 1; s <= 3; s++) {
         int rc = enqueue_stage_ctx(c, s, nlaunch);
         if (rc) return rc;
@@ -1302,6 +1320,7 @@ extern "C" int pandora_batch_bytes(const pandora_params* p, int32_t capacity, in
     const long long nfb = (p->f_type == PANDORA_F_SHEAR_DNS && p->ns_deformed == PANDORA_NS_R_CONV) ? 9 : 6;
     long long per = ce * 6 * S + ce * nfb * nz * nkj * nkip + ce * nfb * nz * ny * nkip + ce * (nx + ny + nz);
     if (p->p_track_part) per += ce / 2 * 4 * R + 2 * 8 * 14 * np + 4 * np;
+    per += 8 * (3 * (kkmax_of(p) + 1) + 3) * 592LL;   // the statistics' partial sums, at most
     per += 1 << 20;   // clock, forcing, shells, member descriptors, allocator granularity
     *bytes = per * capacity;
     return PANDORA_OK;
@@ -1325,7 +1344,8 @@ extern "C" int pandora_batch_create(const pandora_params* cls, int32_t capacity,
     if ((e = cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming)) != cudaSuccess) {
+        (e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&b->ev_side, cudaEventDisableTiming)) != cudaSuccess) {
         batch_release(b); return cuda_fail(e, "batch streams");
     }
     b->m.assign(capacity, nullptr);

@@ -103,6 +103,7 @@ template <class T> struct FieldsT {
     const C *tw_x, *tw_y, *tw_z;
     Clock* clock;
     double* shell;      // [3*(kkmax+1) + 3] shell sums (e, d), p11,p22,p33, mode counts
+    double* part;       // [stats_ctas][3*(kkmax+1) + 3] partial shell sums of the statistics' CTAs
 };
 using Fields = FieldsT<double>;
 
@@ -248,11 +249,12 @@ template <class T>
 cudaError_t launch_xpass(const Geo& g, const Member<T>* M, int B, int want_phys, int want_cfl, cudaStream_t st);
 template <class T> cudaError_t launch_ypass_fwd(const Geo& g, const Member<T>* M, int B, cudaStream_t st);
 template <class T>
-cudaError_t launch_zpass_fwd_update(const Geo& g, const Member<T>* M, int B, int stage, int mode, cudaStream_t st);
+cudaError_t launch_zpass_fwd_update(const Geo& g, const Member<T>* M, int B, int stage, int mode, cudaStream_t st,
+                                    cudaEvent_t before_update = nullptr);   // an event K5b waits for, K5a not
 template <class T>
-cudaError_t launch_stats(const Geo& g, const Member<T>* M, int B, double* shell, cudaStream_t st);
+cudaError_t launch_stats(const Geo& g, const Member<T>* M, int B, cudaStream_t st);
 template <class T>
-cudaError_t launch_stage_scalars(const Geo& g, const Member<T>* M, int B, const ForceParams& fp, int stage,
+cudaError_t launch_stage_scalars(const Geo& g, const Member<T>* M, int B, const ForceParams& fp, int stage, bool advance,
                                  cudaStream_t st);
 template <class T> cudaError_t launch_advance_time(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st);
 template <class T>
@@ -276,6 +278,8 @@ template <class T> cudaError_t launch_xcorr_cospec(const Member<T>& m, double* P
 // form converts it), particle initialisation and the per-step spatial sort.
 cudaError_t launch_init_fluid(const Geo& g, const Fields& f, const InitParams& ip, cudaStream_t st);
 cudaError_t launch_reset_clock(Clock* ck, int tstep, double t, double b13, double bi13, cudaStream_t st);
+// Step number and time of the next step (and the frame, where `frame`), the rest of the clock kept.
+cudaError_t launch_set_clock(Clock* ck, int tstep, double t, bool frame, double b13, double bi13, cudaStream_t st);
 cudaError_t launch_set_idle(Clock* ck, cudaStream_t st);
 cudaError_t launch_init_particles(const Geo& g, const Particles& p, uint64_t key, double dia,
                                   cudaStream_t st);
@@ -288,6 +292,11 @@ cudaError_t launch_convert(const float2* in, double2* out, long long n, cudaStre
 cudaError_t launch_phys_component(const double* phys, int c, double* out, long long n, cudaStream_t st);
 cudaError_t launch_phys_component(const float* phys, int c, double* out, long long n, cudaStream_t st);
 size_t shell_words(const Geo& g);
+// CTAs of the statistics kernel, the rows of FieldsT::part.
+int stats_ctas(const Geo& g);
+// Does k_stage_scalars also advance the stage's time (else launch_advance_time does)?  Flows
+// whose K5b and particles read neither the frame nor the step number after it.
+inline bool scalars_advance(const Geo& g, long long np) { return !g.shear && np == 0; }
 
 // Shared-memory configuration (set once per process per device).
 template <class T> cudaError_t configure_kernels(const Geo& g);
