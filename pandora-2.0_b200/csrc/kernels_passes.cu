@@ -112,7 +112,7 @@ cudaError_t launch_zpass_fwd_update(const Geo& g, const Member<T>* M, int B, int
     if (before_update && (e = cudaStreamWaitEvent(st, before_update, 0)) != cudaSuccess) return e;
     return for_member_sets(M, B, [&](const auto& ms, int nb) {
         constexpr int CAP = std::decay_t<decltype(ms)>::cap;
-        const dim3 grid((unsigned)((g.S + 255) / 256), nb);
+        const dim3 grid((unsigned)((g.nkj * g.nkk + 255) / 256), (unsigned)g.nki, nb);
         if (g.rrot) k_rk_update<2, T, CAP><<<grid, 256, 0, st>>>(ms, stage);
         else if (g.shear) k_rk_update<1, T, CAP><<<grid, 256, 0, st>>>(ms, stage);
         else if (g.visc_if) k_rk_update<3, T, CAP><<<grid, 256, 0, st>>>(ms, stage);
