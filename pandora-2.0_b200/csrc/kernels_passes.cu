@@ -41,7 +41,7 @@ template <class T> cudaError_t configure_kernels(const Geo& g) {
 }
 
 template <class T>
-cudaError_t launch_zpass_inv(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st, const ZMaps* maps) {
+cudaError_t launch_zpass_inv(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st, const ZMaps* maps, bool pdl) {
     // DEALIASING 2/3: f_RK3PrepareRealSpace first zeroes the modes outside the cutoff
     // (src/pf_rk3.f90:269-277): k_dealias writes those zeros (it reads nothing) ahead of
     // K1, whose loads then carry no mask test
@@ -50,16 +50,16 @@ cudaError_t launch_zpass_inv(const Geo& g, const Member<T>* M, int B, int stage,
         if (e != cudaSuccess) return e;
     }
     switch (g.nz) {
-#define PD_L(N) case N: return zpass_inv_n<N, T>(g, M, B, stage, st, maps);
+#define PD_L(N) case N: return zpass_inv_n<N, T>(g, M, B, stage, st, maps, pdl);
         PD_FOR_EACH_N(PD_L)
 #undef PD_L
     default: return cudaErrorInvalidValue;
     }
 }
 
-template <class T> cudaError_t launch_ypass_inv(const Geo& g, const Member<T>* M, int B, cudaStream_t st) {
+template <class T> cudaError_t launch_ypass_inv(const Geo& g, const Member<T>* M, int B, cudaStream_t st, bool pdl) {
     switch (g.ny) {
-#define PD_L(N) case N: return ypass_inv_n<N, T>(g, M, B, st);
+#define PD_L(N) case N: return ypass_inv_n<N, T>(g, M, B, st, pdl);
         PD_FOR_EACH_N(PD_L)
 #undef PD_L
     default: return cudaErrorInvalidValue;
@@ -67,9 +67,9 @@ template <class T> cudaError_t launch_ypass_inv(const Geo& g, const Member<T>* M
 }
 
 template <class T>
-cudaError_t launch_xpass(const Geo& g, const Member<T>* M, int B, int want_phys, int want_cfl, cudaStream_t st) {
+cudaError_t launch_xpass(const Geo& g, const Member<T>* M, int B, int want_phys, int want_cfl, cudaStream_t st, bool pdl) {
     switch (g.nx) {
-#define PD_L(N) case N: return xpass_n<N, T>(g, M, B, want_phys, want_cfl, st);
+#define PD_L(N) case N: return xpass_n<N, T>(g, M, B, want_phys, want_cfl, st, pdl);
         PD_FOR_EACH_N(PD_L)
 #undef PD_L
     default: return cudaErrorInvalidValue;
@@ -86,9 +86,9 @@ cudaError_t launch_xpass_stats(const Geo& g, const Member<T>* M, double* rs, cud
     }
 }
 
-template <class T> cudaError_t launch_ypass_fwd(const Geo& g, const Member<T>* M, int B, cudaStream_t st) {
+template <class T> cudaError_t launch_ypass_fwd(const Geo& g, const Member<T>* M, int B, cudaStream_t st, bool pdl) {
     switch (g.ny) {
-#define PD_L(N) case N: return ypass_fwd_n<N, T>(g, M, B, st);
+#define PD_L(N) case N: return ypass_fwd_n<N, T>(g, M, B, st, pdl);
         PD_FOR_EACH_N(PD_L)
 #undef PD_L
     default: return cudaErrorInvalidValue;
@@ -97,12 +97,12 @@ template <class T> cudaError_t launch_ypass_fwd(const Geo& g, const Member<T>* M
 
 template <class T>
 cudaError_t launch_zpass_fwd_update(const Geo& g, const Member<T>* M, int B, int stage, int mode, cudaStream_t st,
-                                    cudaEvent_t before_update) {
+                                    cudaEvent_t before_update, bool pdl) {
     cudaError_t e = cudaErrorInvalidValue;
     switch (g.nz) {
 #define PD_L(N)                                    \
     case N:                                        \
-        e = zpass_fwd_n<N, T>(g, M, B, mode, st);  \
+        e = zpass_fwd_n<N, T>(g, M, B, mode, st, pdl);  \
         break;
         PD_FOR_EACH_N(PD_L)
 #undef PD_L
@@ -204,12 +204,12 @@ cudaError_t launch_phys_component(const float* phys, int c, double* out, long lo
 
 #define PD_INST(T)                                                                                       \
     template cudaError_t configure_kernels<T>(const Geo&);                                               \
-    template cudaError_t launch_zpass_inv<T>(const Geo&, const Member<T>*, int, int, cudaStream_t, const ZMaps*); \
-    template cudaError_t launch_ypass_inv<T>(const Geo&, const Member<T>*, int, cudaStream_t);           \
-    template cudaError_t launch_xpass<T>(const Geo&, const Member<T>*, int, int, int, cudaStream_t);     \
+    template cudaError_t launch_zpass_inv<T>(const Geo&, const Member<T>*, int, int, cudaStream_t, const ZMaps*, bool); \
+    template cudaError_t launch_ypass_inv<T>(const Geo&, const Member<T>*, int, cudaStream_t, bool);           \
+    template cudaError_t launch_xpass<T>(const Geo&, const Member<T>*, int, int, int, cudaStream_t, bool);     \
     template cudaError_t launch_xpass_stats<T>(const Geo&, const Member<T>*, double*, cudaStream_t);    \
-    template cudaError_t launch_ypass_fwd<T>(const Geo&, const Member<T>*, int, cudaStream_t);           \
-    template cudaError_t launch_zpass_fwd_update<T>(const Geo&, const Member<T>*, int, int, int, cudaStream_t, cudaEvent_t);
+    template cudaError_t launch_ypass_fwd<T>(const Geo&, const Member<T>*, int, cudaStream_t, bool);           \
+    template cudaError_t launch_zpass_fwd_update<T>(const Geo&, const Member<T>*, int, int, int, cudaStream_t, cudaEvent_t, bool);
 PD_INST(double)
 PD_INST(float)
 #undef PD_INST

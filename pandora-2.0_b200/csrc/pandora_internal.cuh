@@ -243,14 +243,16 @@ cudaError_t make_zmaps(const Geo& g, double2* const* u, ZMaps* out, bool* ok);
 // kernel that reads its inputs element-wise from global memory.
 template <class T>
 cudaError_t launch_zpass_inv(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st,
-                             const ZMaps* maps = nullptr);
-template <class T> cudaError_t launch_ypass_inv(const Geo& g, const Member<T>* M, int B, cudaStream_t st);
+                             const ZMaps* maps = nullptr, bool pdl = false);
+// pdl: the launch may overlap the end of the kernel before it in the stream (launch_after)
+template <class T> cudaError_t launch_ypass_inv(const Geo& g, const Member<T>* M, int B, cudaStream_t st, bool pdl = false);
 template <class T>
-cudaError_t launch_xpass(const Geo& g, const Member<T>* M, int B, int want_phys, int want_cfl, cudaStream_t st);
-template <class T> cudaError_t launch_ypass_fwd(const Geo& g, const Member<T>* M, int B, cudaStream_t st);
+cudaError_t launch_xpass(const Geo& g, const Member<T>* M, int B, int want_phys, int want_cfl, cudaStream_t st, bool pdl = false);
+template <class T> cudaError_t launch_ypass_fwd(const Geo& g, const Member<T>* M, int B, cudaStream_t st, bool pdl = false);
 template <class T>
 cudaError_t launch_zpass_fwd_update(const Geo& g, const Member<T>* M, int B, int stage, int mode, cudaStream_t st,
-                                    cudaEvent_t before_update = nullptr);   // an event K5b waits for, K5a not
+                                    cudaEvent_t before_update = nullptr,   // an event K5b waits for, K5a not
+                                    bool pdl = false);
 template <class T>
 cudaError_t launch_stats(const Geo& g, const Member<T>* M, int B, cudaStream_t st);
 template <class T>

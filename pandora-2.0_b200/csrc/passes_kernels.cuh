@@ -85,6 +85,15 @@ __device__ __forceinline__ void store_point(float* p, float a, float b, float c)
     *reinterpret_cast<float4*>(p) = make_float4(a, b, c, 0.0f);
 }
 
+// Start of a pass kernel: the kernel after it may be set up from now on, and this one goes on
+// once the kernel before it has ended and its writes are visible.  Every CTA comes here first, an
+// idle member's too: a kernel whose CTAs all left at once would end before the one ahead of it
+// (a chunk of idle members in a batch), and the kernel behind it would start too early.  A
+// launch without the attribute passes at once.
+__device__ __forceinline__ void grid_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <int N> constexpr int xps() {
     return (N == 16 || N == 32 || N == 48) ? 2
          : ((N == 24 || N == 64 || N == 96) ? 3 : ((N == 384 || N == 512 || N == 1024) ? 5 : 4));
@@ -200,6 +209,7 @@ __global__ void __launch_bounds__(32, RS ? XCfgStats<NX, T>::ctas() : XCfg<NX, T
     using C = typename FieldsT<T>::C;
     using XP = pdfft::FusedPlan<NX>;
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.y];
+    grid_wait();
     if (!mm.active) return;
     if constexpr (CAP > 1) {   // a batch slot between members
         if (mm.F.clock->status & PD_ST_IDLE) return;
@@ -447,6 +457,7 @@ __global__ void __launch_bounds__(32 * ConvCfg<NX, T>::NW, 1) k_xpass_conv(const
     using C = typename FieldsT<T>::C;
     using XP = pdfft::FusedPlan<NX>;   // the backward plan r0, r1, r2 (run unfused here)
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.y];
+    grid_wait();
     if (!mm.active) return;
     if constexpr (CAP > 1) {   // a batch slot between members
         if (mm.F.clock->status & PD_ST_IDLE) return;
@@ -699,6 +710,7 @@ template <int FORM, class T, int CAP>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_rk_update(const __grid_constant__ MemberSet<T, CAP> ms, int stage) {
     using C = typename FieldsT<T>::C;
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.z];
+    grid_wait();
     if (!mm.active) return;
     if constexpr (CAP > 1) {   // a batch slot between members
         if (mm.F.clock->status & PD_ST_IDLE) return;
@@ -728,17 +740,20 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_rk_update(const
 // inputs straight from HBM and the last pass writing its outputs straight to
 // HBM, so a 256-point line crosses shared memory once (one block barrier).
 // ---------------------------------------------------------------------------
-template <int N, bool TWO = false> struct TCfg {
-    // Radix plan: Plan<N>, or with TWO (the y passes and K5a) for FP32 512-point
+// KIND: 0 K1, 1 the y passes, 2 K5a.
+template <int N, int KIND = 0> struct TCfg {
+    // Radix plan: Plan<N>, or in the y passes and K5a for FP32 512-point
     // lines the two-pass (32, 16): one shared-memory round trip instead of two.  An
     // FP64 item of radix 32 does not fit the registers of two CTAs per SM, and K1
     // (vorticity loads in its first pass) measured slower with it.
-    template <class T> static constexpr bool two() { return TWO && sizeof(T) == 4 && N == 512; }
+    template <class T> static constexpr bool two() { return KIND > 0 && sizeof(T) == 4 && N == 512; }
     template <class T> static constexpr int r0() { return two<T>() ? 32 : pdfft::Plan<N>::r0; }
     template <class T> static constexpr int r1() { return two<T>() ? 16 : pdfft::Plan<N>::r1; }
     template <class T> static constexpr int r2() { return two<T>() ? 0 : pdfft::Plan<N>::r2; }
-    // threads per CTA: one butterfly per thread in the widest pass of a tile of 8 lines
-    template <class T> static constexpr int nt() { return pdfft::tile_threads_for<N, r0<T>(), r1<T>(), r2<T>()>(); }
+    // threads per CTA: one butterfly per thread in the widest pass of a tile (of 8 lines' worth)
+    template <class T> static constexpr int nt() {
+        return pdfft::tile_threads_for<N, r0<T>(), r1<T>(), r2<T>(), (lines<T>() == 4 ? 4 : 8)>();
+    }
     // Lines per tile: 8 (FP64: one 128-byte row of complex values, so the quarter
     // warp of a shared-memory wavefront owns the lines of one butterfly and every
     // access of a pass is whole rows).  FP32 tiles of 512-point lines take 16 lines,
@@ -746,12 +761,24 @@ template <int N, bool TWO = false> struct TCfg {
     // two-way bank conflicts and global rows are 64 bytes); elsewhere the doubled
     // tile costs occupancy (1024) or a half-empty last tile (nkip = 88 at 256) and
     // measured slower.
-    template <class T> static constexpr int lines() { return (sizeof(T) == 4 && N == 512) ? 16 : 8; }
+    // The FP64 y passes of 640 and 896 points take 4 lines, two or four CTAs per SM instead of one
+    // whose 512 threads wait at its barriers (640^3: K2 4.69 -> 4.08 ms, K4 2.22 -> 1.84; 896^3 12.2
+    // -> 10.5, 5.79 -> 4.89; slower at 768, 8.0 -> 8.5, and 1024, 13.3 -> 13.9).
+    template <class T> static constexpr int lines() {
+        return (sizeof(T) == 4 && N == 512) ? 16 : (KIND == 1 && sizeof(T) == 8 && (N == 640 || N == 896) ? 4 : 8);
+    }
     // resident CTAs per SM asked of the register allocator: an FP32 tile of 16 lines
-    // holds the registers and shared memory of an FP64 one, of 8 lines half of them
+    // holds the registers and shared memory of an FP64 one, of 8 lines half of them.  FP64 tiles of
+    // 512 threads: two (64 registers) where they fit, against one of 128 registers (384^3: K2
+    // 1.18 -> 0.92 ms, K4 0.57 -> 0.43, K5 0.71 -> 0.59; 320^3 K4 0.30 -> 0.18; 448^3 K4 0.70 -> 0.43; 640^3
+    // K1 3.30 -> 3.07, K5 2.97 -> 2.64), but one for K5a at 320 and 448 points (0.31 against 0.35
+    // ms, 0.79 against 0.84).
     template <class T> static constexpr int minb() {
         constexpr int NT = nt<T>();
-        return (sizeof(T) == 8 || lines<T>() == 16) ? (NT <= 128 ? (N == 192 ? 4 : 5) : (NT <= 256 ? 2 : (N == 512 ? 2 : 1)))
+        if (lines<T>() == 4) return NT <= 256 ? 4 : 2;
+        if (sizeof(T) == 8 && NT > 256)
+            return (KIND == 2 && (N == 320 || N == 448)) || (KIND == 1 && N == 768) || N > 768 ? 1 : 2;
+        return (sizeof(T) == 8 || lines<T>() == 16) ? (NT <= 128 ? (N == 192 ? 4 : 5) : 2)
                                                     : (NT <= 128 ? (N == 192 ? 6 : 8) : (NT <= 256 ? 4 : 2));
     }
     // pad rows of the FP32 tiles of 8 lines (64-byte rows); at 1024 points, two butterflies per
@@ -794,6 +821,7 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<T>(),
     using C = typename FieldsT<T>::C;
     constexpr int nf = FORM == 3 ? 9 : 6;
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.x / nf];
+    grid_wait();
     if (!mm.active) return;
     if constexpr (CAP > 1) {   // a batch slot between members
         if (mm.F.clock->status & PD_ST_IDLE) return;
@@ -945,6 +973,7 @@ __global__ void __launch_bounds__(ZStage<NZ>::nt, 2) k_zpass_inv_tma(const __gri
     constexpr int LT = ZS::lines, BK = ZS::BK, NB = ZS::NB;
     constexpr int nf = FORM == 3 ? 9 : 6;
     const Member<double>& mm = ms.m[0];
+    grid_wait();
     if (!mm.active) return;
     const Fields F = mm.F;
     const Geo g = mm.g;
@@ -1041,14 +1070,134 @@ __global__ void __launch_bounds__(ZStage<NZ>::nt, 2) k_zpass_inv_tma(const __gri
     }
 }
 
+// ---------------------------------------------------------------------------
+// K1 with the velocity rows staged by asynchronous element copies (cp.async; any length, batches,
+// FP32 rows, which a tensor map cannot describe: NKK is odd, so they start at 8-byte
+// boundaries).  As k_zpass_inv_tma: one CTA forms every field of its tile from rows that arrive
+// once, whole and coalesced.  (The element-wise K1 reads u across lines, 16 or 32 bytes of each
+// row per warp load, once per field that needs it.)
+// ---------------------------------------------------------------------------
+template <int N, class T> struct SCfg {
+    using C = typename Cplx<T>::type;
+    static constexpr int ce = (int)sizeof(C);
+    static constexpr int r0 = pdfft::Plan<N>::r0, r1 = pdfft::Plan<N>::r1, r2 = pdfft::Plan<N>::r2;
+    static constexpr int lines = (N > 512 || (sizeof(T) == 8 && N > 256)) ? 4 : 8;
+    static constexpr int ps = pdfft::tile_pad<ce * lines, r0>();
+    // row pitch: the lanes of a wavefront (M values of 128 bytes) read q consecutive k of each line
+    static constexpr int NKK = 2 * (N / 3) + 1, M = 128 / ce, q = M / lines;
+    static constexpr int P = NKK + ((q - NKK % M) % M + M) % M;
+    static constexpr int nt = pdfft::tile_threads_for<N, r0, r1, r2, lines>();
+    static constexpr size_t smem = (size_t)ce * (3 * lines * P + tile_rows<N, ps>() * lines + N);
+    static constexpr int fit = (int)(232448 / (smem + 1024));
+    static constexpr int regs = sizeof(T) == 4 && nt >= 512 ? 64 : 128;
+    static constexpr int byreg = 65536 / (nt * regs);
+    static constexpr int minb = fit < 1 ? 1 : (fit < byreg ? fit : (byreg < 1 ? 1 : byreg));
+    static_assert(nt % lines == 0, "a thread owns one line of the tile");
+};
+__device__ __forceinline__ void copy_async(float2* dst, const float2* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async(double2* dst, const double2* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+template <int NZ, int FORM, class T, int CAP>
+__global__ void __launch_bounds__(SCfg<NZ, T>::nt, SCfg<NZ, T>::minb) k_zpass_inv_staged(const __grid_constant__ MemberSet<T, CAP> ms,
+                                                                                         int stage, long long pf_ctas) {
+    using C = typename FieldsT<T>::C;
+    using S = SCfg<NZ, T>;
+    constexpr int nf = FORM == 3 ? 9 : 6, LT = S::lines, P = S::P, NKK = S::NKK, KK = NZ / 3;
+    const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.z];
+    grid_wait();
+    if (!mm.active) return;
+    if constexpr (CAP > 1) {   // a batch slot between members
+        if (mm.F.clock->status & PD_ST_IDLE) return;
+    }
+    const FieldsT<T>& F = mm.F;
+    const Geo& g = mm.g;
+    C* const stg = smem_as<C>();                     // [3][LT][P]
+    C* const s = stg + 3 * LT * P;
+    C* const tw = s + tile_rows<NZ, S::ps>() * LT;   // the twiddle table
+    const int i0 = blockIdx.x * LT, j = blockIdx.y, tid = threadIdx.x;
+    const int nkj = g.nkj, nki = g.nki;
+    if (stage == 1 && blockIdx.x == 0 && j == 0 && tid == 0) F.clock->ucfl_bits = 0ull;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const C* const uc = F.u[c] + ((long long)i0 * nkj + j) * NKK;
+        for (int x = tid; x < LT * NKK; x += S::nt) {
+            const int l = x / NKK, k = x - l * NKK;
+            C* const d = stg + (c * LT + l) * P + k;
+            if (i0 + l < nki) copy_async(d, uc + (long long)l * nkj * NKK + k);
+            else *d = mk(T(0), T(0));
+        }
+    }
+    for (int e = tid; e < NZ; e += S::nt) copy_async(tw + e, F.tw_z + e);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // the rows of the CTA one wave of resident CTAs later, into L2 while this one transforms
+    if (pf_ctas > 0 && tid < 3 * LT) {
+        const long long nxt = blockIdx.x + (long long)gridDim.x * blockIdx.y + pf_ctas;
+        if (nxt < (long long)gridDim.x * gridDim.y) {
+            const int i = (int)(nxt % gridDim.x) * LT + tid % LT, j2 = (int)(nxt / gridDim.x), c = tid / LT;
+            const C* const uc = c == 0 ? F.u[0] : (c == 1 ? F.u[1] : F.u[2]);
+            if (i < nki) prefetch_l2(uc + ((long long)i * nkj + j2) * NKK, NKK * sizeof(C));
+        }
+    }
+    const T k2 = (T)wvn(j, g.kj);
+    const long long zs = (long long)nkj * g.nkip;
+#pragma unroll 1
+    for (int f = 0; f < nf; f++) {
+        // vorticity: the components and coefficients of the thread's line (tid % LT)
+        const int ca = FORM == 3 || f < 3 ? f % 3 : (f == 3 ? 1 : 0), cb = f == 5 ? 1 : 2;
+        const bool three = FORM == 1 && f == 5;
+        VortLine<T> vl;
+        if constexpr (FORM == 1 || FORM == 2) {
+            if (f >= 3) vl = vort_line<FORM, T>(bf_as<T>(make_bf(g, F.clock)), f - 3, (T)(i0 + tid % LT), k2);
+        }
+        const C* const ra = stg + ca * LT * P;
+        const C* const rb = stg + cb * LT * P;
+        const C* const rc = stg + 2 * LT * P;
+        auto ld = [&](int z, int l, auto band) -> C {
+            constexpr int B = decltype(band)::value;
+            int k;
+            if (B == 1 || (B == 3 && z <= KK)) k = z;
+            else if (B == 2 || z >= NZ - KK) k = z - NZ + NKK;
+            else return mk(T(0), T(0));
+            const C a = ra[l * P + k];
+            if (f < 3) return a;
+            const T k3 = B == 1 ? (T)z : (B == 2 ? (T)(z - NZ) : (T)wvn(k, KK));
+            if constexpr (FORM == 3) {   // i k2 u_c or i k3 u_c (f_RK3Derivative, src/pf_rk3.f90:3735-3743)
+                const T kd = f < 6 ? k2 : k3;
+                return mk(-kd * a.y, kd * a.x);
+            } else {
+                const C b = rb[l * P + k];
+                if constexpr (FORM == 0) {   // omega = i k x u (src/pf_rk3.f90:402-407,520-525,630-634)
+                    const T k1 = (T)(i0 + l);
+                    const T ka = f == 3 ? -k3 : (f == 4 ? k3 : -k2), kb = f == 3 ? -k2 : (f == 4 ? k1 : -k1);
+                    return mk(-ka * a.y - -kb * b.y, ka * a.x - kb * b.x);
+                } else {
+                    C c3;
+                    if (three) c3 = rc[l * P + k];
+                    return vort_mode<T, C>(vl, k3, a, b, three ? &c3 : nullptr);
+                }
+            }
+        };
+        C* dst = F.zb + (((long long)f * NZ) * nkj + j) * g.nkip + i0;
+        auto st = [&](int z, int l, C v) { dst[z * zs + l] = v; };
+        pdfft::fft_tile_io<NZ, +1, LT, S::nt, S::r0, S::r1, S::r2, KK, 0, S::ps>(s, tw, tid, ld, st);
+        __syncthreads();   // the tile buffer is read by the last pass before the next field's first pass
+    }
+}
+
 // K2: backward y transforms of field f = blockIdx.z, j zero-padded into
 // [KJ+1, NY-KJ-1] (f_RK3TransformjiFs2Rs, src/pf_rk3.f90:1458-1473).  nf = six fields, or
 // nine in the R-conv form, per member.
 template <int NY, class T, int CAP, int CN = 0>
-__global__ void __launch_bounds__(TCfg<NY, true>::template nt<T>(), TCfg<NY, true>::template minb<T>()) k_ypass_inv(const __grid_constant__ MemberSet<T, CAP> ms,
+__global__ void __launch_bounds__(TCfg<NY, 1>::template nt<T>(), TCfg<NY, 1>::template minb<T>()) k_ypass_inv(const __grid_constant__ MemberSet<T, CAP> ms,
                                                                                                           int nf) {
     using C = typename FieldsT<T>::C;
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.z / nf];
+    grid_wait();
     if (!mm.active) return;
     if constexpr (CAP > 1) {   // a batch slot between members
         if (mm.F.clock->status & PD_ST_IDLE) return;
@@ -1058,7 +1207,7 @@ __global__ void __launch_bounds__(TCfg<NY, true>::template nt<T>(), TCfg<NY, tru
     // CN > 0: a cubic grid of CN points a side, every size a compile-time constant
     const int nz_ = CN ? CN : g.nz, nkip_ = CN ? (CN / 3 + 1 + 7) / 8 * 8 : g.nkip;
     C* s = smem_as<C>();
-    constexpr int LT = TCfg<NY>::template lines<T>();
+    constexpr int LT = TCfg<NY, 1>::template lines<T>();
     const int i0 = blockIdx.x * LT, z = blockIdx.y, f = blockIdx.z % nf;
     const int lmax = nkip_ - i0;
     constexpr int KJ = NY / 3, NKJ = 2 * KJ + 1;   // g.kj, g.nkj (the 2/3 rule)
@@ -1076,15 +1225,16 @@ __global__ void __launch_bounds__(TCfg<NY, true>::template nt<T>(), TCfg<NY, tru
         if (LT > 8 && l >= lmax) return;
         dst[y * rs + l] = v;
     };
-    TCfg<NY, true>::template transform<+1, LT, KJ, 0>(s, F.tw_y, ld, st);
+    TCfg<NY, 1>::template transform<+1, LT, KJ, 0>(s, F.tw_y, ld, st);
 }
 
 // K4: forward y transforms of NL field f = blockIdx.z, truncated to j
 // (f_RK3TransformjiRs2Fs, src/pf_rk3.f90:1902-1938).
 template <int NY, class T, int CAP, int CN = 0>
-__global__ void __launch_bounds__(TCfg<NY, true>::template nt<T>(), TCfg<NY, true>::template minb<T>()) k_ypass_fwd(const __grid_constant__ MemberSet<T, CAP> ms) {
+__global__ void __launch_bounds__(TCfg<NY, 1>::template nt<T>(), TCfg<NY, 1>::template minb<T>()) k_ypass_fwd(const __grid_constant__ MemberSet<T, CAP> ms) {
     using C = typename FieldsT<T>::C;
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.z / 3];
+    grid_wait();
     if (!mm.active) return;
     if constexpr (CAP > 1) {   // a batch slot between members
         if (mm.F.clock->status & PD_ST_IDLE) return;
@@ -1094,7 +1244,7 @@ __global__ void __launch_bounds__(TCfg<NY, true>::template nt<T>(), TCfg<NY, tru
     // CN > 0: a cubic grid of CN points a side, every size a compile-time constant
     const int nz_ = CN ? CN : g.nz, nkip_ = CN ? (CN / 3 + 1 + 7) / 8 * 8 : g.nkip;
     C* s = smem_as<C>();
-    constexpr int LT = TCfg<NY>::template lines<T>();
+    constexpr int LT = TCfg<NY, 1>::template lines<T>();
     const int i0 = blockIdx.x * LT, z = blockIdx.y, f = blockIdx.z % 3;
     const int lmax = nkip_ - i0;
     constexpr int KJ = NY / 3, NKJ = 2 * KJ + 1;   // g.kj, g.nkj (the 2/3 rule)
@@ -1111,15 +1261,16 @@ __global__ void __launch_bounds__(TCfg<NY, true>::template nt<T>(), TCfg<NY, tru
         if (B == 1 || (B == 3 && y <= KJ)) dst[y * rs + l] = v;
         else if (B == 2 || y >= NY - KJ) dst[(y - NY + NKJ) * rs + l] = v;
     };
-    TCfg<NY, true>::template transform<-1, LT, 0, KJ>(s, F.tw_y, ld, st);
+    TCfg<NY, 1>::template transform<-1, LT, 0, KJ>(s, F.tw_y, ld, st);
 }
 
 // K5a: forward z transforms of NL field f = blockIdx.z, x 1/(NX NY NZ), truncated
 // to k, stored as rows of NL-hat [c][i][j][k].
 template <int NZ, class T, int CAP>
-__global__ void __launch_bounds__(TCfg<NZ, true>::template nt<T>(), TCfg<NZ, true>::template minb<T>()) k_zpass_fwd(const __grid_constant__ MemberSet<T, CAP> ms, int mode) {
+__global__ void __launch_bounds__(TCfg<NZ, 2>::template nt<T>(), TCfg<NZ, 2>::template minb<T>()) k_zpass_fwd(const __grid_constant__ MemberSet<T, CAP> ms, int mode) {
     using C = typename FieldsT<T>::C;
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.z / 3];
+    grid_wait();
     if (!mm.active) return;
     if constexpr (CAP > 1) {   // a batch slot between members
         if (mm.F.clock->status & PD_ST_IDLE) return;
@@ -1127,7 +1278,7 @@ __global__ void __launch_bounds__(TCfg<NZ, true>::template nt<T>(), TCfg<NZ, tru
     const FieldsT<T> F = mm.F;
     const Geo g = mm.g;
     C* s = smem_as<C>();
-    constexpr int LT = TCfg<NZ>::template lines<T>();
+    constexpr int LT = TCfg<NZ, 2>::template lines<T>();
     const int i0 = blockIdx.x * LT, j = blockIdx.y, f = blockIdx.z % 3;
     const int lmax = g.nkip - i0;
     // NL-hat into the y-pencil buffer, or (mode 1) into rk
@@ -1153,7 +1304,7 @@ __global__ void __launch_bounds__(TCfg<NZ, true>::template nt<T>(), TCfg<NZ, tru
         else return;
         dst[l * istride + k] = mk(v.x * norm, v.y * norm);
     };
-    TCfg<NZ, true>::template transform<-1, LT, 0, KK>(s, F.tw_z, ld, st);
+    TCfg<NZ, 2>::template transform<-1, LT, 0, KK>(s, F.tw_z, ld, st);
 }
 
 
@@ -1174,17 +1325,29 @@ template <int N> constexpr bool batch_len() {
     return N == 32 || N == 48 || N == 64 || N == 96 || N == 128 || N == 192 || N == 256;
 }
 
+// Lengths and forms whose K1 stages its rows with asynchronous copies.  Step, element-wise ->
+// staged: 128^3 FP64 0.317 -> 0.305 ms, 192^3 R-conv 1.85 -> 1.77 (FP32-mixed 1.13 -> 1.07), 256^3
+// R-conv 4.36 -> 4.28 (2.21 -> 2.16), 224^3 2.32 -> 2.27 (1.53 -> 1.46), 320^3 7.65 -> 6.95 (4.50 ->
+// 4.26), 448^3 19.6 -> 18.1 (11.8 -> 11.4), 384^3 FP32-mixed 6.56 -> 6.22, 512^3 10.46 -> 10.41 (FP64
+// there: k_zpass_inv_tma).  Level at 112 and 160; slower at 64 (0.072 -> 0.076) and 96, whose few
+// threads per CTA leave the copies exposed, at 256 without the nine fields of R-conv to share
+// them, and at 1024 (5.4 -> 7.0 ms per stage), one CTA of whose tiles fits an SM.
+template <int N, class T, int FORM> constexpr bool staged_len() {
+    return N == 128 || N == 192 || N == 224 || N == 320 || N == 384 || N == 448 || (N == 256 && FORM == 3) ||
+           (N == 512 && sizeof(T) == 4);
+}
+
 // Per-length launchers (passes_n.cuh).  Every launcher takes the batch's geometry g
 // (grid sizes and flow type, common to all members), the host array M of its B member
 // descriptors and the stream; the members go to the kernels by value, kBatchChunk per launch.
 template <int N, class T> cudaError_t configure_n(const Geo& g);
 template <int N, class T>
-cudaError_t zpass_inv_n(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st, const ZMaps* maps);
-template <int N, class T> cudaError_t ypass_inv_n(const Geo& g, const Member<T>* M, int B, cudaStream_t st);
+cudaError_t zpass_inv_n(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st, const ZMaps* maps, bool pdl);
+template <int N, class T> cudaError_t ypass_inv_n(const Geo& g, const Member<T>* M, int B, cudaStream_t st, bool pdl);
 template <int N, class T>
-cudaError_t xpass_n(const Geo& g, const Member<T>* M, int B, int want_phys, int want_cfl, cudaStream_t st);
+cudaError_t xpass_n(const Geo& g, const Member<T>* M, int B, int want_phys, int want_cfl, cudaStream_t st, bool pdl);
 template <int N, class T> cudaError_t xpass_stats_n(const Geo& g, const Member<T>* M, double* rs, cudaStream_t st);
-template <int N, class T> cudaError_t ypass_fwd_n(const Geo& g, const Member<T>* M, int B, cudaStream_t st);
-template <int N, class T> cudaError_t zpass_fwd_n(const Geo& g, const Member<T>* M, int B, int mode, cudaStream_t st);
+template <int N, class T> cudaError_t ypass_fwd_n(const Geo& g, const Member<T>* M, int B, cudaStream_t st, bool pdl);
+template <int N, class T> cudaError_t zpass_fwd_n(const Geo& g, const Member<T>* M, int B, int mode, cudaStream_t st, bool pdl);
 
 }  // namespace pd

@@ -25,6 +25,23 @@ template <typename K> static cudaError_t set_smem(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Launches `kernel`, with `pdl` as a programmatic dependent of the kernel before it in the
+// stream: its CTAs may be set up while that kernel drains, and wait at grid_wait() for its end.
+template <class... KA, class... A>
+static void launch_after(bool pdl, void (*kernel)(KA...), dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, args...);   // the callers read cudaGetLastError
+}
+
 #define PD_CAP(S) std::decay_t<decltype(S)>::cap
 
 // Dynamic shared memory limits of the kernels of length N that the geometry uses, for
@@ -37,20 +54,33 @@ template <int N, class T, int CAP> static cudaError_t configure_cap(const Geo& g
             if ((e = set_smem(k_zpass_inv<N, 1, T, CAP, N>, TCfg<N>::template smem<T>()))) return e;
             if ((e = set_smem(k_zpass_inv<N, 2, T, CAP, N>, TCfg<N>::template smem<T>()))) return e;
             if ((e = set_smem(k_zpass_inv<N, 3, T, CAP, N>, TCfg<N>::template smem<T>()))) return e;
-            if ((e = set_smem(k_ypass_inv<N, T, CAP, N>, TCfg<N, true>::template smem<T>()))) return e;
-            if ((e = set_smem(k_ypass_fwd<N, T, CAP, N>, TCfg<N, true>::template smem<T>()))) return e;
+            if ((e = set_smem(k_ypass_inv<N, T, CAP, N>, TCfg<N, 1>::template smem<T>()))) return e;
+            if ((e = set_smem(k_ypass_fwd<N, T, CAP, N>, TCfg<N, 1>::template smem<T>()))) return e;
         }
+    }
+    if (g.nz == N) {
+        cudaError_t es = cudaSuccess;
+        auto staged = [&](auto form) {
+            constexpr int FORM = decltype(form)::value;
+            if constexpr (staged_len<N, T, FORM>())
+                if (!es) es = set_smem(k_zpass_inv_staged<N, FORM, T, CAP>, SCfg<N, T>::smem);
+        };
+        staged(std::integral_constant<int, 0>{});
+        staged(std::integral_constant<int, 1>{});
+        staged(std::integral_constant<int, 2>{});
+        staged(std::integral_constant<int, 3>{});
+        if (es) return es;
     }
     if (g.nz == N) {
         if ((e = set_smem(k_zpass_inv<N, 0, T, CAP>, TCfg<N>::template smem<T>()))) return e;
         if ((e = set_smem(k_zpass_inv<N, 1, T, CAP>, TCfg<N>::template smem<T>()))) return e;
         if ((e = set_smem(k_zpass_inv<N, 2, T, CAP>, TCfg<N>::template smem<T>()))) return e;
         if ((e = set_smem(k_zpass_inv<N, 3, T, CAP>, TCfg<N>::template smem<T>()))) return e;
-        if ((e = set_smem(k_zpass_fwd<N, T, CAP>, TCfg<N, true>::template smem<T>()))) return e;
+        if ((e = set_smem(k_zpass_fwd<N, T, CAP>, TCfg<N, 2>::template smem<T>()))) return e;
     }
     if (g.ny == N) {
-        if ((e = set_smem(k_ypass_inv<N, T, CAP>, TCfg<N, true>::template smem<T>()))) return e;
-        if ((e = set_smem(k_ypass_fwd<N, T, CAP>, TCfg<N, true>::template smem<T>()))) return e;
+        if ((e = set_smem(k_ypass_inv<N, T, CAP>, TCfg<N, 1>::template smem<T>()))) return e;
+        if ((e = set_smem(k_ypass_fwd<N, T, CAP>, TCfg<N, 1>::template smem<T>()))) return e;
     }
     if (g.nx == N) {
         if constexpr (xlpw_len<N>()) {   // at most 20 KB per warp: no opt-in needed beyond this
@@ -86,7 +116,7 @@ template <int N, class T> cudaError_t configure_n(const Geo& g) {
 // K1 (z length N): the staged kernel for a single FP64 simulation with tensor maps, else
 // the element-wise kernel of the flow's form.
 template <int N, class T>
-cudaError_t zpass_inv_n(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st, const ZMaps* maps) {
+cudaError_t zpass_inv_n(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st, const ZMaps* maps, bool pdl) {
     if constexpr (std::is_same<T, double>::value && ZStage<N>::enabled) {
         if (maps && B == 1) {
             MemberSet<double, 1> one;
@@ -94,10 +124,10 @@ cudaError_t zpass_inv_n(const Geo& g, const Member<T>* M, int B, int stage, cuda
             const dim3 grid((unsigned)(g.nkip / ZStage<N>::lines), g.nkj);
             constexpr int NT = ZStage<N>::nt;
             constexpr size_t sm = ZStage<N>::smem;
-            if (!g.shear) k_zpass_inv_tma<N, 0><<<grid, NT, sm, st>>>(one, *maps, stage);
-            else if (!g.rrot) k_zpass_inv_tma<N, 1><<<grid, NT, sm, st>>>(one, *maps, stage);
-            else if (!g.rconv) k_zpass_inv_tma<N, 2><<<grid, NT, sm, st>>>(one, *maps, stage);
-            else k_zpass_inv_tma<N, 3><<<grid, NT, sm, st>>>(one, *maps, stage);
+            if (!g.shear) launch_after(pdl, k_zpass_inv_tma<N, 0>, grid, NT, sm, st, one, *maps, stage);
+            else if (!g.rrot) launch_after(pdl, k_zpass_inv_tma<N, 1>, grid, NT, sm, st, one, *maps, stage);
+            else if (!g.rconv) launch_after(pdl, k_zpass_inv_tma<N, 2>, grid, NT, sm, st, one, *maps, stage);
+            else launch_after(pdl, k_zpass_inv_tma<N, 3>, grid, NT, sm, st, one, *maps, stage);
             return cudaGetLastError();
         }
     }
@@ -107,16 +137,24 @@ cudaError_t zpass_inv_n(const Geo& g, const Member<T>* M, int B, int stage, cuda
             const dim3 grid(pass_fields(g) * nb, TCfg<N>::template tiles<T>(g), g.nkj);
             constexpr int NT = TCfg<N>::template nt<T>();
             const size_t sm = TCfg<N>::template smem<T>();
-            auto go = [&](auto kern) {
-                const long long pf = CAP == 1 ? resident_ctas(kern, NT, sm) : 0;
-                kern<<<grid, NT, sm, st>>>(ms, stage, pf);
+            auto go = [&](auto form, auto cn) {
+                constexpr int FORM = decltype(form)::value, CN = decltype(cn)::value;
+                if constexpr (staged_len<N, T, FORM>()) {
+                    using S = SCfg<N, T>;
+                    auto kern = k_zpass_inv_staged<N, FORM, T, CAP>;
+                    const long long pf = CAP == 1 ? resident_ctas(kern, S::nt, S::smem) : 0;
+                    launch_after(pdl, kern, dim3((unsigned)(g.nkip / S::lines), g.nkj, nb), S::nt, S::smem, st, ms, stage, pf);
+                } else {
+                    auto kern = k_zpass_inv<N, FORM, T, CAP, CN>;
+                    const long long pf = CAP == 1 ? resident_ctas(kern, NT, sm) : 0;
+                    launch_after(pdl, kern, grid, NT, sm, st, ms, stage, pf);
+                }
             };
             auto form = [&](auto cn) {
-                constexpr int CN = decltype(cn)::value;
-                if (!g.shear) go(k_zpass_inv<N, 0, T, CAP, CN>);
-                else if (!g.rrot) go(k_zpass_inv<N, 1, T, CAP, CN>);
-                else if (!g.rconv) go(k_zpass_inv<N, 2, T, CAP, CN>);
-                else go(k_zpass_inv<N, 3, T, CAP, CN>);
+                if (!g.shear) go(std::integral_constant<int, 0>{}, cn);
+                else if (!g.rrot) go(std::integral_constant<int, 1>{}, cn);
+                else if (!g.rconv) go(std::integral_constant<int, 2>{}, cn);
+                else go(std::integral_constant<int, 3>{}, cn);
             };
             if constexpr (cube_len<N, T>()) {
                 if (is_cube(g, N)) { form(std::integral_constant<int, N>{}); return; }
@@ -126,23 +164,23 @@ cudaError_t zpass_inv_n(const Geo& g, const Member<T>* M, int B, int stage, cuda
     });
 }
 
-template <int N, class T> cudaError_t ypass_inv_n(const Geo& g, const Member<T>* M, int B, cudaStream_t st) {
+template <int N, class T> cudaError_t ypass_inv_n(const Geo& g, const Member<T>* M, int B, cudaStream_t st, bool pdl) {
     return for_member_sets(M, B, [&](const auto& ms, int nb) {
         constexpr int CAP = PD_CAP(ms);
         if constexpr (CAP == 1 || batch_len<N>()) {
-            const dim3 grid(TCfg<N, true>::template tiles<T>(g), g.nz, pass_fields(g) * nb);
-            constexpr int NT = TCfg<N, true>::template nt<T>();
-            constexpr size_t sm = TCfg<N, true>::template smem<T>();
+            const dim3 grid(TCfg<N, 1>::template tiles<T>(g), g.nz, pass_fields(g) * nb);
+            constexpr int NT = TCfg<N, 1>::template nt<T>();
+            constexpr size_t sm = TCfg<N, 1>::template smem<T>();
             if constexpr (cube_len<N, T>()) {
-                if (is_cube(g, N)) { k_ypass_inv<N, T, CAP, N><<<grid, NT, sm, st>>>(ms, pass_fields(g)); return; }
+                if (is_cube(g, N)) { launch_after(pdl, k_ypass_inv<N, T, CAP, N>, grid, NT, sm, st, ms, pass_fields(g)); return; }
             }
-            k_ypass_inv<N, T, CAP><<<grid, NT, sm, st>>>(ms, pass_fields(g));
+            launch_after(pdl, k_ypass_inv<N, T, CAP>, grid, NT, sm, st, ms, pass_fields(g));
         }
     });
 }
 
 template <int N, class T>
-cudaError_t xpass_n(const Geo& g, const Member<T>* M, int B, int want_phys, int want_cfl, cudaStream_t st) {
+cudaError_t xpass_n(const Geo& g, const Member<T>* M, int B, int want_phys, int want_cfl, cudaStream_t st, bool pdl) {
     const long long lines = (long long)g.ny * g.nz;
     return for_member_sets(M, B, [&](const auto& ms, int nb) {
         constexpr int CAP = PD_CAP(ms);
@@ -151,8 +189,8 @@ cudaError_t xpass_n(const Geo& g, const Member<T>* M, int B, int want_phys, int 
                 constexpr int NW = ConvCfg<N, T>::NW;
                 const long long nl = (lines + NW - 1) / NW;
                 const long long pf = CAP == 1 ? NW * resident_ctas(k_xpass_conv<N, T, CAP>, 32 * NW, ConvCfg<N, T>::smem) : 0;
-                k_xpass_conv<N, T, CAP><<<dim3((unsigned)nl, nb), 32 * NW, ConvCfg<N, T>::smem, st>>>(ms, want_phys,
-                                                                                                  want_cfl, pf);
+                launch_after(pdl, k_xpass_conv<N, T, CAP>, dim3((unsigned)nl, nb), 32 * NW, ConvCfg<N, T>::smem, st, ms,
+                             want_phys, want_cfl, pf);
                 return;
             }
             auto go = [&](auto lpwc) {
@@ -160,8 +198,8 @@ cudaError_t xpass_n(const Geo& g, const Member<T>* M, int B, int want_phys, int 
                 const long long nl = (lines + LPW - 1) / LPW;
                 // L2 prefetch distance: one wave of resident CTAs (single simulations)
                 const long long pf = CAP == 1 ? LPW * resident_ctas(k_xpass<N, T, CAP, false, LPW>, 32, smem_kx<N, T, LPW>()) : 0;
-                k_xpass<N, T, CAP, false, LPW><<<dim3((unsigned)nl, nb), 32, smem_kx<N, T, LPW>(), st>>>(ms, want_phys,
-                                                                                                       want_cfl, pf, nullptr);
+                launch_after(pdl, k_xpass<N, T, CAP, false, LPW>, dim3((unsigned)nl, nb), 32, smem_kx<N, T, LPW>(), st, ms,
+                             want_phys, want_cfl, pf, (double*)nullptr);
             };
             if constexpr (xlpw_len<N>()) {
                 const int lpw = g.xlpw > 0 ? g.xlpw : XCfg<N, T>::lpw;
@@ -188,41 +226,41 @@ template <int N, class T> cudaError_t xpass_stats_n(const Geo& g, const Member<T
     return cudaGetLastError();
 }
 
-template <int N, class T> cudaError_t ypass_fwd_n(const Geo& g, const Member<T>* M, int B, cudaStream_t st) {
+template <int N, class T> cudaError_t ypass_fwd_n(const Geo& g, const Member<T>* M, int B, cudaStream_t st, bool pdl) {
     return for_member_sets(M, B, [&](const auto& ms, int nb) {
         constexpr int CAP = PD_CAP(ms);
         if constexpr (CAP == 1 || batch_len<N>()) {
-            const dim3 grid(TCfg<N, true>::template tiles<T>(g), g.nz, 3 * nb);
-            constexpr int NT = TCfg<N, true>::template nt<T>();
-            constexpr size_t sm = TCfg<N, true>::template smem<T>();
+            const dim3 grid(TCfg<N, 1>::template tiles<T>(g), g.nz, 3 * nb);
+            constexpr int NT = TCfg<N, 1>::template nt<T>();
+            constexpr size_t sm = TCfg<N, 1>::template smem<T>();
             if constexpr (cube_len<N, T>()) {
-                if (is_cube(g, N)) { k_ypass_fwd<N, T, CAP, N><<<grid, NT, sm, st>>>(ms); return; }
+                if (is_cube(g, N)) { launch_after(pdl, k_ypass_fwd<N, T, CAP, N>, grid, NT, sm, st, ms); return; }
             }
-            k_ypass_fwd<N, T, CAP><<<grid, NT, sm, st>>>(ms);
+            launch_after(pdl, k_ypass_fwd<N, T, CAP>, grid, NT, sm, st, ms);
         }
     });
 }
 
 // K5a: forward z transforms (mode 1: NL-hat into rk, the transform test hook).
 template <int N, class T>
-cudaError_t zpass_fwd_n(const Geo& g, const Member<T>* M, int B, int mode, cudaStream_t st) {
+cudaError_t zpass_fwd_n(const Geo& g, const Member<T>* M, int B, int mode, cudaStream_t st, bool pdl) {
     return for_member_sets(M, B, [&](const auto& ms, int nb) {
         constexpr int CAP = PD_CAP(ms);
         if constexpr (CAP == 1 || batch_len<N>())
-            k_zpass_fwd<N, T, CAP><<<dim3(TCfg<N, true>::template tiles<T>(g), g.nkj, 3 * nb),
-                                     TCfg<N, true>::template nt<T>(), TCfg<N, true>::template smem<T>(), st>>>(ms, mode);
+            launch_after(pdl, k_zpass_fwd<N, T, CAP>, dim3(TCfg<N, 2>::template tiles<T>(g), g.nkj, 3 * nb),
+                         TCfg<N, 2>::template nt<T>(), TCfg<N, 2>::template smem<T>(), st, ms, mode);
     });
 }
 #undef PD_CAP
 
 #define PD_PASSES_INST_T(N, T)                                                                            \
     template cudaError_t configure_n<N, T>(const Geo&);                                                   \
-    template cudaError_t zpass_inv_n<N, T>(const Geo&, const Member<T>*, int, int, cudaStream_t, const ZMaps*); \
-    template cudaError_t ypass_inv_n<N, T>(const Geo&, const Member<T>*, int, cudaStream_t);              \
-    template cudaError_t xpass_n<N, T>(const Geo&, const Member<T>*, int, int, int, cudaStream_t);        \
+    template cudaError_t zpass_inv_n<N, T>(const Geo&, const Member<T>*, int, int, cudaStream_t, const ZMaps*, bool); \
+    template cudaError_t ypass_inv_n<N, T>(const Geo&, const Member<T>*, int, cudaStream_t, bool);              \
+    template cudaError_t xpass_n<N, T>(const Geo&, const Member<T>*, int, int, int, cudaStream_t, bool);        \
     template cudaError_t xpass_stats_n<N, T>(const Geo&, const Member<T>*, double*, cudaStream_t);        \
-    template cudaError_t ypass_fwd_n<N, T>(const Geo&, const Member<T>*, int, cudaStream_t);              \
-    template cudaError_t zpass_fwd_n<N, T>(const Geo&, const Member<T>*, int, int, cudaStream_t);
+    template cudaError_t ypass_fwd_n<N, T>(const Geo&, const Member<T>*, int, cudaStream_t, bool);              \
+    template cudaError_t zpass_fwd_n<N, T>(const Geo&, const Member<T>*, int, int, cudaStream_t, bool);
 #define PD_PASSES_INST(N) PD_PASSES_INST_T(N, double) PD_PASSES_INST_T(N, float)
 
 }  // namespace pd
