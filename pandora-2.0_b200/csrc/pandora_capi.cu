@@ -155,6 +155,15 @@ static long long force_calls(int NK) {
            3LL * NK * (2LL * NK + 1) * (2LL * NK + 1);
 }
 
+// The side stream of a step, of the highest priority: its few CTAs (statistics, sort, scalars) go
+// ahead of the main stream's next kernel, whose CTAs would otherwise take every free slot and
+// leave the update waiting for them.
+static cudaError_t create_side(cudaStream_t* s) {
+    int lo = 0, hi = 0;
+    const cudaError_t e = cudaDeviceGetStreamPriorityRange(&lo, &hi);
+    return e != cudaSuccess ? e : cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, hi);
+}
+
 static void release(pandora_handle* h) {
     if (!h) return;
     cudaSetDevice(h->dev);
@@ -307,7 +316,7 @@ extern "C" int pandora_create(const pandora_params* p, pandora_handle** out) {
         cudaGetLastError(); release(h); return PANDORA_ERR_OOM;
     }
     if ((e = cudaStreamCreateWithFlags(&h->own, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = create_side(&h->side)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&h->ev_side, cudaEventDisableTiming)) != cudaSuccess) {
@@ -683,13 +692,16 @@ template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, 
         return cudaEventRecordWithFlags(h->tev[stage - 1][ps - 1][end], s, cudaEventRecordExternal);
     };
     PD_CK(mark(1, 0, c.st));
-    PD_CK(launch_zpass_inv(g, M, B, stage, c.st, c.zmaps)); n += g.dealias_cut > 0.0 ? 2 : 1;   // k_dealias first
+    // programmatic dependents of the kernel before them (K5b or the time advance, K1, K2, K3 or
+    // the particles, K4); with pass timing an event stands between the passes
+    const bool pdl = !h || h->timing == 0;
+    PD_CK(launch_zpass_inv(g, M, B, stage, c.st, c.zmaps, pdl && stage > 1)); n += g.dealias_cut > 0.0 ? 2 : 1;   // k_dealias first
     PD_CK(mark(1, 1, c.st));
     PD_CK(mark(2, 0, c.st));
-    PD_CK(launch_ypass_inv(g, M, B, c.st)); n++;
+    PD_CK(launch_ypass_inv(g, M, B, c.st, pdl)); n++;
     PD_CK(mark(2, 1, c.st));
     PD_CK(mark(3, 0, c.st));
-    PD_CK(launch_xpass(g, M, B, part ? 1 : 0, stage == 1 ? 1 : 0, c.st)); n++;
+    PD_CK(launch_xpass(g, M, B, part ? 1 : 0, stage == 1 ? 1 : 0, c.st, pdl)); n++;
     PD_CK(mark(3, 1, c.st));
     const bool adv = scalars_advance(g, c.np);
     if (part) {
@@ -711,10 +723,10 @@ template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, 
         PD_CK(mark(6, 1, c.st));
     }
     PD_CK(mark(4, 0, c.st));
-    PD_CK(launch_ypass_fwd(g, M, B, c.st)); n++;
+    PD_CK(launch_ypass_fwd(g, M, B, c.st, pdl)); n++;
     PD_CK(mark(4, 1, c.st));
     PD_CK(mark(5, 0, c.st));
-    PD_CK(launch_zpass_fwd_update(g, M, B, stage, 0, c.st, side ? c.ev_side : nullptr)); n += 2;   // forward z FFT, RK update
+    PD_CK(launch_zpass_fwd_update(g, M, B, stage, 0, c.st, side ? c.ev_side : nullptr, pdl)); n += 2;   // forward z FFT, RK update
     PD_CK(mark(5, 1, c.st));
     if (!adv) { PD_CK(launch_advance_time(g, M, B, stage, c.st)); n++; }
     if (nlaunch) *nlaunch += n;
@@ -1342,7 +1354,7 @@ extern "C" int pandora_batch_create(const pandora_params* cls, int32_t capacity,
     b->cap = capacity;
     cudaError_t e;
     if ((e = cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = create_side(&b->side)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->ev_side, cudaEventDisableTiming)) != cudaSuccess) {
