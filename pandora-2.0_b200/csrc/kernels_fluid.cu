@@ -758,17 +758,20 @@ template <class T> cudaError_t launch_check_finite(const Geo& g, const Member<T>
 // it; the modes DEALIASING 2/3 drops are left out, as the real-space field holds none.
 // One CTA per m plane with a fixed-order block sum: P[2m], P[2m+1] = Re, Im.
 template <class T>
-__global__ void __launch_bounds__(256) k_xcorr_cospec(const __grid_constant__ MemberSet<T, 1> ms, double* P) {
+__global__ void __launch_bounds__(1024) k_xcorr_cospec(const __grid_constant__ MemberSet<T, 1> ms, double* P) {
     const FieldsT<T> F = ms.m[0].F;
     const Geo g = ms.m[0].g;
     const BF bf = make_bf(g, F.clock);
     const bool dealias = g.dealias_cut > 0.0;
     const int i = blockIdx.x;
-    const long long plane = (long long)g.nkj * g.nkk, base = (long long)i * plane;
+    const int plane = g.nkj * g.nkk;
+    const long long base = (long long)i * plane;
     double re = 0.0, im = 0.0;
-    for (long long q = threadIdx.x; q < plane; q += blockDim.x) {
-        const int j = (int)(q / g.nkk), k = (int)(q % g.nkk);
-        if (dealias && dealias_drop(g, bf, (double)i, wvn(j, g.kj), wvn(k, g.kk))) continue;
+    for (int q = threadIdx.x; q < plane; q += blockDim.x) {
+        if (dealias) {
+            const int j = q / g.nkk, k = q - j * g.nkk;
+            if (dealias_drop(g, bf, (double)i, wvn(j, g.kj), wvn(k, g.kk))) continue;
+        }
         const double2 b = to_d(F.u[0][base + q]);
         double2 a = b;
         if (g.shear) {
@@ -778,7 +781,7 @@ __global__ void __launch_bounds__(256) k_xcorr_cospec(const __grid_constant__ Me
         re += a.x * b.x + a.y * b.y;
         im += a.y * b.x - a.x * b.y;
     }
-    __shared__ double sr[8], si[8];
+    __shared__ double sr[32], si[32];
     for (int o = 16; o > 0; o >>= 1) {
         re += __shfl_xor_sync(0xffffffffu, re, o);
         im += __shfl_xor_sync(0xffffffffu, im, o);
@@ -787,7 +790,7 @@ __global__ void __launch_bounds__(256) k_xcorr_cospec(const __grid_constant__ Me
     __syncthreads();
     if (threadIdx.x == 0) {
         double tr = 0.0, ti = 0.0;
-        for (int w = 0; w < 8; w++) { tr += sr[w]; ti += si[w]; }
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) { tr += sr[w]; ti += si[w]; }
         P[2 * i] = tr;
         P[2 * i + 1] = ti;
     }
@@ -796,7 +799,7 @@ __global__ void __launch_bounds__(256) k_xcorr_cospec(const __grid_constant__ Me
 template <class T> cudaError_t launch_xcorr_cospec(const Member<T>& m, double* P, cudaStream_t st) {
     MemberSet<T, 1> one;
     one.m[0] = m;
-    k_xcorr_cospec<T><<<(unsigned)m.g.nki, 256, 0, st>>>(one, P);
+    k_xcorr_cospec<T><<<(unsigned)m.g.nki, 1024, 0, st>>>(one, P);
     return cudaGetLastError();
 }
 

@@ -999,11 +999,15 @@ extern "C" int pandora_x_correlation(pandora_handle* h, double* r, int32_t n) {
     PD_CK(cudaMemcpyAsync(P.data(), h->rsbuf, sizeof(double) * 2 * nki, cudaMemcpyDeviceToHost, h->st));
     PD_CK(cudaStreamSynchronize(h->st));
     const double npts = (double)h->g.R, w = 6.283185307179586476925286766559005768 / (double)nx;
+    // the phases m l mod nx (reduced exactly) take nx values: their cosines and sines once, not
+    // for each of the nl x nki terms (0.3 ms of host time at 256 points)
+    std::vector<double> cs((size_t)2 * nx);
+    for (int q = 0; q < nx; q++) { cs[2 * q] = std::cos(w * (double)q); cs[2 * q + 1] = std::sin(w * (double)q); }
     for (int l = 0; l < nl; l++) {
         double acc = 0.0;
         for (int m = 0; m < nki; m++) {
-            const double th = w * (double)(((long long)m * l) % nx);   // the phase reduced exactly
-            const double t = P[2 * m] * std::cos(th) + P[2 * m + 1] * std::sin(th);
+            const size_t q = (size_t)(((long long)m * l) % nx);
+            const double t = P[2 * m] * cs[2 * q] + P[2 * m + 1] * cs[2 * q + 1];
             acc += m == 0 ? t : 2.0 * t;
         }
         r[l] = npts * acc;
