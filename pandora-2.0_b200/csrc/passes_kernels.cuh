@@ -444,15 +444,20 @@ __global__ void __launch_bounds__(32, RS ? XCfgStats<NX, T>::ctas() : XCfg<NX, T
 // and then one at a time.  Optionally writes the physical velocity (laboratory
 // components) for the particles.  Batches: the member is blockIdx.y, as in K3.
 // ---------------------------------------------------------------------------
+// One warp per CTA, as K3: the pass is bound by its shared-memory wavefronts and by warps in
+// flight, and eight-warp CTAs held their registers until the last line was done.  192^3 per step
+// 1.756 -> 1.708 ms FP64, 1.07 -> 0.936 FP32-mixed; 256^3 4.28 -> 3.74 and 2.155 -> 1.93.
 template <int N, class T> struct ConvCfg {
-    static constexpr int per_warp = 4 * xas<N>() * (int)sizeof(typename Cplx<T>::type);
-    static constexpr int fit = (200 * 1024) / per_warp;
-    static constexpr int NW = fit >= 8 ? 8 : (fit < 1 ? 1 : fit);
-    static constexpr size_t smem = (size_t)NW * per_warp;
+    static constexpr size_t smem = 4 * xas<N>() * sizeof(typename Cplx<T>::type);
+    // CTAs per SM asked of the register allocator, in steps of four (XCfg::ctas): FP64 with 12
+    // 1.716 ms at 192^3, FP32 with 20 0.975
+    static constexpr int fit = (int)(232448 / (smem + 1024)) / 4 * 4;
+    static constexpr int want = sizeof(T) == 8 ? 16 : 24;
+    static constexpr int ctas = fit < 4 ? 4 : (fit < want ? fit : want);
 };
 
 template <int NX, class T, int CAP>
-__global__ void __launch_bounds__(32 * ConvCfg<NX, T>::NW, 1) k_xpass_conv(const __grid_constant__ MemberSet<T, CAP> ms,
+__global__ void __launch_bounds__(32, ConvCfg<NX, T>::ctas) k_xpass_conv(const __grid_constant__ MemberSet<T, CAP> ms,
                                                                           int want_phys, int want_cfl, long long pf_lines) {
     using C = typename FieldsT<T>::C;
     using XP = pdfft::FusedPlan<NX>;   // the backward plan r0, r1, r2 (run unfused here)
@@ -464,15 +469,14 @@ __global__ void __launch_bounds__(32 * ConvCfg<NX, T>::NW, 1) k_xpass_conv(const
     }
     const FieldsT<T> F = mm.F;
     const Geo g = mm.g;
-    constexpr int XPS = xps<NX>(), XAS = xas<NX>(), NA = xna<NX>(), NW = ConvCfg<NX, T>::NW;
+    constexpr int XPS = xps<NX>(), XAS = xas<NX>(), NA = xna<NX>();
     constexpr int KB = NX / 3;
     constexpr int R0 = XP::r0, R1 = XP::r1, R2 = XP::r2, NP = XP::np;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int lane = threadIdx.x;
     const long long lines = (long long)g.ny * g.nz;
     const C* tw = F.tw_x;
-    const long long q = (long long)blockIdx.x * NW + w;
-    if (q >= lines) return;                       // whole warp; no block barrier follows
-    C* s = smem_as<C>() + (size_t)w * 4 * XAS;
+    const long long q = blockIdx.x;
+    C* s = smem_as<C>();
     constexpr int NKI = NX / 3 + 1, NKIP = (NKI + 7) / 8 * 8;   // g.nki, g.nkip
     const long long fstride = lines * NKIP;
     C* b = F.yb + q * NKIP;
@@ -559,7 +563,7 @@ __global__ void __launch_bounds__(32 * ConvCfg<NX, T>::NW, 1) k_xpass_conv(const
     __syncwarp();
     if (want_cfl) {
         for (int o = 16; o > 0; o >>= 1) umax = fmax(umax, __shfl_xor_sync(0xffffffffu, umax, o));
-        if (threadIdx.x % 32 == 0) atomicMax(&F.clock->ucfl_bits, (unsigned long long)__double_as_longlong((double)umax));
+        if (lane == 0) atomicMax(&F.clock->ucfl_bits, (unsigned long long)__double_as_longlong((double)umax));
     }
     if (pf_lines > 0 && q + pf_lines < lines && lane < 9)
         prefetch_l2(F.yb + lane * fstride + (q + pf_lines) * NKIP, NKI * sizeof(C));

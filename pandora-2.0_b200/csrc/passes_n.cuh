@@ -186,11 +186,9 @@ cudaError_t xpass_n(const Geo& g, const Member<T>* M, int B, int want_phys, int 
         constexpr int CAP = PD_CAP(ms);
         if constexpr (CAP == 1 || batch_len<N>()) {
             if (g.rconv) {   // R-conv: its own x pass
-                constexpr int NW = ConvCfg<N, T>::NW;
-                const long long nl = (lines + NW - 1) / NW;
-                const long long pf = CAP == 1 ? NW * resident_ctas(k_xpass_conv<N, T, CAP>, 32 * NW, ConvCfg<N, T>::smem) : 0;
-                launch_after(pdl, k_xpass_conv<N, T, CAP>, dim3((unsigned)nl, nb), 32 * NW, ConvCfg<N, T>::smem, st, ms,
-                             want_phys, want_cfl, pf);
+                auto kern = k_xpass_conv<N, T, CAP>;
+                const long long pf = CAP == 1 ? resident_ctas(kern, 32, ConvCfg<N, T>::smem) : 0;
+                launch_after(pdl, kern, dim3((unsigned)lines, nb), 32, ConvCfg<N, T>::smem, st, ms, want_phys, want_cfl, pf);
                 return;
             }
             auto go = [&](auto lpwc) {
