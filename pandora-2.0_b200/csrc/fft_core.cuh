@@ -140,7 +140,8 @@ constexpr unsigned odd_bits(unsigned z) { return even_bits(z >> 1); }
 constexpr double kSqrtHalf = 0.7071067811865475244008444;
 constexpr double kSin60 = 0.8660254037844386467637232;
 
-// DFTs of 2..32 points in registers.  Z: mask of the inputs that are zero at compile time.
+// DFTs of 2..32 points in registers (2, 3, 4, 5, 7, 8, 10, 12, 14, 16, 20, 24, 28, 32).  Z: mask
+// of the inputs that are zero at compile time.
 template <int S, unsigned Z = 0, class C> PD_HD void dft2(C* v) {
     C a = v[0], b = v[1];
     addsub<(Z & 1u) != 0, (Z & 2u) != 0>(a, b, v[0], v[1]);
@@ -289,6 +290,54 @@ template <int R, int S, unsigned Z = 0, class C> PD_HD void dft_prime(C* v) {
     }
 }
 
+// R = P Q with P = 2, 4 or 8 and Q = 3, 5 or 7, without twiddles (the prime-factor mapping of
+// Good, 1958): with n = Q n1 + P n2 mod R the kernel splits into exp(2 pi i n1 k / P) exp(2 pi i n2 k / Q), so
+// P-point DFTs over n1 and Q-point DFTs over n2 give X_k for k = k1 mod P, k = k2 mod Q.
+template <int I, int N, class F> PD_HD void for_range(F& f);
+template <int I> struct Ix { static constexpr int value = I; };
+template <int I, int N, class F> PD_HD void for_range(F& f) {
+    if constexpr (I < N) {
+        f(Ix<I>{});
+        for_range<I + 1, N>(f);
+    }
+}
+template <int P, int Q> constexpr int crt(int k1, int k2) {
+    for (int k = 0; k < P * Q; k++)
+        if (k % P == k1 && k % Q == k2) return k;
+    return -1;
+}
+template <int P, int Q> constexpr unsigned pfa_mask(unsigned z, int n2) {
+    unsigned r = 0;
+    for (int n1 = 0; n1 < P; n1++) r |= ((z >> ((Q * n1 + P * n2) % (P * Q))) & 1u) << n1;
+    return r;
+}
+template <int P, int Q, int S, unsigned Z = 0, class C> PD_HD void dft_pfa(C* v) {
+    C y[P][Q];
+    auto rows = [&](auto ix) {
+        constexpr int n2 = decltype(ix)::value;
+        C t[P];
+#pragma unroll
+        for (int n1 = 0; n1 < P; n1++) t[n1] = v[(Q * n1 + P * n2) % (P * Q)];
+        if constexpr (P == 2) dft2<S, pfa_mask<P, Q>(Z, n2)>(t);
+        else if constexpr (P == 4) dft4<S, pfa_mask<P, Q>(Z, n2)>(t);
+        else dft8<S, pfa_mask<P, Q>(Z, n2)>(t);
+#pragma unroll
+        for (int n1 = 0; n1 < P; n1++) y[n1][n2] = t[n1];
+    };
+    for_range<0, Q>(rows);
+    auto cols = [&](auto ix) {
+        constexpr int k1 = decltype(ix)::value;
+        if constexpr (Q == 3) dft3<S>(y[k1]);
+        else dft_prime<Q, S>(y[k1]);
+        auto put = [&](auto iy) {
+            constexpr int k2 = decltype(iy)::value, k = crt<P, Q>(k1, k2);
+            v[k] = y[k1][k2];
+        };
+        for_range<0, Q>(put);
+    };
+    for_range<0, P>(cols);
+}
+
 template <int R, int S, unsigned Z = 0, class C> PD_HD void dft(C* v) {
     if constexpr (R == 2) dft2<S, Z>(v);
     else if constexpr (R == 3) dft3<S>(v);
@@ -298,12 +347,19 @@ template <int R, int S, unsigned Z = 0, class C> PD_HD void dft(C* v) {
     else if constexpr (R == 12) dft12<S>(v);
     else if constexpr (R == 32) dft32<S, Z>(v);
     else if constexpr (R == 5 || R == 7) dft_prime<R, S, Z>(v);
+    else if constexpr (R == 10) dft_pfa<2, 5, S, Z>(v);
+    else if constexpr (R == 14) dft_pfa<2, 7, S, Z>(v);
+    else if constexpr (R == 20) dft_pfa<4, 5, S, Z>(v);
+    else if constexpr (R == 24) dft_pfa<8, 3, S, Z>(v);
+    else if constexpr (R == 28) dft_pfa<4, 7, S, Z>(v);
     else static_assert(R == 2, "unsupported radix");
 }
 
 // Radix schedule per transform length.  Supported N: 2^a * {1,3,5,7} from 16 to 1024,
-// factored into the radices below (2, 3, 4, 5, 7, 8, 12, 16; 32 in warp plans) in at most three passes;
-// lengths with a factor 3 take a radix-12 pass where that saves a pass.
+// factored into at most three radices.  Composite radices with a factor 3, 5 or 7 where they save
+// a pass, each a shared-memory round trip and a barrier: two passes against three took the shear
+// step of 160^3 from 0.819 to 0.659 ms (FP32-mixed 0.452 -> 0.377), 224^3 2.02 -> 1.64 (1.28 ->
+// 0.91), 320^3 5.49 -> 4.99 (3.30 -> 2.72), 384^3 12.1 -> 9.32 (6.23 -> 4.66).
 template <int N> struct Plan { static constexpr int r0 = 0, r1 = 0, r2 = 0; };
 #define PD_PLAN(N_, A, B, C) \
     template <> struct Plan<N_> { static constexpr int r0 = A, r1 = B, r2 = C; };
@@ -318,12 +374,12 @@ PD_PLAN(80, 5, 16, 0)
 PD_PLAN(96, 8, 12, 0)
 PD_PLAN(112, 7, 16, 0)
 PD_PLAN(128, 8, 16, 0)
-PD_PLAN(160, 5, 4, 8)
+PD_PLAN(160, 10, 16, 0)
 PD_PLAN(192, 16, 12, 0)
-PD_PLAN(224, 7, 4, 8)
+PD_PLAN(224, 14, 16, 0)
 PD_PLAN(256, 16, 16, 0)
-PD_PLAN(320, 5, 8, 8)
-PD_PLAN(384, 3, 8, 16)
+PD_PLAN(320, 20, 16, 0)
+PD_PLAN(384, 24, 16, 0)
 PD_PLAN(448, 7, 8, 8)
 PD_PLAN(512, 8, 8, 8)
 PD_PLAN(640, 5, 8, 16)
@@ -562,13 +618,24 @@ template <int N> constexpr bool wplan_ok() {
     return WPlan<N>::r0 * (WPlan<N>::r1 ? WPlan<N>::r1 : 1) * (WPlan<N>::r2 ? WPlan<N>::r2 : 1) == N;
 }
 
-// Fewer, larger passes (radix 16) for kernels limited by shared-memory bandwidth
-// rather than by registers: each pass costs a full read and write of the line.
+// Fewer, larger passes for kernels limited by shared-memory bandwidth rather than by registers:
+// each pass costs a full read and write of the line.  The two-pass plans of 160 to 448 points
+// took the shear step of 160^3 from 0.872 to 0.819 ms (FP32-mixed 0.503 -> 0.452), 224^3 2.27 ->
+// 2.02, 320^3 6.6 -> 5.49, 448^3 16.8 -> 13.95 (11.4 -> 7.98); those of 640 to 896 points, which
+// in FP32 also let the product step run in registers, 640^3 67.8 -> 63.1 (30.5 -> 22.9), 768^3
+// 125.9 -> 117.7 (48.2 -> 39.4), 896^3 181.2 -> 166.0.
 template <int N> struct WPlanL : WPlan<N> {};
 template <> struct WPlanL<128> { static constexpr int r0 = 16, r1 = 8, r2 = 0; };
+template <> struct WPlanL<160> { static constexpr int r0 = 10, r1 = 16, r2 = 0; };
+template <> struct WPlanL<224> { static constexpr int r0 = 14, r1 = 16, r2 = 0; };
 template <> struct WPlanL<256> { static constexpr int r0 = 16, r1 = 16, r2 = 0; };
+template <> struct WPlanL<320> { static constexpr int r0 = 20, r1 = 16, r2 = 0; };
 template <> struct WPlanL<384> { static constexpr int r0 = 32, r1 = 12, r2 = 0; };
+template <> struct WPlanL<448> { static constexpr int r0 = 28, r1 = 16, r2 = 0; };
 template <> struct WPlanL<512> { static constexpr int r0 = 32, r1 = 16, r2 = 0; };
+template <> struct WPlanL<640> { static constexpr int r0 = 20, r1 = 32, r2 = 0; };
+template <> struct WPlanL<768> { static constexpr int r0 = 24, r1 = 32, r2 = 0; };
+template <> struct WPlanL<896> { static constexpr int r0 = 28, r1 = 32, r2 = 0; };
 template <> struct WPlanL<1024> { static constexpr int r0 = 32, r1 = 32, r2 = 0; };
 
 // Plan of a backward transform, a pointwise product and a forward transform run

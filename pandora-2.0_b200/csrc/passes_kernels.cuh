@@ -96,7 +96,7 @@ __device__ __forceinline__ void grid_wait() {
 
 template <int N> constexpr int xps() {
     return (N == 16 || N == 32 || N == 48) ? 2
-         : ((N == 24 || N == 64 || N == 96) ? 3 : ((N == 384 || N == 512 || N == 1024) ? 5 : 4));
+         : ((N == 24 || N == 64 || N == 96) ? 3 : ((N == 384 || N >= 512) ? 5 : 4));
 }
 template <int N> constexpr int xas() { return (tile_rows<N, xps<N>()>() + 7) / 8 * 8 + 4; }
 
@@ -119,13 +119,15 @@ template <int N, class T> struct XCfg {
     // Pads per length: the fewest wavefronts of all accesses of the pass, counted over quarter
     // (FP64) or half warps (FP32) with this lane mapping.
     static constexpr int pad64() {
-        return N == 16 ? 2 : N == 48 ? 3 + 16 * 5 : (N == 56 || N == 112 || N == 224 || N == 256) ? 4
-             : N == 80 ? 3 + 16 * 4 : N == 128 ? 3 + 16 * 6 : (N == 192 || N == 512) ? 4 + 16 * 7 : N == 384 ? 5 : 3;
+        return N == 16 ? 2 : N == 48 ? 3 + 16 * 5 : (N == 56 || N == 112 || N == 224 || N == 256 || N == 448) ? 4
+             : N == 80 ? 3 + 16 * 4 : N == 128 ? 3 + 16 * 6 : N == 160 ? 4 + 16 * 5
+             : (N == 192 || N == 320 || N == 512) ? 4 + 16 * 7 : N == 384 ? 5 : 3;
     }
     static constexpr int pad32() {
-        return N == 16 ? 2 : N == 48 ? 3 + 16 * 5 : (N == 56 || N == 112 || N == 128 || N == 256) ? 4
-             : N == 80 ? 3 + 16 * 4 : N == 192 ? 4 + 16 * 6 : N == 512 ? 4 + 16 * 8
-             : (N == 160 || N == 224 || N == 384 || N == 1024) ? 5 : 3;
+        return N == 16 ? 2 : N == 48 ? 3 + 16 * 5 : (N == 56 || N == 112 || N == 128 || N == 224 || N == 256) ? 4
+             : N == 80 ? 3 + 16 * 4 : N == 160 ? 4 + 16 * 5 : N == 192 ? 4 + 16 * 6 : N == 320 ? 5 + 16 * 6
+             : (N == 448 || N == 512) ? 4 + 16 * 8 : N == 640 ? 5 + 16 * 6 : N == 896 ? 5 + 16 * 8
+             : (N == 384 || N >= 768) ? 5 : 3;
     }
     static constexpr int ps = !triple ? xps<N>() : (sizeof(T) == 8 ? pad64() : pad32());
     static constexpr int q = sizeof(T) == 8 ? 8 : 16;
@@ -744,16 +746,26 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_rk_update(const
 // inputs straight from HBM and the last pass writing its outputs straight to
 // HBM, so a 256-point line crosses shared memory once (one block barrier).
 // ---------------------------------------------------------------------------
+// FP32 lines of 448 and 640 to 896 points take two passes, one shared-memory round trip and one
+// barrier instead of two (shear step of 448^3 7.92 -> 6.92 ms, 640^3 35.5 -> 30.4, 768^3 56.4 ->
+// 48.1).  Not FP64: a butterfly of radix 28 or 32 leaves too few warps (448^3 13.8 -> 14.3).
+// Not 1024 points, whose (32, 32) fits three CTAs but waits on its loads (1024^3 89.0 -> 99.9).
+template <int N, class T> struct TPlan : pdfft::Plan<N> {};
+template <> struct TPlan<448, float> { static constexpr int r0 = 28, r1 = 16, r2 = 0; };
+template <> struct TPlan<640, float> { static constexpr int r0 = 20, r1 = 32, r2 = 0; };
+template <> struct TPlan<768, float> { static constexpr int r0 = 24, r1 = 32, r2 = 0; };
+template <> struct TPlan<896, float> { static constexpr int r0 = 28, r1 = 32, r2 = 0; };
+
 // KIND: 0 K1, 1 the y passes, 2 K5a.
 template <int N, int KIND = 0> struct TCfg {
-    // Radix plan: Plan<N>, or in the y passes and K5a for FP32 512-point
+    // Radix plan: TPlan, or in the y passes and K5a for FP32 512-point
     // lines the two-pass (32, 16): one shared-memory round trip instead of two.  An
     // FP64 item of radix 32 does not fit the registers of two CTAs per SM, and K1
-    // (vorticity loads in its first pass) measured slower with it.
+    // (vorticity loads in its first pass) gains nothing from it.
     template <class T> static constexpr bool two() { return KIND > 0 && sizeof(T) == 4 && N == 512; }
-    template <class T> static constexpr int r0() { return two<T>() ? 32 : pdfft::Plan<N>::r0; }
-    template <class T> static constexpr int r1() { return two<T>() ? 16 : pdfft::Plan<N>::r1; }
-    template <class T> static constexpr int r2() { return two<T>() ? 0 : pdfft::Plan<N>::r2; }
+    template <class T> static constexpr int r0() { return two<T>() ? 32 : TPlan<N, T>::r0; }
+    template <class T> static constexpr int r1() { return two<T>() ? 16 : TPlan<N, T>::r1; }
+    template <class T> static constexpr int r2() { return two<T>() ? 0 : TPlan<N, T>::r2; }
     // threads per CTA: one butterfly per thread in the widest pass of a tile (of 8 lines' worth)
     template <class T> static constexpr int nt() {
         return pdfft::tile_threads_for<N, r0<T>(), r1<T>(), r2<T>(), (lines<T>() == 4 ? 4 : 8)>();
@@ -777,13 +789,14 @@ template <int N, int KIND = 0> struct TCfg {
     // 1.18 -> 0.92 ms, K4 0.57 -> 0.43, K5 0.71 -> 0.59; 320^3 K4 0.30 -> 0.18; 448^3 K4 0.70 -> 0.43; 640^3
     // K1 3.30 -> 3.07, K5 2.97 -> 2.64), but one for K5a at 320 and 448 points (0.31 against 0.35
     // ms, 0.79 against 0.84).
+    // FP32 items of radix 32 take 80 registers: three CTAs of 256 threads.
     template <class T> static constexpr int minb() {
         constexpr int NT = nt<T>();
         if (lines<T>() == 4) return NT <= 256 ? 4 : 2;
         if (sizeof(T) == 8 && NT > 256)
             return (KIND == 2 && (N == 320 || N == 448)) || (KIND == 1 && N == 768) || N > 768 ? 1 : 2;
         return (sizeof(T) == 8 || lines<T>() == 16) ? (NT <= 128 ? (N == 192 ? 4 : 5) : 2)
-                                                    : (NT <= 128 ? (N == 192 ? 6 : 8) : (NT <= 256 ? 4 : 2));
+                                                    : (NT <= 128 ? (N == 192 ? 6 : 8) : (NT <= 256 ? (r1<T>() == 32 ? 3 : 4) : 2));
     }
     // pad rows of the FP32 tiles of 8 lines (64-byte rows); at 1024 points, two butterflies per
     // thread, the padded index does not fit the 64 registers (K2 of 1024^3 5.50 -> 5.85 ms)
@@ -1084,7 +1097,7 @@ __global__ void __launch_bounds__(ZStage<NZ>::nt, 2) k_zpass_inv_tma(const __gri
 template <int N, class T> struct SCfg {
     using C = typename Cplx<T>::type;
     static constexpr int ce = (int)sizeof(C);
-    static constexpr int r0 = pdfft::Plan<N>::r0, r1 = pdfft::Plan<N>::r1, r2 = pdfft::Plan<N>::r2;
+    static constexpr int r0 = TPlan<N, T>::r0, r1 = TPlan<N, T>::r1, r2 = TPlan<N, T>::r2;
     static constexpr int lines = (N > 512 || (sizeof(T) == 8 && N > 256)) ? 4 : 8;
     static constexpr int ps = pdfft::tile_pad<ce * lines, r0>();
     // row pitch: the lanes of a wavefront (M values of 128 bytes) read q consecutive k of each line

@@ -58,6 +58,21 @@ def test_mixed_nonlinear_every_tile_shape(gpu_lib, dims):
     assert e < 1e-5, e
 
 
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("n", [160, 224, 320, 384, 448, 640, 768, 896])
+def test_mixed_nonlinear_two_pass_lengths(gpu_lib, n, axis):
+    """The lengths of the prime-factor radices in FP32 along each axis (their plans are not those
+    of FP64 from 448 points on); odd numbers of lines and of tiles on the other two."""
+    p = gpu_lib.workload_params("iso_decay", 32)
+    dims = [24, 16, 16]
+    dims[axis] = n
+    p.nodes_x, p.nodes_y, p.nodes_z = dims
+    o, s = _mixed(gpu_lib, p)
+    e = rel_l2_fields(s.nonlinear(), o.nonlinear())
+    s.close()
+    assert e < 1e-5, e   # the bar of the other lengths
+
+
 def test_mixed_decay_10_steps(gpu_lib):
     p = gpu_lib.workload_params("iso_decay", 64)
     o, s = _mixed(gpu_lib, p)
