@@ -785,16 +785,15 @@ template <int N, int KIND = 0> struct TCfg {
     }
     // resident CTAs per SM asked of the register allocator: an FP32 tile of 16 lines
     // holds the registers and shared memory of an FP64 one, of 8 lines half of them.  FP64 tiles of
-    // 512 threads: two (64 registers) where they fit, against one of 128 registers (384^3: K2
-    // 1.18 -> 0.92 ms, K4 0.57 -> 0.43, K5 0.71 -> 0.59; 320^3 K4 0.30 -> 0.18; 448^3 K4 0.70 -> 0.43; 640^3
-    // K1 3.30 -> 3.07, K5 2.97 -> 2.64), but one for K5a at 320 and 448 points (0.31 against 0.35
-    // ms, 0.79 against 0.84).
+    // 512 threads: two (64 registers) where they fit, against one of 128 registers (448^3 K4 0.70 ->
+    // 0.43 ms; 640^3 K1 3.30 -> 3.07, K5 2.97 -> 2.64), but one for K5a at 448 points (0.79 against
+    // 0.84).
     // FP32 items of radix 32 take 80 registers: three CTAs of 256 threads.
     template <class T> static constexpr int minb() {
         constexpr int NT = nt<T>();
         if (lines<T>() == 4) return NT <= 256 ? 4 : 2;
         if (sizeof(T) == 8 && NT > 256)
-            return (KIND == 2 && (N == 320 || N == 448)) || (KIND == 1 && N == 768) || N > 768 ? 1 : 2;
+            return (KIND == 2 && N == 448) || (KIND == 1 && N == 768) || N > 768 ? 1 : 2;
         return (sizeof(T) == 8 || lines<T>() == 16) ? (NT <= 128 ? (N == 192 ? 4 : 5) : 2)
                                                     : (NT <= 128 ? (N == 192 ? 6 : 8) : (NT <= 256 ? (r1<T>() == 32 ? 3 : 4) : 2));
     }
