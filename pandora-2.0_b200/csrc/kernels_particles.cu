@@ -261,13 +261,17 @@ __global__ void __launch_bounds__(256, part_ctas<ORD, T>()) k_particles(const __
         // p_ControlInitPartVelocity(BF) at the release step (src/pp_control.f90:378-516)
         if (release) { up[q] = uc[q]; pr[q] = 0.0; ur[q] = 0.0; }
     }
+    // shear: minus the homogeneous source amat up (p_RK3ComputeHomogeneousSourceTerm,
+    // src/pp_rk3.f90:1080-1102); amat has the single entry (1,3).  Exchanged ahead of the drag
+    // branch, which parts a warp that holds tracers and heavy particles.
+    double hs0 = 0.0;
+    if (bfrot) {       // uniform over the CTA
+        double up3 = up[NC - 1];
+        if constexpr (NC == 1) up3 = __shfl_sync(0xffffffffu, up[0], base + 2);
+        hs0 = g.shear_s * up3;
+    }
     if (dpv > 0.0) {   // uniform over the group
         const double tau = ((dpv * dpv) / (18.0 * mm.pp.f_nu)) * (mm.pp.p_rho / mm.pp.f_rho);
-        // shear: minus the homogeneous source amat up (p_RK3ComputeHomogeneousSourceTerm,
-        // src/pp_rk3.f90:1080-1102); amat has the single entry (1,3)
-        double up3 = up[NC - 1];
-        if constexpr (NC == 1) up3 = __shfl_sync(__activemask(), up[0], base + 2);
-        const double hs0 = bfrot ? g.shear_s * up3 : 0.0;
 #pragma unroll
         for (int q = 0; q < NC; q++) {
             const bool first = NC == 3 ? q == 0 : sub == 0;

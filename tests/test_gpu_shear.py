@@ -198,6 +198,39 @@ def test_shear_particles(gpu_lib):
     s.close()
 
 
+@pytest.mark.parametrize("order", [2, 4, 6])
+def test_shear_tracers_among_heavy_particles(gpu_lib, order):
+    """Tracers (diameter 0) and heavy particles in the same warps, BF-rot: the drag branch parts
+    a warp, and the source term S up3 of a heavy particle's first component comes from the
+    thread of its third (orders 3 to 6; up to order 2 one thread holds all three).  Across the
+    remesh (step 9), positions and velocities against the oracle; the number of particles is no
+    multiple of a warp's."""
+    import oracle as O
+    p = _shear(gpu_lib, 32, remesh_t=4, npart=2043)
+    p.p_interp_order, p.p_rho = order, 1000.0
+    o = O.Oracle(p)
+    s = gpu_lib.Simulation(p)
+    s.init_fluid()
+    s.init_particles()
+    xp, up, ur, pr, _ = s.get_particles()
+    dp = np.where(np.random.default_rng(order).random(len(xp)) < 0.5, 0.0, 0.01)
+    s.set_particles(xp, up, ur, pr, dp)
+    o.set_state(s.get_state())
+    o.set_particles(xp, up, ur, pr, dp)
+    t = 0.0
+    for step in range(1, 13):
+        t, _ = o.step(step, t)
+        s.step(step)
+    xg, ug, _, _, dg = s.get_particles()
+    xo, uo = o.get_particles(p.p_np_global)[:2]
+    s.check_status()
+    s.close()
+    assert np.array_equal(dg, dp)
+    d = np.abs(xg - xo)
+    assert np.minimum(d, 2 * np.pi - d).max() < 1e-10
+    assert rel_l2(ug, uo) < 1e-10      # the bars of the other particle tests
+
+
 @pytest.mark.parametrize("form", [0, 1, 2, 3])
 @pytest.mark.parametrize("dims", [(32, 48, 512), (24, 16, 512)])
 def test_staged_k1_lengths_and_forms(gpu_lib, form, dims):
