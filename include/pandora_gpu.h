@@ -203,7 +203,7 @@ int pandora_init_particles(pandora_handle* h);
 int pandora_rk3_step(pandora_handle* h, int32_t tstep, double* simtime, double* dt);
 /* nsteps steps tstep0 .. tstep0+nsteps-1, enqueued on the stream without host
  * synchronisation (simtime/dt live on the device); *simtime is updated when
- * sync != 0. */
+ * sync != 0.  Refused (PANDORA_ERR_CUDA) on a stream that is being captured. */
 int pandora_rk3_advance(pandora_handle* h, int32_t tstep0, int32_t nsteps, int32_t sync,
                         double* simtime);
 /* One stage (1..3) of step tstep at time `time`; *dt in/out as in f_RK3Stage*. */

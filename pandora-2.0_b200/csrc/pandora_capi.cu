@@ -804,6 +804,10 @@ extern "C" int pandora_rk3_advance(pandora_handle* h, int32_t tstep0, int32_t ns
                                    double* simtime) {
     if (!h || nsteps < 0 || !simtime) return PANDORA_ERR_INVALID_ARG;
     cudaSetDevice(h->dev);
+    // no part of a caller's graph: its replays would each begin again at this call's step and time
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    PD_CK(cudaStreamIsCapturing(h->st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return cuda_fail(cudaErrorStreamCaptureUnsupported, "pandora_rk3_advance");
     int rc = set_clock(h, tstep0, *simtime);
     if (rc) return rc;
     if (h->use_graph) {

@@ -285,6 +285,38 @@ def test_advance_matches_steps(gpu_lib):
     b.close()
 
 
+def test_advance_is_refused_under_capture(gpu_lib):
+    """Steps set the clock from the call's arguments, so they are no part of a caller's graph:
+    on a capturing stream the call fails, with and without the step's own graph in hand, the
+    capture stays usable, and the simulation goes on as if the call had not been made."""
+    import torch
+    p = gpu_lib.workload_params("iso_decay", 32)
+    a, b = gpu_lib.Simulation(p), gpu_lib.Simulation(p)
+    a.init_fluid()
+    b.init_fluid()
+    st = torch.cuda.Stream()
+    b.set_stream(st.cuda_stream)
+    for step in range(1, 3):
+        with torch.cuda.stream(st):
+            g = torch.cuda.CUDAGraph()
+            x = torch.zeros(4, device="cuda")
+            g.capture_begin(capture_error_mode="thread_local")
+            x.add_(1.0)
+            for sync in (False, True):
+                with pytest.raises(gpu_lib.PandoraError) as ei:
+                    b.advance(1, sync=sync)
+                assert ei.value.status == -3
+            g.capture_end()
+        assert b.tstep == step - 1
+        a.advance(1)
+        b.advance(1)
+        assert b.simtime == a.simtime
+        assert all(np.array_equal(u, v) for u, v in zip(a.get_state(), b.get_state()))
+    b.set_stream(None)
+    a.close()
+    b.close()
+
+
 def test_nan_detection(gpu_lib):
     p = gpu_lib.workload_params("iso_decay", 16)
     with gpu_lib.Simulation(p) as s:
