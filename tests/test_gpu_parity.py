@@ -287,8 +287,9 @@ def test_advance_matches_steps(gpu_lib):
 
 def test_advance_is_refused_under_capture(gpu_lib):
     """Steps set the clock from the call's arguments, so they are no part of a caller's graph:
-    on a capturing stream the call fails, with and without the step's own graph in hand, the
-    capture stays usable, and the simulation goes on as if the call had not been made."""
+    on a capturing stream the call fails, with and without the step's own graph in hand and for
+    no steps at all (which would record the clock's values alone), the capture stays usable,
+    and the simulation goes on as if the call had not been made."""
     import torch
     p = gpu_lib.workload_params("iso_decay", 32)
     a, b = gpu_lib.Simulation(p), gpu_lib.Simulation(p)
@@ -302,9 +303,9 @@ def test_advance_is_refused_under_capture(gpu_lib):
             x = torch.zeros(4, device="cuda")
             g.capture_begin(capture_error_mode="thread_local")
             x.add_(1.0)
-            for sync in (False, True):
+            for n, sync in ((0, False), (1, False), (1, True)):
                 with pytest.raises(gpu_lib.PandoraError) as ei:
-                    b.advance(1, sync=sync)
+                    b.advance(n, sync=sync)
                 assert ei.value.status == -3
             g.capture_end()
         assert b.tstep == step - 1
