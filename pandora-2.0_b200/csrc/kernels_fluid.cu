@@ -221,7 +221,7 @@ __device__ __forceinline__ void advance_clock(const Geo& g, Clock* ck, int stage
     }
 }
 
-// advance: the kernel ends by advancing the stage's time (scalars_advance).
+// advance: the stage (1..3) to whose end the kernel advances the time (scalars_advance), 0: none.
 template <class T, int CAP>
 __global__ void __launch_bounds__(256) k_stage_scalars(const __grid_constant__ MemberSet<T, CAP> ms, int stage, int advance) {
     const Member<T>& mm = ms.m[CAP == 1 ? 0 : blockIdx.x];
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(256) k_stage_scalars(const __grid_constant__ M
     if (tstep >= fp.stop) {
         for (long long q = tid; q < 3 * fstride; q += blockDim.x) F.forcing[q] = mk(0.0, 0.0);
         __syncthreads();   // every thread has read the step number
-        if (advance && tid == 0) advance_clock(g, ck, stage);
+        if (advance && tid == 0) advance_clock(g, ck, advance);
         return;
     }
     const long long calls = fp.calls_per_stage;
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256) k_stage_scalars(const __grid_constant__ M
     }
     __syncthreads();
     for (int q = tid; q < 3 * plane; q += blockDim.x) ff[(q / plane) * fstride + q % plane] = pl[q];
-    if (advance && tid == 0) advance_clock(g, ck, stage);   // behind the barriers that follow its reads
+    if (advance && tid == 0) advance_clock(g, ck, advance);   // behind the barriers that follow its reads
 }
 
 template <class T, int CAP>
@@ -715,10 +715,10 @@ cudaError_t configure_fluid_kernels(const Geo& g, const ForceParams& fp) {
 }
 
 template <class T>
-cudaError_t launch_stage_scalars(const Geo& g, const Member<T>* M, int B, const ForceParams& fp, int stage, bool advance,
+cudaError_t launch_stage_scalars(const Geo& g, const Member<T>* M, int B, const ForceParams& fp, int stage, int advance,
                                  cudaStream_t st) {
     return for_member_sets(M, B, [&](const auto& ms, int nm) {
-        k_stage_scalars<T, PD_CAP(ms)><<<nm, 256, stage_scalars_smem(g, fp), st>>>(ms, stage, advance ? 1 : 0);
+        k_stage_scalars<T, PD_CAP(ms)><<<nm, 256, stage_scalars_smem(g, fp), st>>>(ms, stage, advance);
     });
 }
 
@@ -806,7 +806,7 @@ template <class T> cudaError_t launch_xcorr_cospec(const Member<T>& m, double* P
 #define PD_INST(T)                                                                                   \
     template cudaError_t launch_xcorr_cospec<T>(const Member<T>&, double*, cudaStream_t);            \
     template cudaError_t launch_stats<T>(const Geo&, const Member<T>*, int, cudaStream_t);           \
-    template cudaError_t launch_stage_scalars<T>(const Geo&, const Member<T>*, int, const ForceParams&, int, bool, \
+    template cudaError_t launch_stage_scalars<T>(const Geo&, const Member<T>*, int, const ForceParams&, int, int, \
                                                  cudaStream_t);                                      \
     template cudaError_t launch_advance_time<T>(const Geo&, const Member<T>*, int, int, cudaStream_t); \
     template cudaError_t launch_check_finite<T>(const Geo&, const Member<T>*, int, cudaStream_t);    \

@@ -655,6 +655,8 @@ template <class T> struct StepCtx {
     const Particles* sortP;      // the particles the sort reorders
     pandora_handle* timing;      // null: no pass timing
     const ZMaps* zmaps;          // null: K1 reads u element-wise (batches, FP32, other lengths)
+    bool unforced;               // no forcing acts in this step (unforced_step)
+    bool known_dt;               // the step's dt does not wait for the velocity's maximum
 };
 
 template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, int* nlaunch) {
@@ -703,15 +705,25 @@ template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, 
     PD_CK(mark(3, 0, c.st));
     PD_CK(launch_xpass(g, M, B, part ? 1 : 0, stage == 1 ? 1 : 0, c.st, pdl)); n++;
     PD_CK(mark(3, 1, c.st));
-    const bool adv = scalars_advance(g, c.np);
-    if (part) {
-        PD_CK(launch_stage_scalars(g, M, B, *c.fp, stage, adv, c.st)); n++;
-    } else {
-        PD_CK(cudaEventRecord(c.ev_fork, c.st));
-        PD_CK(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
-        PD_CK(launch_stage_scalars(g, M, B, *c.fp, stage, adv, c.side)); n++;
+    // Without forcing the scalars of stage 1 set the step's dt and zero forcing and, where they
+    // advance the time, that of the whole step (no kernel of stages 2 and 3 reads it then).
+    // Every fork of a step costs a new state's first step about 50 us of the graph's instantiation:
+    // 32^3 decay 430 us with a fork in every stage, 340 with those of stage 1, 290 where the
+    // scalars of stage 1 follow the statistics as well (without a side stream 255, and 100 us
+    // instead of 70 for the steps after it).  A forced flow, whose scalars draw every stage's
+    // random numbers, earns its forks back in six steps (265 -> 440 us, then 112 -> 82).
+    const bool adv = scalars_advance(g, c.np), scalars = stage == 1 || !c.unforced;
+    const int to = !adv ? 0 : (c.unforced ? 3 : stage);
+    if (part && scalars) {
+        PD_CK(launch_stage_scalars(g, M, B, *c.fp, stage, to, c.st)); n++;
+    } else if (scalars) {
+        if (!(c.unforced && c.known_dt)) {   // else they need nothing of K3 and follow the statistics
+            PD_CK(cudaEventRecord(c.ev_fork, c.st));
+            PD_CK(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
+        }
+        PD_CK(launch_stage_scalars(g, M, B, *c.fp, stage, to, c.side)); n++;
     }
-    const bool side = stage == 1 || !part;   // work on the side stream to wait for
+    const bool side = stage == 1 || (!part && scalars);   // work on the side stream to wait for
     if (side) PD_CK(cudaEventRecord(c.ev_side, c.side));
     // The particle advance (it needs K3's physical velocity and the stage's dt) runs in
     // the main stream between K3 and K4: on a second stream beside K4/K5 it slowed them
@@ -733,7 +745,7 @@ template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, 
     return PANDORA_OK;
 }
 
-template <class T> static int enqueue_stage_t(pandora_handle* h, int stage, int* nlaunch) {
+template <class T> static int enqueue_stage_t(pandora_handle* h, int stage, bool unforced, int* nlaunch) {
     const Member<T> self = self_of<T>(h);   // copied into each launch's parameters
     StepCtx<T> c{};
     c.g = &h->g;
@@ -752,27 +764,38 @@ template <class T> static int enqueue_stage_t(pandora_handle* h, int stage, int*
     c.sortP = &h->P;
     c.timing = h;
     c.zmaps = (h->zmaps_ok && !h->mixed) ? &h->zmaps : nullptr;
+    c.unforced = unforced;
+    c.known_dt = h->sp.rk3_timestep == PANDORA_RK3_TIMESTEP_FIXED ||
+                 (h->sp.rk3_timestep == PANDORA_RK3_TIMESTEP_DECIDE && h->sp.f_type != PANDORA_F_ISOTROPIC &&
+                  h->sp.f_type != PANDORA_F_ISOTROPIC_DEFORMED);
     return enqueue_stage_ctx(c, stage, nlaunch);
 }
 
-static int enqueue_stage(pandora_handle* h, int stage, int* nlaunch) {
-    return h->mixed ? enqueue_stage_t<float>(h, stage, nlaunch) : enqueue_stage_t<double>(h, stage, nlaunch);
+// unforced: of a step whose stage 1 goes before (a stage called alone zeroes or advances the
+// forcing, which the caller may have set, itself)
+static int enqueue_stage(pandora_handle* h, int stage, bool unforced, int* nlaunch) {
+    return h->mixed ? enqueue_stage_t<float>(h, stage, unforced, nlaunch) : enqueue_stage_t<double>(h, stage, unforced, nlaunch);
 }
 
-static int enqueue_step(pandora_handle* h) {
+// Whole steps whose numbers start at tstep0 are never forced where force_stop is 0 or less, unless
+// the caller counts from below it.
+static bool unforced_step(const pandora_handle* h, int tstep0) { return h->fp.stop <= 0 && tstep0 >= h->fp.stop; }
+
+static int enqueue_step(pandora_handle* h, bool unforced) {
     int n = 0;
     for (int s = 1; s <= 3; s++) {
-        int rc = enqueue_stage(h, s, &n);
+        int rc = enqueue_stage(h, s, unforced, &n);
         if (rc) return rc;
     }
     h->launches_per_step = n;
     return PANDORA_OK;
 }
 
+// The graph of a step: unforced for flows that have no forcing (unforced_step of a usual number).
 static int build_graph(pandora_handle* h) {
     if (h->exec) return PANDORA_OK;
     PD_CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
-    int rc = enqueue_step(h);
+    int rc = enqueue_step(h, h->fp.stop <= 0);
     cudaGraph_t gr = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->st, &gr);
     if (rc) { if (gr) cudaGraphDestroy(gr); return rc; }
@@ -810,12 +833,13 @@ extern "C" int pandora_rk3_advance(pandora_handle* h, int32_t tstep0, int32_t ns
     if (cap != cudaStreamCaptureStatusNone) return cuda_fail(cudaErrorStreamCaptureUnsupported, "pandora_rk3_advance");
     int rc = set_clock(h, tstep0, *simtime);
     if (rc) return rc;
-    if (h->use_graph) {
+    const bool unforced = unforced_step(h, tstep0);
+    if (h->use_graph && unforced == (h->fp.stop <= 0)) {
         rc = build_graph(h);
         if (rc) return rc;
         for (int s = 0; s < nsteps; s++) PD_CK(cudaGraphLaunch(h->exec, h->st));
     } else {
-        for (int s = 0; s < nsteps; s++) if ((rc = enqueue_step(h))) return rc;
+        for (int s = 0; s < nsteps; s++) if ((rc = enqueue_step(h, unforced))) return rc;
     }
     if (!sync) return PANDORA_OK;
     PD_CK(cudaMemcpyAsync(h->clock_host, h->clock, sizeof(Clock), cudaMemcpyDeviceToHost, h->st));
@@ -841,7 +865,7 @@ extern "C" int pandora_rk3_stage(pandora_handle* h, int32_t stage, int32_t tstep
     if (stage == 1) h->clock_host->t0 = time;
     h->clock_host->dt = *dt;
     PD_CK(cudaMemcpyAsync(h->clock, h->clock_host, sizeof(Clock), cudaMemcpyHostToDevice, h->st));
-    int rc = enqueue_stage(h, stage, nullptr);
+    int rc = enqueue_stage(h, stage, false, nullptr);
     if (rc) return rc;
     PD_CK(cudaMemcpyAsync(h->clock_host, h->clock, sizeof(Clock), cudaMemcpyDeviceToHost, h->st));
     PD_CK(cudaStreamSynchronize(h->st));
@@ -1077,7 +1101,8 @@ extern "C" int pandora_launches_per_step(pandora_handle* h, int32_t* n) {
     if (!h->launches_per_step) {
         // count without launching: same sequence as enqueue_step
         const bool part = h->particles_on && h->P.np > 0;
-        h->launches_per_step = 1 + 3 * (8 + (part ? 1 : 0) - (scalars_advance(h->g, part ? h->P.np : 0) ? 1 : 0)) + (part ? 5 : 0) + (h->g.shear ? (part ? 2 : 1) : 0);
+        h->launches_per_step = 1 + 3 * (8 + (part ? 1 : 0) - (scalars_advance(h->g, part ? h->P.np : 0) ? 1 : 0)) + (part ? 5 : 0) +
+                               (h->g.shear ? (part ? 2 : 1) : 0) - (h->fp.stop <= 0 ? 2 : 0) + (h->g.dealias_cut > 0.0 ? 3 : 0);
     }
     *n = h->launches_per_step;
     return PANDORA_OK;

@@ -256,7 +256,7 @@ cudaError_t launch_zpass_fwd_update(const Geo& g, const Member<T>* M, int B, int
 template <class T>
 cudaError_t launch_stats(const Geo& g, const Member<T>* M, int B, cudaStream_t st);
 template <class T>
-cudaError_t launch_stage_scalars(const Geo& g, const Member<T>* M, int B, const ForceParams& fp, int stage, bool advance,
+cudaError_t launch_stage_scalars(const Geo& g, const Member<T>* M, int B, const ForceParams& fp, int stage, int advance,
                                  cudaStream_t st);
 template <class T> cudaError_t launch_advance_time(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st);
 template <class T>

@@ -318,6 +318,66 @@ def test_advance_is_refused_under_capture(gpu_lib):
     b.close()
 
 
+def test_launches_per_step(gpu_lib):
+    """The launches of a step, counted before the first one as it then takes them; a flow without
+    forcing takes the stage scalars in stage 1 only (each further branch of the step's graph
+    costs a new simulation's first step its share of the instantiation)."""
+    def count(name, npart=0, stop=None, **kw):
+        p = gpu_lib.workload_params(name, 32)
+        p.p_track_part, p.p_np_global = (1, npart) if npart else (0, 0)
+        if stop is not None:
+            p.force_stop = stop
+        for k, v in kw.items():
+            setattr(p, k, v)
+        with gpu_lib.Simulation(p) as s:
+            s.init_fluid()
+            if npart:
+                s.init_particles()
+            n = s.launches_per_step()
+            s.step()
+            assert s.launches_per_step() == n, (name, npart, stop)
+            return n
+
+    forced = count("iso_forced_particles", stop=10)
+    assert count("iso_forced_particles", stop=0) == forced - 2
+    assert count("iso_decay") == forced - 2
+    assert count("iso_decay", dealiasing=2) == forced + 1       # one more ahead of each K1
+    with_part = count("iso_forced_particles", 256, stop=10)
+    assert count("iso_forced_particles", 256, stop=0) == with_part - 2
+    count("shear")
+    count("shear", 256)
+
+
+@pytest.mark.parametrize("npart", [0, 256])
+def test_step_number_below_force_stop(gpu_lib, npart):
+    """Forcing acts in every step whose number lies below FORCE_STOP, also where that is 0 and
+    the caller counts from -2: the steps equal the stages called one by one, and from step 0 on
+    there is no forcing left."""
+    p = gpu_lib.workload_params("iso_forced_particles", 32)
+    p.force_stop = 0
+    p.p_track_part, p.p_np_global = (1, npart) if npart else (0, 0)
+    a, b = gpu_lib.Simulation(p), gpu_lib.Simulation(p)
+    for s in (a, b):
+        s.init_fluid()
+        if npart:
+            s.init_particles()
+    t = 0.0
+    for step in (-2, -1, 0, 1):
+        a.simtime = t
+        dt = a.step(step)
+        d = b.stage(1, step, t, 0.0)
+        d = b.stage(2, step, t + d / 3, d)
+        d = b.stage(3, step, t + 0.75 * d, d)
+        assert d == dt
+        assert all(np.array_equal(u, v) for u, v in zip(a.get_state(), b.get_state())), step
+        assert all(np.array_equal(u, v) for u, v in zip(a.get_forcing(), b.get_forcing())), step
+        assert any(np.abs(f).max() > 0.0 for f in a.get_forcing()) == (step < 0), step
+        t = a.simtime
+        assert t == pytest.approx((step + 3) * dt, rel=1e-14)
+    a.close()
+    b.close()
+
+
 def test_nan_detection(gpu_lib):
     p = gpu_lib.workload_params("iso_decay", 16)
     with gpu_lib.Simulation(p) as s:
