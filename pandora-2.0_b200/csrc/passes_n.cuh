@@ -47,36 +47,33 @@ static void launch_after(bool pdl, void (*kernel)(KA...), dim3 grid, int threads
 // Dynamic shared memory limits of the kernels of length N that the geometry uses, for
 // member sets of CAP.
 template <int N, class T, int CAP> static cudaError_t configure_cap(const Geo& g) {
-    cudaError_t e;
+    cudaError_t e = cudaSuccess;
+    // the K1 that zpass_inv_n launches for each form: staged, or element-wise (also for a cubic
+    // grid where the length has that form)
+    auto k1 = [&](auto form) {
+        constexpr int FORM = decltype(form)::value;
+        if (e) return;
+        if constexpr (staged_len<N, T, FORM>()) {
+            e = set_smem(k_zpass_inv_staged<N, FORM, T, CAP>, SCfg<N, T>::smem);
+        } else {
+            e = set_smem(k_zpass_inv<N, FORM, T, CAP>, TCfg<N>::template smem<T>());
+            if constexpr (cube_len<N, T>())
+                if (!e && is_cube(g, N)) e = set_smem(k_zpass_inv<N, FORM, T, CAP, N>, TCfg<N>::template smem<T>());
+        }
+    };
+    if (g.nz == N) {
+        k1(std::integral_constant<int, 0>{});
+        k1(std::integral_constant<int, 1>{});
+        k1(std::integral_constant<int, 2>{});
+        k1(std::integral_constant<int, 3>{});
+        if (e) return e;
+        if ((e = set_smem(k_zpass_fwd<N, T, CAP>, TCfg<N, 2>::template smem<T>()))) return e;
+    }
     if constexpr (cube_len<N, T>()) {
         if (is_cube(g, N)) {
-            if ((e = set_smem(k_zpass_inv<N, 0, T, CAP, N>, TCfg<N>::template smem<T>()))) return e;
-            if ((e = set_smem(k_zpass_inv<N, 1, T, CAP, N>, TCfg<N>::template smem<T>()))) return e;
-            if ((e = set_smem(k_zpass_inv<N, 2, T, CAP, N>, TCfg<N>::template smem<T>()))) return e;
-            if ((e = set_smem(k_zpass_inv<N, 3, T, CAP, N>, TCfg<N>::template smem<T>()))) return e;
             if ((e = set_smem(k_ypass_inv<N, T, CAP, N>, TCfg<N, 1>::template smem<T>()))) return e;
             if ((e = set_smem(k_ypass_fwd<N, T, CAP, N>, TCfg<N, 1>::template smem<T>()))) return e;
         }
-    }
-    if (g.nz == N) {
-        cudaError_t es = cudaSuccess;
-        auto staged = [&](auto form) {
-            constexpr int FORM = decltype(form)::value;
-            if constexpr (staged_len<N, T, FORM>())
-                if (!es) es = set_smem(k_zpass_inv_staged<N, FORM, T, CAP>, SCfg<N, T>::smem);
-        };
-        staged(std::integral_constant<int, 0>{});
-        staged(std::integral_constant<int, 1>{});
-        staged(std::integral_constant<int, 2>{});
-        staged(std::integral_constant<int, 3>{});
-        if (es) return es;
-    }
-    if (g.nz == N) {
-        if ((e = set_smem(k_zpass_inv<N, 0, T, CAP>, TCfg<N>::template smem<T>()))) return e;
-        if ((e = set_smem(k_zpass_inv<N, 1, T, CAP>, TCfg<N>::template smem<T>()))) return e;
-        if ((e = set_smem(k_zpass_inv<N, 2, T, CAP>, TCfg<N>::template smem<T>()))) return e;
-        if ((e = set_smem(k_zpass_inv<N, 3, T, CAP>, TCfg<N>::template smem<T>()))) return e;
-        if ((e = set_smem(k_zpass_fwd<N, T, CAP>, TCfg<N, 2>::template smem<T>()))) return e;
     }
     if (g.ny == N) {
         if ((e = set_smem(k_ypass_inv<N, T, CAP>, TCfg<N, 1>::template smem<T>()))) return e;
@@ -113,8 +110,8 @@ template <int N, class T> cudaError_t configure_n(const Geo& g) {
     return cudaSuccess;
 }
 
-// K1 (z length N): the staged kernel for a single FP64 simulation with tensor maps, else
-// the element-wise kernel of the flow's form.
+// K1 (z length N): the tensor-copy kernel for a single FP64 simulation with tensor maps, else the
+// copy-staged kernel (staged_len) or the element-wise kernel of the flow's form.
 template <int N, class T>
 cudaError_t zpass_inv_n(const Geo& g, const Member<T>* M, int B, int stage, cudaStream_t st, const ZMaps* maps, bool pdl) {
     if constexpr (std::is_same<T, double>::value && ZStage<N>::enabled) {
