@@ -571,8 +571,6 @@ template <int ROWB, int R0> constexpr int tile_pad() {
     return (ROWB >= 128 || R0 % 2 != 0) ? 0 : (R0 == 8 ? 3 : (R0 == 16 ? 4 : (R0 == 32 ? 5 : (R0 == 4 ? 2 : 0))));
 }
 
-// Threads per CTA of a direct tile transform of L = 8 lines: one item per thread
-// in the widest pass, at most 512.
 // Threads of a tile transform of L lines with the radix plan (R0, R1, R2): one
 // butterfly per thread in the pass with the most, 64..512.
 template <int N, int R0, int R1, int R2, int L = 8> constexpr int tile_threads_for() {
@@ -582,7 +580,6 @@ template <int N, int R0, int R1, int R2, int L = 8> constexpr int tile_threads_f
     constexpr int m = L * (a > b ? (a > c ? a : c) : (b > c ? b : c));
     return m < 64 ? 64 : (m > 512 ? 512 : m);
 }
-template <int N> constexpr int tile_threads() { return tile_threads_for<N, Plan<N>::r0, Plan<N>::r1, Plan<N>::r2>(); }
 
 // Radix schedule of the warp-level transforms (one line per warp): radix 8 where
 // possible so that a pass has N/8 items, about one per lane.
@@ -662,27 +659,6 @@ template <int N> constexpr bool wplanl_ok() {
 }
 
 #if defined(__CUDACC__)
-// One pass of a single line owned by one warp: the line is column 0 of `s`
-// (element n at s[prow<PS>(n)*LP]); only __syncwarp() separates the halves.
-template <int N, int R, int NS, int S, int LP, int PS, class C>
-__device__ __forceinline__ void wpass(C* s, const C* __restrict__ tw, int lane) {
-    constexpr int WORK = N / R;
-    constexpr int IT = (WORK + 31) / 32;
-    C v[IT][R];
-#pragma unroll
-    for (int it = 0; it < IT; it++) {
-        const int w = lane + it * 32;
-        if (WORK % 32 == 0 || w < WORK) pass_load<N, R, NS, S, 1, LP, PS>(s, tw, w, v[it]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int it = 0; it < IT; it++) {
-        const int w = lane + it * 32;
-        if (WORK % 32 == 0 || w < WORK) pass_store<N, R, NS, 1, LP, PS>(s, w, v[it]);
-    }
-    __syncwarp();
-}
-
 // NA lines transformed in lockstep by one warp (interleaved columns 0..NA-1 for
 // AS = 0, else separate arrays AS elements apart): each pass has NA times the
 // independent work of a single line, which fills the lanes a radix-16 pass of
@@ -739,30 +715,6 @@ __device__ __forceinline__ void wpasses(C* s, const C* __restrict__ tw, int lane
     if constexpr (P0 <= 0 && 0 < P1) wpass_n<N, R0, 1, S, LP, PS, NA, AS, KL, NP == 1 ? KS : 0, W>(s, tw, lane);
     if constexpr (P0 <= 1 && 1 < P1 && NP > 1) wpass_n<N, R1, R0, S, LP, PS, NA, AS, 0, NP == 2 ? KS : 0, W>(s, tw, lane);
     if constexpr (P0 <= 2 && 2 < P1 && NP > 2) wpass_n<N, R2, R0 * R1, S, LP, PS, NA, AS, 0, KS, W>(s, tw, lane);
-}
-
-template <int N, int S, int LP, int PS, int NA, bool LOWPASS = false, int AS = 0, class C>
-__device__ __forceinline__ void fft_warp_n(C* s, const C* __restrict__ tw, int lane) {
-    static_assert(wplan_ok<N>() && wplanl_ok<N>(), "no warp radix plan for this length");
-    constexpr int R0 = LOWPASS ? WPlanL<N>::r0 : WPlan<N>::r0;
-    constexpr int R1 = LOWPASS ? WPlanL<N>::r1 : WPlan<N>::r1;
-    constexpr int R2 = LOWPASS ? WPlanL<N>::r2 : WPlan<N>::r2;
-    wpass_n<N, R0, 1, S, LP, PS, NA, AS>(s, tw, lane);
-    if constexpr (R1 != 0) wpass_n<N, R1, R0, S, LP, PS, NA, AS>(s, tw, lane);
-    if constexpr (R2 != 0) wpass_n<N, R2, R0 * R1, S, LP, PS, NA, AS>(s, tw, lane);
-}
-
-// Full length-N transform of the line at column 0 of `s` by the calling warp
-// (the caller makes the line's data visible to the warp before the call).
-template <int N, int S, int LP, int PS, bool LOWPASS = false, class C>
-__device__ __forceinline__ void fft_warp(C* s, const C* __restrict__ tw, int lane) {
-    static_assert(wplan_ok<N>() && wplanl_ok<N>(), "no warp radix plan for this length");
-    constexpr int R0 = LOWPASS ? WPlanL<N>::r0 : WPlan<N>::r0;
-    constexpr int R1 = LOWPASS ? WPlanL<N>::r1 : WPlan<N>::r1;
-    constexpr int R2 = LOWPASS ? WPlanL<N>::r2 : WPlan<N>::r2;
-    wpass<N, R0, 1, S, LP, PS>(s, tw, lane);
-    if constexpr (R1 != 0) wpass<N, R1, R0, S, LP, PS>(s, tw, lane);
-    if constexpr (R2 != 0) wpass<N, R2, R0 * R1, S, LP, PS>(s, tw, lane);
 }
 
 // In-place pass over a [N][LP] shared tile with NT threads; items w = tid + it*NT.

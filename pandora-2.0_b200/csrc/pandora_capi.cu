@@ -638,8 +638,7 @@ extern "C" int pandora_init_particles(pandora_handle* h) {
 // the main stream before the particle advance.  Captured into the step graph, the
 // fork and join become graph edges.
 // What one stage of a batch needs: the batch's geometry, its device member array
-// of B slots, the particles per member, the shell sums (B x shell_words,
-// contiguous), the streams, and for a single simulation the particle sort and the
+// of B slots, the particles per member, the streams, and for a single simulation the particle sort and the
 // pass-timing events.
 template <class T> struct StepCtx {
     const Geo* g;
@@ -648,7 +647,6 @@ template <class T> struct StepCtx {
     long long np;
     int order;
     const ForceParams* fp;
-    double* shell;
     cudaStream_t st, side;
     cudaEvent_t ev_fork, ev_join, ev_side;
     const PartSort* sort;        // null: no per-step particle sort (batches)
@@ -754,7 +752,6 @@ template <class T> static int enqueue_stage_t(pandora_handle* h, int stage, bool
     c.np = (h->particles_on && h->P.np > 0) ? h->P.np : 0;
     c.order = h->pp.order;
     c.fp = &h->fp;
-    c.shell = h->shell_step;
     c.st = h->st;
     c.side = h->side;
     c.ev_fork = h->ev_fork;
@@ -1340,7 +1337,6 @@ template <class T> static int batch_enqueue_step(pandora_batch* b, int* nlaunch)
     c.np = b->cls.p_track_part ? b->cls.p_np_global : 0;
     c.order = b->cls.p_interp_order;
     c.fp = &b->m[0]->fp;         // only its size (the forcing radius) is used at launch
-    c.shell = b->shell;
     c.st = b->st;
     c.side = b->side;
     c.ev_fork = b->ev_fork;

@@ -1097,7 +1097,7 @@ template <int N, class T> struct SCfg {
     using C = typename Cplx<T>::type;
     static constexpr int ce = (int)sizeof(C);
     static constexpr int r0 = TPlan<N, T>::r0, r1 = TPlan<N, T>::r1, r2 = TPlan<N, T>::r2;
-    static constexpr int lines = (N > 512 || (sizeof(T) == 8 && N > 256)) ? 4 : 8;
+    static constexpr int lines = sizeof(T) == 8 && N > 256 ? 4 : 8;
     static constexpr int ps = pdfft::tile_pad<ce * lines, r0>();
     // row pitch: the lanes of a wavefront (M values of 128 bytes) read q consecutive k of each line
     static constexpr int NKK = 2 * (N / 3) + 1, M = 128 / ce, q = M / lines;
