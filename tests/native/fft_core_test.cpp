@@ -30,13 +30,14 @@ static void emu_passes(std::vector<double2>& s, const std::vector<double2>& tw) 
 // The x pass's transform chain on one line (three arrays AS apart, band KB = N/3):
 // backward transforms of band-limited arrays (first pass reading only the band),
 // NL = omega x u at every point, forward transforms of (n1 + i n2) and n3 written
-// only in the band; with FusedPlan::fused the third array's last backward pass,
-// the product and the first forward pass run per item as the kernel runs them.
+// only in the band.  With FusedPlan::fused the third array's last backward pass, the product and
+// the first forward pass run per item as the kernel runs them; with TRIPLE the last backward pass
+// of all three arrays does, and the forward plan is the backward one reversed.
 // Checked against direct long-double DFTs and the product.
-template <int N, int PS>
+template <int N, int PS, bool TRIPLE = false>
 static double check_xchain() {
     using FP = FusedPlan<N>;
-    constexpr int KB = N / 3, AS = (N + (N >> PS) + 7) / 8 * 8 + 4;
+    constexpr int KB = N / 3, AS = (tile_rows<N, PS>() + 7) / 8 * 8 + (TRIPLE ? 0 : 4);
     constexpr int R0 = FP::r0, R1 = FP::r1, R2 = FP::r2, NP = FP::np;
     std::vector<double2> tw(N);
     for (int e = 0; e < N; e++) {
@@ -52,13 +53,36 @@ static double check_xchain() {
                 x[(size_t)p * N + n] = v;
                 s[(size_t)p * AS + prow<PS>(n)] = v;
             }
-    emu_passes<N, +1, PS, 2, AS, R0, R1, R2, 0, NP, KB>(s, tw);
+    emu_passes<N, +1, PS, 2, AS, R0, R1, R2, 0, TRIPLE ? NP - 1 : NP, KB>(s, tw);
     auto nl = [](double u1, double u2, double u3, double w1, double w2, double w3, double& n3) {
         n3 = u2 * w1 - u1 * w2;
         return mk(u3 * w2 - u2 * w3, u1 * w3 - u3 * w1);
     };
     std::vector<double2> a2(s.begin() + 2 * AS, s.begin() + 3 * AS);
-    if constexpr (FP::fused) {
+    if constexpr (TRIPLE) {
+        constexpr int RL = FP::rl, NRL = FP::nrl;
+        emu_passes<N, +1, PS, 1, 0, R0, R1, R2, 0, NP - 1, KB>(a2, tw);
+        std::vector<double2> v((size_t)3 * NRL * RL);
+        for (int j = 0; j < NRL; j++) {   // every item reads ...
+            double2 *v0 = &v[(size_t)3 * RL * j], *v1 = v0 + RL, *v2 = v1 + RL;
+            pass_load<N, RL, NRL, +1, 1, 1, PS, 0>(s.data(), tw.data(), j, v0);
+            pass_load<N, RL, NRL, +1, 1, 1, PS, 0>(s.data() + AS, tw.data(), j, v1);
+            pass_load<N, RL, NRL, +1, 1, 1, PS, 0>(a2.data(), tw.data(), j, v2);
+        }
+        for (int j = 0; j < NRL; j++) {   // ... before any writes
+            double2 *v0 = &v[(size_t)3 * RL * j], *v1 = v0 + RL, *v2 = v1 + RL;
+            for (int r = 0; r < RL; r++) {
+                double n3;
+                v0[r] = nl(v0[r].x, v0[r].y, v1[r].x, v1[r].y, v2[r].x, v2[r].y, n3);
+                v1[r] = mk(n3, 0.0);
+            }
+            dft<RL, -1>(v0);
+            pass_store<N, RL, 1, 1, 1, PS, 0>(s.data(), j, v0);
+            dft<RL, -1>(v1);
+            pass_store<N, RL, 1, 1, 1, PS, 0>(s.data() + AS, j, v1);
+        }
+        emu_passes<N, -1, PS, 2, AS, RL, (R2 ? R1 : R0), (R2 ? R0 : 0), 1, NP, 0, KB>(s, tw);
+    } else if constexpr (FP::fused) {
         constexpr int RL = FP::rl, NRL = FP::nrl;
         emu_passes<N, +1, PS, 1, 0, R0, R1, R2, 0, NP - 1, KB>(a2, tw);
         std::vector<double2> v((size_t)NRL * RL), xx((size_t)NRL * RL);
@@ -89,7 +113,7 @@ static double check_xchain() {
             s[AS + prow<PS>(n)] = mk(n3, 0.0);
         }
     }
-    emu_passes<N, -1, PS, 2, AS, FP::f0, FP::f1, FP::f2, FP::fused ? 1 : 0, NP, 0, KB>(s, tw);
+    if constexpr (!TRIPLE) emu_passes<N, -1, PS, 2, AS, FP::f0, FP::f1, FP::f2, FP::fused ? 1 : 0, NP, 0, KB>(s, tw);
     // direct: backward DFTs, product, forward DFTs
     std::vector<long double> ph((size_t)6 * N);
     for (int p = 0; p < 3; p++)
@@ -348,6 +372,19 @@ int main() {
     RUNX(192, 4); RUNX(256, 4); RUNX(384, 5); RUNX(512, 5); RUNX(768, 4); RUNX(1024, 5);
     RUNX(40, 4); RUNX(56, 4); RUNX(80, 4); RUNX(112, 4); RUNX(160, 4); RUNX(224, 4); RUNX(320, 4);
     RUNX(448, 4); RUNX(640, 4); RUNX(896, 4);
+#define RUNT(N, P, Q)                                                                        \
+    do {                                                                                     \
+        double e = check_xchain<N, P, true>(), e2 = check_xchain<N, Q, true>();              \
+        printf("x chain, three arrays N=%4d PS=%d %d err %.2e %.2e\n", N, P, Q, e, e2);     \
+        if (!(e < 1e-13 && e2 < 1e-13)) bad++;                                               \
+    } while (0)
+    // the pads of the FP64 and of the FP32 x pass (in FP64 arithmetic here)
+    RUNT(16, 2, 2); RUNT(24, 3, 3); RUNT(32, 3, 3); RUNT(40, 3, 3); RUNT(48, 3 + 16 * 5, 3 + 16 * 5);
+    RUNT(56, 4, 4); RUNT(64, 3, 3); RUNT(80, 3 + 16 * 4, 3 + 16 * 4); RUNT(96, 3, 3); RUNT(112, 4, 4);
+    RUNT(128, 3 + 16 * 6, 4); RUNT(160, 4 + 16 * 5, 4 + 16 * 5); RUNT(192, 4 + 16 * 7, 4 + 16 * 6); RUNT(224, 4, 4);
+    RUNT(256, 4, 4); RUNT(320, 4 + 16 * 7, 5 + 16 * 6); RUNT(384, 5, 5); RUNT(448, 4, 4 + 16 * 8);
+    RUNT(512, 4 + 16 * 7, 4 + 16 * 8); RUNT(640, 5 + 16 * 6, 5); RUNT(768, 5, 5); RUNT(896, 5 + 16 * 8, 5);
+    RUNT(1024, 5, 5);
 #define RUNB(N, PS)                                                           \
     do {                                                                      \
         double e = check_band<N, 4, PS>(), e0 = check_band<N, 3, 0>();        \

@@ -96,6 +96,51 @@ def test_batch_shear_across_remesh(gpu_lib, form):
         assert tke > 0 and eps > 0 and np.all(np.isfinite(ek))
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("dims,flow", [((32, 32, 128), 0), ((32, 32, 192), 0), ((32, 32, 128), 1), ((32, 32, 192), 2),
+                                       ((32, 32, 128), 3), ((32, 32, 256), 3),
+                                       ((96, 32, 32), 0), ((128, 32, 32), 1), ((192, 32, 32), 0), ((256, 32, 32), 2)])
+def test_batch_staged_k1_and_two_lines_per_warp(gpu_lib, dims, flow, precision):
+    """The copy-staged K1 (z of 128 and 192 points, 256 in the R-conv form) and the x pass of two
+    lines per warp (x of 96 to 256 points), batched: isotropic (0), BF-rot (1), R-rot (2) and
+    R-conv (3) members, one admitted late, beside idle slots."""
+    base = gpu_lib.workload_params("shear" if flow else "iso_decay", 32)
+    base.p_track_part = 0
+    if flow:
+        base.f_remesh_t = 5
+        base.ns_deformed = {1: gpu_lib.NS_BF_ROT, 2: gpu_lib.NS_R_ROT, 3: gpu_lib.NS_R_CONV}[flow]
+    base.nodes_x, base.nodes_y, base.nodes_z = dims
+    base.precision = precision
+    with gpu_lib.Batch(base, 4) as b:
+        s0 = b.admit(_member(base, 41))
+        b.step(2)
+        s1 = b.admit(_member(base, 42), 3)
+        b.step(2)
+        b.sync()
+        assert (s0, s1) == (0, 3)
+        assert _same(b.get_state(s0), _alone(gpu_lib, _member(base, 41), 4)[0])
+        assert _same(b.get_state(s1), _alone(gpu_lib, _member(base, 42), 2)[0])
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batch_idle_launch_chunk(gpu_lib, precision):
+    """34 slots of 32 x 32 x 128 with members in the first launch of each pass only, then in
+    both: the second launch, all idle, must not let the next pass start before the first ended."""
+    base = gpu_lib.workload_params("iso_decay", 32)
+    base.nodes_z = 128
+    base.precision = precision
+    with gpu_lib.Batch(base, 34) as b:
+        for k in range(6):
+            b.admit(_member(base, 51 + k), k)
+        b.step(4)
+        b.admit(_member(base, 61), 33)
+        b.step(2)
+        b.sync()
+        for k in (0, 3, 5):
+            assert _same(b.get_state(k), _alone(gpu_lib, _member(base, 51 + k), 6)[0]), k
+        assert _same(b.get_state(33), _alone(gpu_lib, _member(base, 61), 2)[0])
+
+
 def test_batch_rejects_other_class_and_full(gpu_lib):
     base = gpu_lib.workload_params("iso_decay", 32)
     with gpu_lib.Batch(base, 1) as b:

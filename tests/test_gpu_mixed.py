@@ -62,9 +62,10 @@ def test_mixed_nonlinear_every_tile_shape(gpu_lib, dims):
 @pytest.mark.parametrize("n", [160, 224, 320, 384, 448, 640, 768, 896])
 def test_mixed_nonlinear_two_pass_lengths(gpu_lib, n, axis):
     """The lengths of the prime-factor radices in FP32 along each axis (their plans are not those
-    of FP64 from 448 points on); odd numbers of lines and of tiles on the other two."""
+    of FP64 from 448 points on); along y and z an odd number of tiles of i (three, the last one
+    with a single column of the spectrum)."""
     p = gpu_lib.workload_params("iso_decay", 32)
-    dims = [24, 16, 16]
+    dims = [48, 16, 16]
     dims[axis] = n
     p.nodes_x, p.nodes_y, p.nodes_z = dims
     o, s = _mixed(gpu_lib, p)

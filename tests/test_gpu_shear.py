@@ -258,3 +258,32 @@ def test_staged_k1_lengths_and_forms(gpu_lib, form, dims):
     assert rel_l2_fields(s.nonlinear(), o.nonlinear()) < 1e-12
     s.check_status()
     s.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("form", [1, 2, 3])
+@pytest.mark.parametrize("nz", [128, 192, 256, 320, 448, 512])
+def test_copy_staged_k1_forms(gpu_lib, nz, form, precision):
+    """z lengths whose K1 stages its rows by asynchronous copies (256: R-conv; 512: FP32), in the
+    BF-rot (1), R-rot (2) and R-conv (3) forms and both precisions: the product of one state
+    against the oracle in a frame with bmat(1,3) != 0; the last tile of i partial (17 of 24
+    columns)."""
+    import oracle as O
+    p = _shear(gpu_lib, 32, remesh_t=5)
+    p.ns_deformed = {1: gpu_lib.NS_BF_ROT, 2: gpu_lib.NS_R_ROT, 3: gpu_lib.NS_R_CONV}[form]
+    p.nodes_x, p.nodes_y, p.nodes_z = 48, 16, nz
+    o = O.Oracle(p)
+    p.precision = precision
+    s = gpu_lib.Simulation(p)
+    s.init_fluid()
+    o.set_state(s.get_state())
+    t = 0.0
+    for step in (1, 2):
+        t, _ = o.step(step, t)
+        s.step(step)
+    assert s.frame()[0] != 0.0
+    assert s.frame() == pytest.approx(o.frame(), rel=1e-14)
+    o.set_state(s.get_state())      # the product of one state: no drift of the two runs
+    e = rel_l2_fields(s.nonlinear(), o.nonlinear())
+    s.close()
+    assert e < (1e-5 if precision else 1e-12), e    # the bars of the other product tests
