@@ -19,7 +19,7 @@ BUILD = os.path.join(HERE, "_build")
 PASS_GROUPS = "abcdefghijk"
 SOURCES = (["passes_n%s.cu" % g for g in PASS_GROUPS] +
            ["kernels_passes.cu", "kernels_fluid.cu", "kernels_particles.cu", "pandora_capi.cu", "pandora_static.cu"])
-HEADERS = ["fft_core.cuh", "pandora_internal.cuh", "bfrot.cuh", "passes_kernels.cuh", "passes_n.cuh"]
+HEADERS = ["fft_core.cuh", "mode_index.cuh", "pandora_internal.cuh", "bfrot.cuh", "passes_kernels.cuh", "passes_n.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-Xptxas", "-v"]

@@ -24,6 +24,7 @@
 #include <math.h>
 #include <type_traits>
 #include "fft_core.cuh"
+#include "mode_index.cuh"
 #include "pandora_internal.cuh"
 #include "bfrot.cuh"
 
@@ -724,8 +725,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_rk_update(const
     const FieldsT<T>& F = mm.F;
     const Geo& g = mm.g;
     const C* __restrict__ nlh = F.yb;   // NL-hat from K5a
-    // mode q of the plane i; j from a product with 1 / NKK, exact for planes below 2^19 modes
-    // (0.5 / NKK is more than twice its rounding)
+    // mode q of the plane i
     const int i = blockIdx.y, plane = g.nkj * g.nkk, q = blockIdx.x * 256 + threadIdx.x;
     if (q >= plane) return;
     const long long m = (long long)i * plane + q;
@@ -736,7 +736,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4) k_rk_update(const
         in.u[c] = F.u[c][m];
         if (stage != 1) in.r[c] = F.rk[c][m];
     }
-    const int j = (int)(((float)q + 0.5f) * (1.0f / (float)g.nkk)), k = q - j * g.nkk;
+    int j, k;
+    mode_row(q, g.nkk, j, k);
     rk_mode<FORM, T>(F, g, stage, i, j, k, m, in);
 }
 

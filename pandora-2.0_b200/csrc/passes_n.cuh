@@ -94,6 +94,7 @@ template <int N, class T, int CAP> static cudaError_t configure_cap(const Geo& g
 }
 
 template <int N, class T> cudaError_t configure_n(const Geo& g) {
+    static_assert(N <= kMaxLength, "mode_row covers the planes of lengths up to kMaxLength");
     cudaError_t e;
     if constexpr (std::is_same<T, double>::value && ZStage<N>::enabled) {
         if (g.nz == N) {

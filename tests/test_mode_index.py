@@ -1,16 +1,17 @@
-"""The row of a mode in the update kernel (k_rk_update): j = floor((q + 1/2) * (1 / NKK)) in 32-bit
-floating point, for every mode q of the largest plane that a z length can meet."""
-import numpy as np
-import pytest
+"""The row of a mode in the update kernel (mode_row of csrc/mode_index.cuh, as k_rk_update calls
+it), for every mode q of the largest plane that a z length can meet."""
+import os
+import shutil
+import subprocess
 
-LENGTHS = sorted(2 ** a * f for a in range(3, 11) for f in (1, 3, 5, 7) if 16 <= 2 ** a * f <= 1024)
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-@pytest.mark.parametrize("nz", LENGTHS)
-def test_row_of_a_mode(nz):
-    nkk, nkj = 2 * (nz // 3) + 1, 2 * (1024 // 3) + 1
-    q = np.arange(nkj * nkk, dtype=np.int64)
-    assert q.size < 1 << 19
-    inv = np.float32(1.0) / np.float32(nkk)
-    j = ((q.astype(np.float32) + np.float32(0.5)) * inv).astype(np.int64)
-    assert np.array_equal(j, q // nkk)
+def test_row_of_a_mode(tmp_path):
+    cxx = shutil.which("g++") or "/usr/bin/g++"
+    exe = tmp_path / "mode_index_test"
+    subprocess.run([cxx, "-std=c++17", "-O2", "-I", os.path.join(ROOT, "pandora-2.0_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "native", "mode_index_test.cpp"), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.stdout.strip() == "23 lengths OK"
