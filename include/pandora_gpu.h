@@ -157,7 +157,11 @@ int pandora_sizes(const pandora_params* p, int32_t* nki, int32_t* nkj, int32_t* 
 /*
  * Allocates the device state for one simulation on the current CUDA device
  * (replaces ProgramInit's f_ArraysInit/f_FftwInit/f_ForceInit,
- * src/pg_control.f90:52-146).  The state starts at zero.
+ * src/pg_control.f90:52-146).  The state starts at zero.  With particles the
+ * physical velocity takes four reals a point in a buffer of its own, or, where
+ * that does not fit on the device, shares the z-pencil buffer (same results;
+ * pandora_realspace_stats and pandora_nonlinear then pass part of it through
+ * host memory).
  */
 int pandora_create(const pandora_params* p, pandora_handle** out);
 int pandora_destroy(pandora_handle* h);
@@ -300,7 +304,8 @@ int pandora_pass_times(pandora_handle* h, float* ms);
  * the host; the batch is not re-entrant.
  */
 typedef struct pandora_batch pandora_batch;
-/* Device bytes a batch of this class and capacity allocates (for admission control). */
+/* Device bytes a batch of this class and capacity allocates (for admission control); members
+ * keep their physical velocity in the z-pencil buffer. */
 int pandora_batch_bytes(const pandora_params* cls, int32_t capacity, int64_t* bytes);
 /* Capacity > 1 needs grid lengths of 32, 48, 64, 96, 128, 192 or 256 on every axis (the
  * ensemble's sizes; other lengths: PANDORA_ERR_UNSUPPORTED, or capacity 1). */

@@ -664,8 +664,8 @@ __global__ void k_check_finite(const __grid_constant__ MemberSet<T, CAP> ms) {
 // host launchers
 // ---------------------------------------------------------------------------
 
-int stats_ctas(const Geo& g) {
-    const long long rows = (long long)g.nki * g.nkj;
+int stats_ctas(int nki, int nkj) {
+    const long long rows = (long long)nki * nkj;
     return (int)std::min<long long>(4LL * sm_count(), std::max<long long>(1, rows / 8));
 }
 
@@ -673,7 +673,7 @@ int stats_ctas(const Geo& g) {
 template <class T>
 cudaError_t launch_stats(const Geo& g, const Member<T>* M, int B, cudaStream_t st) {
     const size_t nsh = shell_words(g);
-    const int gi = stats_ctas(g);
+    const int gi = stats_ctas(g.nki, g.nkj);
     cudaError_t e = for_member_sets(M, B, [&](const auto& ms, int nm) {
         k_stats<T, PD_CAP(ms)><<<dim3((unsigned)gi, nm), 256, sizeof(double) * nsh, st>>>(ms, gi);
     });

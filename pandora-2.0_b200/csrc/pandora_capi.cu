@@ -59,6 +59,11 @@ struct pandora_handle {
     bool particles_on = false;
     ZMaps zmaps{};                    // tensor maps of u for the staged K1 (FP64, z lengths that have it)
     bool zmaps_ok = false;
+    // The physical velocity begins at field 3 of the z-pencil buffer, one allocation for both: it
+    // lives from the x pass to the particle advance, when no z pencil does, and K4 writes fields
+    // 0 to 2 only.  16/3 instead of 20/3 reals a point.  Batch members, and a simulation that
+    // does not fit otherwise; a pass run outside a step then keeps what it overwrites (PhysKeep).
+    bool phys_shared = false;
 };
 
 static thread_local char g_errmsg[256];
@@ -169,7 +174,8 @@ static void release(pandora_handle* h) {
     cudaSetDevice(h->dev);
     if (h->exec) cudaGraphExecDestroy(h->exec);
     if (h->graph) cudaGraphDestroy(h->graph);
-    cudaFree(h->fbuf); cudaFree(h->F.zb); cudaFree(h->F.yb); cudaFree(h->F.phys);
+    cudaFree(h->fbuf); cudaFree(h->F.zb); cudaFree(h->F.yb);
+    if (!h->phys_shared) cudaFree(h->F.phys);
     cudaFree(h->F.forcing); cudaFree(h->tw); cudaFree(h->clock); cudaFree(h->shell_step);
     cudaFree(h->pbuf); cudaFree(h->pbuf2); cudaFree(h->nlbuf); cudaFree(h->rsbuf);
     cudaFree(h->sort.key); cudaFree(h->sort.count); cudaFree(h->sort.block_sums);
@@ -242,7 +248,15 @@ static int validate(const pandora_params* p) {
     return PANDORA_OK;
 }
 
-extern "C" int pandora_create(const pandora_params* p, pandora_handle** out) {
+// Bytes of one field of the z pencils, of the physical velocity, and of both in one allocation.
+static size_t zfield_bytes(const Geo& g, size_t ce) { return ce * (size_t)g.nz * g.nkj * g.nkip; }
+static size_t phys_bytes(const Geo& g, size_t ce) { return ce / 2 * 4 * (size_t)g.R; }
+static size_t shared_bytes(const Geo& g, size_t ce) {
+    return 3 * zfield_bytes(g, ce) + std::max((size_t)(pass_fields(g) - 3) * zfield_bytes(g, ce), phys_bytes(g, ce));
+}
+
+// shared: the physical velocity in the z-pencil buffer (pandora_handle::phys_shared).
+static int create_handle(const pandora_params* p, bool shared, pandora_handle** out) {
     if (!out) return PANDORA_ERR_INVALID_ARG;
     *out = nullptr;
     int rc = validate(p);
@@ -296,18 +310,20 @@ extern "C" int pandora_create(const pandora_params* p, pandora_handle** out) {
         e = cudaMalloc((void**)&(ptr), (bytes));                          \
         if (e != cudaSuccess) { cudaGetLastError(); release(h); return PANDORA_ERR_OOM; } \
     } while (0)
-    // fields in the stored precision; zb (6 x NZ x NKJ x NKIP values, NZ >= NKK and
+    // fields in the stored precision; yb (6 x NZ x NY x NKIP values, NZ >= NKK, NY >= NKJ and
     // NKIP >= NKI) always holds 3S FP64 values, the conversion scratch of the mixed form.
     // The R-conv form carries 9 fields through the inverse z and y passes.
+    h->phys_shared = shared && h->particles_on;
     PD_ALLOC(h->fbuf, ce * 6 * (size_t)g.S);
-    PD_ALLOC(h->F.zb, ce * (size_t)pass_fields(g) * g.nz * g.nkj * g.nkip);
+    PD_ALLOC(h->F.zb, h->phys_shared ? shared_bytes(g, ce) : (size_t)pass_fields(g) * zfield_bytes(g, ce));
     PD_ALLOC(h->F.yb, ce * (size_t)pass_fields(g) * g.nz * g.ny * g.nkip);
-    if (h->particles_on) PD_ALLOC(h->F.phys, ce / 2 * 4 * (size_t)g.R);
+    if (h->phys_shared) h->F.phys = reinterpret_cast<double*>(reinterpret_cast<char*>(h->F.zb) + 3 * zfield_bytes(g, ce));
+    else if (h->particles_on) PD_ALLOC(h->F.phys, phys_bytes(g, ce));
     PD_ALLOC(h->F.forcing, sizeof(double2) * 3 * (size_t)h->nforce);
     PD_ALLOC(h->tw, ce * (size_t)(g.nx + g.ny + g.nz));
     PD_ALLOC(h->clock, sizeof(Clock));
     const size_t nsh = shell_words(g);
-    PD_ALLOC(h->shell_step, sizeof(double) * nsh * (2 + (size_t)stats_ctas(g)));
+    PD_ALLOC(h->shell_step, sizeof(double) * nsh * (2 + (size_t)stats_ctas(g.nki, g.nkj)));
     h->shell_now = h->shell_step + nsh;
     h->shell_part = h->shell_now + nsh;
 #undef PD_ALLOC
@@ -446,6 +462,11 @@ extern "C" int pandora_create(const pandora_params* p, pandora_handle** out) {
     return PANDORA_OK;
 }
 
+extern "C" int pandora_create(const pandora_params* p, pandora_handle** out) {
+    const int rc = create_handle(p, false, out);
+    return rc == PANDORA_ERR_OOM && p->p_track_part ? create_handle(p, true, out) : rc;
+}
+
 extern "C" int pandora_destroy(pandora_handle* h) {
     if (!h) return PANDORA_ERR_INVALID_ARG;
     release(h);
@@ -479,7 +500,7 @@ static int copy3(pandora_handle* h, double2* const* dev, const double* a, const 
 }
 
 // Three spectral fields of S complex values at the FP64 boundary.  The mixed form
-// stores FP32: the host's FP64 values pass through the z-pencil buffer (free between
+// stores FP32: the host's FP64 values pass through the y-pencil buffer (free between
 // steps) and are converted on the device in either direction.
 static int copy_fields(pandora_handle* h, double2* const* dev64, float2* const* dev32, const double* a,
                        const double* b, const double* c, bool to_dev) {
@@ -487,7 +508,7 @@ static int copy_fields(pandora_handle* h, double2* const* dev64, float2* const* 
     if (!h->mixed) return copy3(h, dev64, a, b, c, (size_t)h->g.S, to_dev);
     cudaSetDevice(h->dev);
     const long long S = h->g.S;
-    double2* scr[3] = {h->F.zb, h->F.zb + S, h->F.zb + 2 * S};
+    double2* scr[3] = {h->F.yb, h->F.yb + S, h->F.yb + 2 * S};
     if (to_dev) {
         int rc = copy3(h, scr, a, b, c, (size_t)S, true);
         if (rc) return rc;
@@ -545,9 +566,9 @@ static int init_fluid_async(pandora_handle* h) {
     ip.b110 = h->p.b110; ip.b220 = h->p.b220; ip.b330 = h->p.b330;
     ip.deformed = (h->p.b110 + h->p.b220 + h->p.b330) > 3 ? 1 : 0;
     ip.key = stream_key(h->p.seed_fluid, TAG_FLUID);
-    if (h->mixed) {   // generated in FP64 into the z-pencil buffer, then rounded once
+    if (h->mixed) {   // generated in FP64 into the y-pencil buffer, then rounded once
         Fields Fd = h->F;
-        for (int c = 0; c < 3; c++) Fd.u[c] = h->F.zb + c * h->g.S;
+        for (int c = 0; c < 3; c++) Fd.u[c] = h->F.yb + c * h->g.S;
         PD_CK(launch_init_fluid(h->g, Fd, ip, h->st));
         for (int c = 0; c < 3; c++) PD_CK(launch_convert(Fd.u[c], h->Ff.u[c], h->g.S, h->st));
         const Member<float> m = self_of<float>(h);
@@ -935,9 +956,38 @@ extern "C" int pandora_last_step_stats(pandora_handle* h, double* ek, int32_t kk
     return PANDORA_OK;
 }
 
+// Where the physical velocity shares the z-pencil buffer, the part of it that K1 overwrites, kept
+// on the host while K1 runs outside a step (the velocity of the last stage stays readable).
+namespace {
+struct PhysKeep {
+    pandora_handle* h;
+    size_t n = 0;
+    void* buf = nullptr;
+    explicit PhysKeep(pandora_handle* hh) : h(hh) {}
+    ~PhysKeep() { free(buf); }
+    int take() {
+        if (!h->phys_shared) return PANDORA_OK;
+        n = std::min((size_t)(pass_fields(h->g) - 3) * zfield_bytes(h->g, h->celem), phys_bytes(h->g, h->celem));
+        if (!(buf = malloc(n))) return PANDORA_ERR_OOM;
+        PD_CK(cudaMemcpyAsync(buf, h->F.phys, n, cudaMemcpyDeviceToHost, h->st));
+        PD_CK(cudaStreamSynchronize(h->st));
+        return PANDORA_OK;
+    }
+    int put() {
+        if (!n) return PANDORA_OK;
+        PD_CK(cudaMemcpyAsync(h->F.phys, buf, n, cudaMemcpyHostToDevice, h->st));
+        PD_CK(cudaStreamSynchronize(h->st));
+        return PANDORA_OK;
+    }
+};
+}  // namespace
+
 extern "C" int pandora_nonlinear(pandora_handle* h, double* n1, double* n2, double* n3) {
     if (!h || !n1 || !n2 || !n3) return PANDORA_ERR_INVALID_ARG;
     cudaSetDevice(h->dev);
+    PhysKeep keep(h);
+    int rc = keep.take();
+    if (rc) return rc;
     if (!h->nlbuf) {
         if (cudaMalloc((void**)&h->nlbuf, h->celem * 3 * (size_t)h->g.S) != cudaSuccess) {
             cudaGetLastError(); return PANDORA_ERR_OOM;
@@ -954,7 +1004,8 @@ extern "C" int pandora_nonlinear(pandora_handle* h, double* n1, double* n2, doub
         PD_CK(launch_ypass_fwd(h->g, Mv, 1, h->st));
         PD_CK(launch_zpass_fwd_update(h->g, Mv, 1, 1, 1, h->st));
         double2* none[3] = {nullptr, nullptr, nullptr};
-        return copy_fields(h, none, Fn.rk, n1, n2, n3, false);
+        rc = copy_fields(h, none, Fn.rk, n1, n2, n3, false);
+        return rc ? rc : keep.put();
     }
     Fields Fn = h->F;
     for (int c = 0; c < 3; c++) Fn.rk[c] = (double2*)h->nlbuf + c * h->g.S;
@@ -965,7 +1016,8 @@ extern "C" int pandora_nonlinear(pandora_handle* h, double* n1, double* n2, doub
     PD_CK(launch_xpass(h->g, Mv, 1, 0, 0, h->st));
     PD_CK(launch_ypass_fwd(h->g, Mv, 1, h->st));
     PD_CK(launch_zpass_fwd_update(h->g, Mv, 1, 1, 1, h->st));
-    return copy3(h, Fn.rk, n1, n2, n3, (size_t)h->g.S, false);
+    rc = copy3(h, Fn.rk, n1, n2, n3, (size_t)h->g.S, false);
+    return rc ? rc : keep.put();
 }
 
 // f_FluidstatsRs2D's sums over the physical field of the current state
@@ -982,6 +1034,9 @@ extern "C" int pandora_realspace_stats(pandora_handle* h, double* out, int32_t n
     if (!h->rsbuf) {
         if (cudaMalloc((void**)&h->rsbuf, sizeof(double) * words) != cudaSuccess) { cudaGetLastError(); return PANDORA_ERR_OOM; }
     }
+    PhysKeep keep(h);
+    int rc = keep.take();
+    if (rc) return rc;
     PD_CK(cudaMemsetAsync(h->rsbuf, 0, sizeof(double) * words, h->st));
     if (h->mixed) {
         const Member<float> mv = self_of<float>(h);
@@ -1002,7 +1057,7 @@ extern "C" int pandora_realspace_stats(pandora_handle* h, double* out, int32_t n
         for (int a = 0; a < 21; a++) out[a] += hb[(size_t)slot * 32 + a];
         for (int a = 21; a < 25; a++) out[a] = std::max(out[a], hb[(size_t)slot * 32 + a]);
     }
-    return PANDORA_OK;
+    return keep.put();
 }
 
 // TS_CORR's longitudinal autocorrelation (f_FluidstatsRs2D, src/pf_fluidstats.f90:933-945):
@@ -1061,9 +1116,9 @@ extern "C" int pandora_get_physical_velocity(pandora_handle* h, double* u1, doub
     if (!h->F.phys) return PANDORA_ERR_UNSUPPORTED;
     cudaSetDevice(h->dev);
     double* d[3] = {u1, u2, u3};
-    // the stored field is interleaved; each component passes through the z-pencil buffer (free
-    // between steps, 6 NZ NKJ NKIP values), widened to FP64 there in the mixed form
-    double* const scr = reinterpret_cast<double*>(h->F.zb);
+    // the stored field is interleaved; each component passes through the y-pencil buffer (free
+    // between steps, 6 NZ NY NKIP values), widened to FP64 there in the mixed form
+    double* const scr = reinterpret_cast<double*>(h->F.yb);
     for (int c = 0; c < 3; c++) {
         if (h->mixed) PD_CK(launch_phys_component(h->Ff.phys, c, scr, h->g.R, h->st));
         else PD_CK(launch_phys_component(h->F.phys, c, scr, h->g.R, h->st));
@@ -1163,7 +1218,11 @@ template <class T> static int profile_pass_t(pandora_handle* h, int32_t pass, in
 extern "C" int pandora_profile_pass(pandora_handle* h, int32_t pass, int32_t reps) {
     if (!h || reps < 0) return PANDORA_ERR_INVALID_ARG;
     cudaSetDevice(h->dev);
-    return h->mixed ? profile_pass_t<float>(h, pass, reps) : profile_pass_t<double>(h, pass, reps);
+    PhysKeep keep(h);
+    int rc = pass == 1 ? keep.take() : PANDORA_OK;
+    if (rc) return rc;
+    rc = h->mixed ? profile_pass_t<float>(h, pass, reps) : profile_pass_t<double>(h, pass, reps);
+    return rc ? rc : keep.put();
 }
 
 extern "C" int pandora_pass_bytes(pandora_handle* h, int32_t pass, double* bytes) {
@@ -1359,9 +1418,11 @@ extern "C" int pandora_batch_bytes(const pandora_params* p, int32_t capacity, in
     const long long ce = p->precision == PANDORA_PREC_FP32_MIXED ? 8 : 16;
     const long long np = p->p_track_part ? p->p_np_global : 0;
     const long long nfb = (p->f_type == PANDORA_F_SHEAR_DNS && p->ns_deformed == PANDORA_NS_R_CONV) ? 9 : 6;
-    long long per = ce * 6 * S + ce * nfb * nz * nkj * nkip + ce * nfb * nz * ny * nkip + ce * (nx + ny + nz);
-    if (p->p_track_part) per += ce / 2 * 4 * R + 2 * 8 * 14 * np + 4 * np;
-    per += 8 * (3 * (kkmax_of(p) + 1) + 3) * 592LL;   // the statistics' partial sums, at most
+    const long long zf = ce * nz * nkj * nkip;
+    long long per = ce * 6 * S + nfb * zf + ce * nfb * nz * ny * nkip + ce * (nx + ny + nz);
+    // the physical velocity from field 3 of the z pencils on (pandora_handle::phys_shared)
+    if (p->p_track_part) per += std::max(0LL, ce / 2 * 4 * R - (nfb - 3) * zf) + 2 * 8 * 14 * np + 4 * np;
+    per += 8LL * (3 * (kkmax_of(p) + 1) + 3) * stats_ctas((int)nki, (int)nkj);   // the statistics' partial sums
     per += 1 << 20;   // clock, forcing, shells, member descriptors, allocator granularity
     *bytes = per * capacity;
     return PANDORA_OK;
@@ -1392,7 +1453,7 @@ extern "C" int pandora_batch_create(const pandora_params* cls, int32_t capacity,
     b->m.assign(capacity, nullptr);
     b->active.assign(capacity, 0);
     for (int i = 0; i < capacity; i++) {
-        rc = pandora_create(cls, &b->m[i]);
+        rc = create_handle(cls, true, &b->m[i]);
         if (rc) { batch_release(b); return rc; }
         b->m[i]->st = b->st;      // every member's copies run in the batch's stream order
     }

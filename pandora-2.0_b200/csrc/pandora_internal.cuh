@@ -295,7 +295,7 @@ cudaError_t launch_phys_component(const double* phys, int c, double* out, long l
 cudaError_t launch_phys_component(const float* phys, int c, double* out, long long n, cudaStream_t st);
 size_t shell_words(const Geo& g);
 // CTAs of the statistics kernel, the rows of FieldsT::part.
-int stats_ctas(const Geo& g);
+int stats_ctas(int nki, int nkj);
 // Does k_stage_scalars also advance the stage's time (else launch_advance_time does)?  Flows
 // whose K5b and particles read neither the frame nor the step number after it.
 inline bool scalars_advance(const Geo& g, long long np) { return !g.shear && np == 0; }

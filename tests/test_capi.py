@@ -86,3 +86,28 @@ def test_strerror():
     L = pandora.load()
     for s in range(0, -11, -1):
         assert L.pandora_strerror(s)
+
+
+@pytest.mark.parametrize("n,npart,mixed,rconv", [(32, 0, 0, 0), (32, 512, 0, 0), (64, 4096, 1, 0), (48, 256, 0, 1)])
+def test_batch_bytes_of_small_classes(n, npart, mixed, rconv):
+    """The bytes a batch is admitted by: the members' buffers, the physical velocity (four reals a
+    point) from the fourth field of the z pencils on, and as many rows of the statistics' partial
+    sums as the statistics have CTAs (an eighth of the (i, j) rows of a small grid)."""
+    import pandora
+    p = pandora.workload_params("shear" if rconv else "iso_decay", n)
+    if rconv:
+        p.ns_deformed = pandora.NS_R_CONV
+    p.precision = mixed
+    p.p_track_part, p.p_np_global = (1, npart) if npart else (0, 0)
+    nki, nkj = n // 3 + 1, 2 * (n // 3) + 1
+    nkip, ce, fields = (nki + 7) // 8 * 8, 8 if mixed else 16, 9 if rconv else 6
+    z, y = ce * n * nkj * nkip, ce * n * n * nkip
+    a, b, c, kkmax = (ctypes.c_int32() for _ in range(4))
+    m = ctypes.c_int64()
+    L = pandora.load()
+    assert L.pandora_sizes(ctypes.byref(p), ctypes.byref(a), ctypes.byref(b), ctypes.byref(c), ctypes.byref(m),
+                           ctypes.byref(kkmax)) == 0
+    want = 6 * ce * m.value + fields * y + 3 * ce * n + 8 * (3 * (kkmax.value + 1) + 3) * (nki * nkj // 8) + (1 << 20)
+    want += 3 * z + max((fields - 3) * z, 2 * ce * n ** 3 if npart else 0) + (2 * 8 * 14 + 4) * npart
+    for cap in (1, 5):
+        assert pandora.batch_bytes(p, cap) == want * cap

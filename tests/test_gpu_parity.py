@@ -378,6 +378,55 @@ def test_step_number_below_force_stop(gpu_lib, npart):
     b.close()
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+def test_physical_velocity_where_memory_is_short(gpu_lib, precision):
+    """A simulation with particles that does not fit with a buffer of its own for the physical
+    velocity is made with the velocity in the z-pencil buffer (as batch members are): the same
+    states, particles and velocities bit for bit, also when passes run outside a step between."""
+    import torch
+    p = gpu_lib.workload_params("iso_forced_particles", 256)
+    p.p_np_global = 1 << 12
+    p.precision = precision
+    word = 4 if precision else 8
+    need = gpu_lib.batch_bytes(p, 1)                     # with the velocity in the z pencils
+    apart = 3 * 2 * word * 256 * 171 * 88                # what a buffer of its own takes in addition
+
+    def run(s):
+        s.init_fluid()
+        s.init_particles()
+        s.advance(2)
+        out = [s.physical_velocity(), s.realspace_sums(), s.nonlinear(), s.get_state()]
+        out.append(s.physical_velocity())
+        s.advance(1)
+        return out + [s.get_state(), s.get_particles()[:2], s.physical_velocity()]
+
+    with gpu_lib.Simulation(p) as s:
+        want = run(s)
+    used = torch.cuda.mem_get_info()[0]
+    with gpu_lib.Simulation(p) as s:
+        used -= torch.cuda.mem_get_info()[0]
+    assert used > need + apart // 2                      # with memory at hand: a buffer of its own
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    filler = torch.empty(free - need - apart // 2, dtype=torch.uint8, device="cuda")
+    before = torch.cuda.mem_get_info()[0]
+    try:
+        s = gpu_lib.Simulation(p)
+        assert before - torch.cuda.mem_get_info()[0] < need + apart // 2
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    got = run(s)
+    s.close()
+    for a, b in zip(got[0], got[4]):
+        assert np.array_equal(a, b)
+    for k, (a, b) in enumerate(zip(got, want)):
+        if k == 1:   # sums of atomics, in any order
+            assert np.allclose(a, b, rtol=1e-12)
+        else:
+            assert all(np.array_equal(x, y) for x, y in zip(a, b)), k
+
+
 def test_nan_detection(gpu_lib):
     p = gpu_lib.workload_params("iso_decay", 16)
     with gpu_lib.Simulation(p) as s:
