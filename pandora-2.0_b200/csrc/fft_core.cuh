@@ -640,9 +640,11 @@ template <> struct WPlanL<1024> { static constexpr int r0 = 32, r1 = 32, r2 = 0;
 // forward transform runs the reversed plan, so that the last backward pass and
 // the first forward pass see the same elements n = j + r * (N / rl) in item j, and
 // the last backward pass of one array, the product and the first forward pass run
-// in registers, one item per lane (nrl = N / rl items, 16..32 of them).  Lines
-// shorter than 256 keep separate passes and the same plan both ways (measured
-// faster at 192: the fused step leaves half the lanes idle there).
+// in registers, one item per lane (nrl = N / rl items, 16..32 of them).  That is the schedule of
+// the lengths whose three arrays do not fit the registers (FP64 from 640 points) and of the
+// statistics pass, whose lines shorter than 256 keep separate passes and the same plan both ways;
+// elsewhere the product step takes all three arrays (the x pass's `triple`), with the reversed
+// plan at every length.
 template <int N> struct FusedPlan {
     static constexpr int r0 = WPlanL<N>::r0, r1 = WPlanL<N>::r1, r2 = WPlanL<N>::r2;
     static constexpr int np = r2 ? 3 : 2;

@@ -654,10 +654,11 @@ extern "C" int pandora_init_particles(pandora_handle* h) {
 // f_RK3Stage{s} (src/pf_rk3.f90:40-200): [s=1: statistics of the state],
 // vorticity + z pass, y pass, x pass with NL (and CFL / physical velocity),
 // dt + forcing, particles, forward y, forward z + RK update, time advance.
-// One stage.  With particles, stage 1 forks a second stream: the spatial sort of
-// the particles runs beside the statistics and the first three passes and joins
-// the main stream before the particle advance.  Captured into the step graph, the
-// fork and join become graph edges.
+// One stage.  Stage 1 forks a second stream for the statistics and, with particles, their spatial
+// sort; stages with scalars and no particles fork it for those.  The sort joins the main
+// stream before the particle advance, the others before the RK update.  Captured into the step
+// graph, the forks and joins become graph edges.
+//
 // What one stage of a batch needs: the batch's geometry, its device member array
 // of B slots, the particles per member, the streams, and for a single simulation the particle sort and the
 // pass-timing events.

@@ -14,11 +14,11 @@
 //   K5 zpass_fwd   zb fields 0..2      -> 3 forward z FFTs, x 1/(NX NY NZ), truncate k, then the
 //                                         per-mode RHS + low-storage RK3 + continuity fix on u, rk
 // Every pass reads and writes HBM once.  The z and y passes (K1, K2, K4, K5a)
-// are tile transforms of 8 lines interleaved in shared memory (pdfft::fft_tile_io):
-// the first radix pass loads its butterfly inputs straight from HBM (rows of 8
-// consecutive i = 128 bytes) and the last pass stores straight to HBM, so a
-// two-pass length crosses shared memory once, behind one block barrier.  The x
-// pass owns whole lines per warp and needs no block barrier at all.
+// are tile transforms of 8 lines (4 or 16 at some lengths) interleaved in shared memory
+// (pdfft::fft_tile_io): the first radix pass loads its butterfly inputs straight from HBM (rows
+// of 8 consecutive i = 128 bytes; K1's staged forms: from rows staged in shared memory) and the
+// last pass stores straight to HBM, so a two-pass length crosses shared memory once, behind one
+// block barrier.  The x pass owns whole lines per warp and needs no block barrier at all.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -86,11 +86,12 @@ __device__ __forceinline__ void store_point(float* p, float a, float b, float c)
     *reinterpret_cast<float4*>(p) = make_float4(a, b, c, 0.0f);
 }
 
-// Start of a pass kernel: the kernel after it may be set up from now on, and this one goes on
-// once the kernel before it has ended and its writes are visible.  Every CTA comes here first, an
-// idle member's too: a kernel whose CTAs all left at once would end before the one ahead of it
-// (a chunk of idle members in a batch), and the kernel behind it would start too early.  A
-// launch without the attribute passes at once.
+// Start of a pass kernel: it goes on once the kernel before it has ended and its writes are
+// visible.  Every CTA comes here first, an idle member's too: a kernel whose CTAs all left at
+// once would end before the one ahead of it (a chunk of idle members in a batch), and the kernel
+// behind it would start too early.  No kernel triggers its dependents itself, so theirs are set
+// up as its last CTAs end (an early trigger placed them unevenly: 64^3 step 0.070 -> 0.082 ms).
+// A launch without the attribute passes at once.
 __device__ __forceinline__ void grid_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -201,8 +202,8 @@ template <int N, class T> struct XCfgStats {
 
 // RS: the real-space statistics pass (the same transforms, plus the moments of every
 // point, reduced per warp into one of kRsSlots copies of the sums in `rs`).
-// LPW: lines per warp (LPW > 1 for short, unfused lines: each group of 32 / LPW lanes
-// transforms its own line).
+// LPW: lines per warp (LPW > 1 for short lines of the triple schedule: each group of 32 / LPW
+// lanes transforms its own line).
 template <int NX, class T, int CAP, bool RS = false, int LPW = 1>
 __global__ void __launch_bounds__(32, RS ? XCfgStats<NX, T>::ctas() : XCfg<NX, T>::ctas()) k_xpass(const __grid_constant__ MemberSet<T, CAP> ms,
                                                                                         int want_phys,
@@ -933,10 +934,10 @@ __global__ void __launch_bounds__(TCfg<NZ>::template nt<T>(),
 
 // ---------------------------------------------------------------------------
 // K1 with the velocity rows staged by the tensor-memory accelerator (FP64, single
-// simulations, z lines of ZStage<NZ>::enabled lengths).  One CTA per tile (8
+// simulations, z lines of ZStage<NZ>::enabled lengths).  One CTA per tile (4
 // consecutive i at one j) forms every field of the tile: the rows
-// u_c[i0..i0+7][j][0..NKK-1] of the three components arrive in shared memory by 3 x NB
-// tensor copies (cp.async.bulk.tensor, boxes of BK k x 1 j x 8 i, completion counted on
+// u_c[i0..i0+3][j][0..NKK-1] of the three components arrive in shared memory by 3 x NB
+// tensor copies (cp.async.bulk.tensor, boxes of BK k x 1 j x 4 i, completion counted on
 // one mbarrier; rows past NKI and k past NKK are filled with zeros by the copy engine).
 // Each field's backward z transform then takes its first-pass inputs from that staging
 // (velocity, or vorticity / gradients formed on the fly) instead of from global memory,
@@ -952,6 +953,7 @@ template <int NZ> struct ZStage {
     // on distinct banks
     static constexpr int BK = BK0 + ((8 / lines - BK0 % 8) % 8 + 8) % 8;
     static_assert(BK <= 128, "tensor box wider than 256 doubles");
+    static_assert((16 * lines * BK) % 128 == 0, "every box lands on a 128-byte boundary");
     static constexpr int words = 3 * NB * lines * BK;            // staged complex values
     static constexpr int r0 = pdfft::Plan<NZ>::r0, r1 = pdfft::Plan<NZ>::r1, r2 = pdfft::Plan<NZ>::r2;
     static constexpr int ps = pdfft::tile_pad<16 * lines, r0>();
@@ -1001,9 +1003,10 @@ __global__ void __launch_bounds__(ZStage<NZ>::nt, 2) k_zpass_inv_tma(const __gri
     const int i0 = blockIdx.x * LT, j = blockIdx.y, tid = threadIdx.x;
     if (stage == 1 && blockIdx.x == 0 && j == 0 && tid == 0) F.clock->ucfl_bits = 0ull;
     const uint32_t ba = smem_u32(bar);
-    // tensor copies land on 128-byte boundaries: each box is 128 BK bytes from a staging
-    // base that must itself be aligned (the dynamic shared memory of this kernel, which has
-    // no static shared memory); otherwise no copy is issued and the status records it
+    // tensor copies land on 128-byte boundaries: the boxes are 16 lines BK bytes (a multiple of
+    // 128) apart from a staging base that must itself be aligned (the dynamic shared memory of
+    // this kernel, which has no static shared memory); otherwise no copy is issued and the status
+    // records it
     if (smem_u32(stg) & 127u) {
         if (tid == 0) atomicOr(&F.clock->status, PD_ST_TIMEOUT);
         return;
@@ -1088,9 +1091,9 @@ __global__ void __launch_bounds__(ZStage<NZ>::nt, 2) k_zpass_inv_tma(const __gri
 }
 
 // ---------------------------------------------------------------------------
-// K1 with the velocity rows staged by asynchronous element copies (cp.async; any length, batches,
-// FP32 rows, which a tensor map cannot describe: NKK is odd, so they start at 8-byte
-// boundaries).  As k_zpass_inv_tma: one CTA forms every field of its tile from rows that arrive
+// K1 with the velocity rows staged by asynchronous element copies (cp.async; the lengths and
+// forms of staged_len, batches, FP32 rows, which a tensor map cannot describe: NKK is odd, so
+// they start at 8-byte boundaries).  As k_zpass_inv_tma: one CTA forms every field of its tile from rows that arrive
 // once, whole and coalesced.  (The element-wise K1 reads u across lines, 16 or 32 bytes of each
 // row per warp load, once per field that needs it.)
 // ---------------------------------------------------------------------------

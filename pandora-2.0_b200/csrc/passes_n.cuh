@@ -26,7 +26,8 @@ template <typename K> static cudaError_t set_smem(K kernel, size_t bytes) {
 }
 
 // Launches `kernel`, with `pdl` as a programmatic dependent of the kernel before it in the
-// stream: its CTAs may be set up while that kernel drains, and wait at grid_wait() for its end.
+// stream: its CTAs may be set up once that kernel's have ended (no kernel triggers earlier), and
+// wait at grid_wait() until its writes are visible.
 template <class... KA, class... A>
 static void launch_after(bool pdl, void (*kernel)(KA...), dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchConfig_t cfg{};
