@@ -676,7 +676,6 @@ template <class T> struct StepCtx {
     pandora_handle* timing;      // null: no pass timing
     const ZMaps* zmaps;          // null: K1 reads u element-wise (batches, FP32, other lengths)
     bool unforced;               // no forcing acts in this step (unforced_step)
-    bool known_dt;               // the step's dt does not wait for the velocity's maximum
 };
 
 template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, int* nlaunch) {
@@ -728,19 +727,18 @@ template <class T> static int enqueue_stage_ctx(const StepCtx<T>& c, int stage, 
     // Without forcing the scalars of stage 1 set the step's dt and zero forcing and, where they
     // advance the time, that of the whole step (no kernel of stages 2 and 3 reads it then).
     // Every fork of a step costs a new state's first step about 50 us of the graph's instantiation:
-    // 32^3 decay 430 us with a fork in every stage, 340 with those of stage 1, 290 where the
-    // scalars of stage 1 follow the statistics as well (without a side stream 255, and 100 us
-    // instead of 70 for the steps after it).  A forced flow, whose scalars draw every stage's
-    // random numbers, earns its forks back in six steps (265 -> 440 us, then 112 -> 82).
+    // 32^3 decay 430 us with a fork in every stage, 320 with those of stage 1 (without a side
+    // stream 255, and 100 us instead of 70 for the steps after it).  Scalars that follow the
+    // statistics without a fork of their own save 50 us more there, but start with K1 and cost
+    // every step 2 us at 32^3 and 3 at 128^3 FP32-mixed.  A forced flow, whose scalars draw every
+    // stage's random numbers, earns its forks back in six steps (265 -> 440 us, then 112 -> 82).
     const bool adv = scalars_advance(g, c.np), scalars = stage == 1 || !c.unforced;
     const int to = !adv ? 0 : (c.unforced ? 3 : stage);
     if (part && scalars) {
         PD_CK(launch_stage_scalars(g, M, B, *c.fp, stage, to, c.st)); n++;
     } else if (scalars) {
-        if (!(c.unforced && c.known_dt)) {   // else they need nothing of K3 and follow the statistics
-            PD_CK(cudaEventRecord(c.ev_fork, c.st));
-            PD_CK(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
-        }
+        PD_CK(cudaEventRecord(c.ev_fork, c.st));
+        PD_CK(cudaStreamWaitEvent(c.side, c.ev_fork, 0));
         PD_CK(launch_stage_scalars(g, M, B, *c.fp, stage, to, c.side)); n++;
     }
     const bool side = stage == 1 || (!part && scalars);   // work on the side stream to wait for
@@ -784,9 +782,6 @@ template <class T> static int enqueue_stage_t(pandora_handle* h, int stage, bool
     c.timing = h;
     c.zmaps = (h->zmaps_ok && !h->mixed) ? &h->zmaps : nullptr;
     c.unforced = unforced;
-    c.known_dt = h->sp.rk3_timestep == PANDORA_RK3_TIMESTEP_FIXED ||
-                 (h->sp.rk3_timestep == PANDORA_RK3_TIMESTEP_DECIDE && h->sp.f_type != PANDORA_F_ISOTROPIC &&
-                  h->sp.f_type != PANDORA_F_ISOTROPIC_DEFORMED);
     return enqueue_stage_ctx(c, stage, nlaunch);
 }
 
