@@ -40,11 +40,11 @@ WORKLOAD = "shear"
 # commands and the raw figures are summarised under profiles/.
 NCU_TRAFFIC_BYTES = {
     ("iso_forced_particles", 256, "fp64_plain"): {
-        "zpass_inv": 432157440, "ypass_inv": 862682752, "xpass_nl": 1177856256, "ypass_fwd": 417905024,
-        "zpass_fwd_update": 261682560 + 549060736, "particles": 605924864},
+        "zpass_inv": 432228736, "ypass_inv": 861288192, "xpass_nl": 1304387584, "ypass_fwd": 417638656,
+        "zpass_fwd_update": 261503232 + 547333888, "particles": 668714624},
     ("shear", 512, "fp64_plain"): {
-        "zpass_inv": 3199086129, "ypass_inv": 7047367930, "xpass_nl": 8904337408, "ypass_fwd": 3324333151,
-        "zpass_fwd_update": 1928149719 + 3921155948, "particles": 1473873920},
+        "zpass_inv": 3254667503, "ypass_inv": 7046917953, "xpass_nl": 9936963584, "ypass_fwd": 3318310388,
+        "zpass_fwd_update": 1921978548 + 3853846898, "particles": 857022464},
 }
 # Seconds of host work the reference arm spends on its timed steps at most (the
 # whole arm, warm-up and set-up included, stays within a few minutes).
